@@ -88,11 +88,29 @@ __device__ __forceinline__ int2 quad_offsets(long long off, long long W, long lo
     return make_int2((int)fwd, (int)bwd);
 }
 
-// The per-step window: 2^-20 (d/R + hmax/d) plus a floor, as the shape of
-// the estimate's error bound 2^-22 (|a| + d/R + hmax/d) demands (the |a| part
-// travels with the chain's maximum).
+// The per-step window of exact f32: 2^-20 (d/R + hmax/d) plus a floor, as the
+// shape of the estimate's error bound 2^-22 (|a| + d/R + hmax/d) demands (the
+// |a| part travels with the chain's maximum).
 __device__ __forceinline__ float step_window(float y, float c, float hmax) {
     return __fadd_rn(__fmul_rn(0x1p-20f, __fadd_rn(c, __fmul_rn(hmax, y))), 0x1p-90f);
+}
+
+// MIXED64's per-step window.  Its estimate takes e = RN(h - h_pov) and folds the
+// observer height o into the step's offset -(d/R + o/d), so that no rounding of
+// it is relative to the elevations themselves: against the real angle a,
+// |estimate - a| <= 2^-24 (3 |a| + 5 d/R + 6 |o|/d) from the roundings of e, 1/d,
+// the offset and the fma, and the FP64 angle adds 2^-53 (hmax/d + ...).  The
+// window 2^-20 (d/R + |o|/d) + 2^-44 hmax/d holds 2.6 x the absolute part of
+// that; kRelMix = 2^-20 of the maximum holds the 3 |a| of both the maximum and a
+// sample near it 2.6 x.  With h_pov + o rounded to f32 first the window was
+// 2^-20 hmax/d: on the sea of a 3601^2 tile with 4500 m peaks every sample past
+// 330 cells fell into it, 7.6e-4 of all samples were re-decided in FP64 and the
+// sweep took 141.8 ms.
+constexpr float kRelMix = 0x1p-20f;
+__device__ __forceinline__ float mix_window(float y, float c, float o, float hmax) {
+    return __fadd_rn(__fadd_rn(__fmul_rn(0x1p-20f, __fadd_rn(c, __fmul_rn(fabsf(o), y))),
+                               __fmul_rn(0x1p-44f, __fmul_rn(hmax, y))),
+                     0x1p-90f);
 }
 
 template <int kPrec> struct SplitTypes;
@@ -260,8 +278,10 @@ k_sweep_split(QueueArgs a) {
                 if constexpr (kFp32) {
                     s_t[i] = make_float4(t.x, -t.z, t.w, 0.0f);
                 } else {
-                    const float g = step_window(t.x, t.z, hmax);
-                    const float zhi = __fadd_rn(-t.z, g), zlo = __fsub_rn(-t.z, g);
+                    const float o = D.observer_height;
+                    const float off = kMix ? -__fadd_rn(t.z, __fmul_rn(o, t.x)) : -t.z;
+                    const float g = kMix ? mix_window(t.x, t.z, o, hmax) : step_window(t.x, t.z, hmax);
+                    const float zhi = __fadd_rn(off, g), zlo = __fsub_rn(off, g);
                     if constexpr (kMix) {
                         s_t[i] = make_float4(t.x, zhi, zlo, t.y);
                         const double4 dt = gd[i];  // {1/d, d/R, d*tan1, d} in double
@@ -335,10 +355,14 @@ k_sweep_split(QueueArgs a) {
             (void)qbase;
             (void)goff;
             (void)gdt;
-            float hp32[K];  // kernel.rs:134, the f32 observer elevation
+            // kernel.rs:134, the f32 observer elevation (MIXED64: the point of
+            // view's own elevation; the observer height is in the step's offset)
+            float hp32[K];
 #pragma unroll
-            for (int k = 0; k < K; k++)
-                hp32[k] = __fadd_rn(__ldg(row_ptr(k / KX) + LX * (k % KX)), D.observer_height);
+            for (int k = 0; k < K; k++) {
+                const float h = __ldg(row_ptr(k / KX) + LX * (k % KX));
+                hp32[k] = kMix ? h : __fadd_rn(h, D.observer_height);
+            }
             // chain k's point-of-view elevation, re-read by the rare exact
             // re-decisions (the address is recomputed rather than kept live)
             auto pov_h = [&](int k) -> float {
@@ -609,8 +633,8 @@ k_sweep_split(QueueArgs a) {
 #pragma unroll
                     for (int k = 0; k < K; k++) {
                         // the initial maximum (-2000, exact) carries the relative part
-                        hi[k] = __fmaf_rn(2000.0f, kRel, -2000.0f);
-                        lo[k] = __fmaf_rn(2000.0f, -kRel, -2000.0f);
+                        hi[k] = __fmaf_rn(2000.0f, kRelMix, -2000.0f);
+                        lo[k] = __fmaf_rn(2000.0f, -kRelMix, -2000.0f);
                         setj(k, -1);
                         acc[k] = (S)0;
                     }
@@ -649,8 +673,8 @@ k_sweep_split(QueueArgs a) {
                         return j < 0 ? (S)kMaxAngle : exact_at(k, (uint32_t)j, load1((uint32_t)j, k));
                     };
                     auto raise = [&](int k, uint32_t st, float fh, float fl, const float4 &t) {
-                        hi[k] = __fmaf_rn(fabsf(fh), kRel, fh);
-                        lo[k] = __fmaf_rn(fabsf(fl), -kRel, fl);
+                        hi[k] = __fmaf_rn(fabsf(fh), kRelMix, fh);
+                        lo[k] = __fmaf_rn(fabsf(fl), -kRelMix, fl);
                         setj(k, (int32_t)st);
                         if constexpr (kMix) acc[k] = __dadd_rn(acc[k], mix_w(st));
                         else acc[k] = __fadd_rn(acc[k], t.w);
@@ -689,8 +713,8 @@ k_sweep_split(QueueArgs a) {
                                 const float fl = __fmaf_rn(e[k], t.x, t.z);
                                 const bool sure = fl > hi[k];
                                 if (sure) {
-                                    hi[k] = __fmaf_rn(fabsf(fh[k]), kRel, fh[k]);
-                                    lo[k] = __fmaf_rn(fabsf(fl), -kRel, fl);
+                                    hi[k] = __fmaf_rn(fabsf(fh[k]), kRelMix, fh[k]);
+                                    lo[k] = __fmaf_rn(fabsf(fl), -kRelMix, fl);
                                     setj(k, (int32_t)i);
                                     if constexpr (kMix) acc[k] = __dadd_rn(acc[k], w);
                                     else acc[k] = __fadd_rn(acc[k], w);
