@@ -297,12 +297,12 @@ int tvs_read_sweep_counters(tvs_context *ctx, uint64_t *counters);
  * at a time, evaluating angles exactly only where a warp's first test passes:
  * a warp holds LX = 8, 16, 32 (L = 1, 2, 3 and again 4, 5, 6; 32 and 16 for
  * L = 7, 8) columns x 32/LX rows of lanes; each lane has four points of view
- * LX columns apart (L <= 3, tiles of 4 LX x 256/LX points), 2 x 2 of them, LX
- * columns and 32/LX rows apart (L = 4..6, tiles of 2 LX x 512/LX), or four of
- * them in one column, 32/LX rows apart (L = 7, 8, tiles of LX x 1024/LX).
- * L = 9 is L = 7's tiling read from four row-interleaved copies of the DEM
+ * LX columns apart (L <= 3), 2 x 2 of them, LX
+ * columns and 32/LX rows apart (L = 4..6), or four of them in one column,
+ * 32/LX rows apart (L = 7, 8); a warp's 128 points are one tile of the queue.
+ * L = 9 is L = 8's tiling read from four row-interleaved copies of the DEM
  * (one 16-byte load per lane and step; the context holds the copies, 4x the
- * DEM, when the DEM fits 32-bit offsets into them, else L = 9 runs as L = 7).
+ * DEM, when the DEM fits 32-bit offsets into them, else L = 9 runs as L = 8).
  * Defaults: the fastest split layout per precision on one B200; rows 2x1 for
  * FP64 (the only layout it runs).  Results do not depend on any of them. */
 typedef struct tvs_sweep_config {

@@ -1,0 +1,71 @@
+"""The split sweep's two ways of adding surfaces (a plane per sector and
+direction, or in turn behind a wait) and its step loop's remainders, against
+each other and the oracle, bit for bit: every decision and every addition is
+the same, so no tolerance applies."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ORACLE_MODE = {"exact32": "exact32", "mixed64": "fp64", "fp32": "fp32"}
+IN_TURN = 0xFFFFFFFE  # no such tile: nothing is held, but the surfaces are added in turn
+
+
+def bits(a):
+    return np.ascontiguousarray(a).view(np.uint32)
+
+
+@pytest.mark.parametrize("precision", ["exact32", "mixed64", "fp32"])
+@pytest.mark.parametrize("w,h,los,rows", [(301, 301, 100, None), (340, 262, 87, (11, 77)),
+                                          (1201, 1201, 400, None)])
+def test_planes_equal_surfaces_added_in_turn(tvs, synth, precision, w, h, los, rows):
+    """1201^2 takes its 180 sectors in more than one launch."""
+    z = np.round(synth.fbm(w, h, 0.75, 3, 0.0, 1500.0))
+    with tvs.Engine(z, w, 30.0, los * 30, height=h, observer_height=1.65, precision=precision,
+                    rows=rows) as eng:
+        planes = eng.run()[:2]
+        eng.set_queue_wait(held_tile=IN_TURN)
+        turn = eng.run()[:2]
+    for a, b in zip(planes, turn):
+        assert np.array_equal(bits(a), bits(b))
+    assert planes[0].any()
+
+
+@pytest.mark.parametrize("precision", ["exact32", "mixed64", "fp32"])
+@pytest.mark.parametrize("los", [8, 11, 54, 56, 58, 60, 110, 112])
+def test_step_loop_remainders(tvs, oracle, synth, precision, los):
+    """Step counts around the loop's unit (2 or 4) and a segment (32), on a grid
+    whose last tiles are cut in both axes."""
+    w = 3 * los + 5
+    z = synth.fbm(w, w, 0.7, los, 0.0, 800.0)
+    g = oracle.geometry(w, 30.0, los * 30)
+    with tvs.Engine(z, w, 30.0, los * 30, observer_height=1.65, precision=precision) as eng:
+        for angle in (0, 38, 90, 141):
+            d, x, _ = oracle.compile_band_data(g, float(angle))
+            want = oracle.sweep_sector(g, z, 1.65, d, x, mode=ORACLE_MODE[precision])[0]
+            cum = np.zeros(eng.count, np.float32)
+            eng.compute_sector(angle, cum)
+            assert np.array_equal(bits(cum), bits(want.astype(np.float32))), angle
+
+
+@pytest.mark.parametrize("observer", [0.0, 1e-6, -2.0, 1.65, 300.0])
+def test_mixed64_guard_band_observer_heights(tvs, oracle, synth, observer):
+    """The guard band's part of the observer height, with the ties that it must
+    re-decide: a plane (every sample's angle the same but for the curvature),
+    whole-metre terrain and a flat sea."""
+    w, los = 160, 50
+    yy, xx = np.mgrid[0:w, 0:w].astype(np.float32)
+    plane = 3000.0 + 12.0 * xx + 7.0 * yy
+    metres = np.round(synth.fbm(w, w, 0.8, 5, 0.0, 90.0))
+    metres[:60] = 0.0
+    g = oracle.geometry(w, 30.0, los * 30)
+    for z in (plane, metres):
+        z = np.ascontiguousarray(z, np.float32)
+        with tvs.Engine(z, w, 30.0, los * 30, observer_height=observer, precision="mixed64") as eng:
+            for angle in (0, 27, 45, 90, 120):
+                d, x, _ = oracle.compile_band_data(g, float(angle))
+                want = oracle.sweep_sector(g, z, observer, d, x, mode="fp64")[0]
+                cum = np.zeros(eng.count, np.float32)
+                eng.compute_sector(angle, cum)
+                assert np.array_equal(bits(cum), bits(want.astype(np.float32))), (observer, angle)

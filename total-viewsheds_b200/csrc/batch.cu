@@ -33,7 +33,9 @@ struct tvs_batch {
     int32_t *d_error = nullptr;
     unsigned long long *d_rechecks = nullptr;
     uint32_t max_step_cap = 0;
-    uint32_t tiles_per_sector = 0;
+    uint32_t tiles_per_sector = 0, chunks = 0;
+    void *d_planes = nullptr;
+    size_t planes_cap = 0;
     tvs::QueueConfig cfg{0, 0, 0, 0, 0};
     bool dems_uploaded = false;
     cudaGraph_t graph = nullptr;
@@ -69,11 +71,29 @@ int upload_dems(tvs_batch *b) {
     std::vector<tvs::QueueDem> d(b->dems.size());
     for (size_t i = 0; i < d.size(); i++) d[i] = tvs_host::queue_dem_of(b->dems[i]);
     uint32_t done_total = 0;
-    tvs::queue_tile(d.data(), (uint32_t)d.size(), b->cfg, &b->tiles_per_sector, &done_total);
+    tvs::queue_tile(d.data(), (uint32_t)d.size(), b->cfg, &b->tiles_per_sector, &done_total,
+                    &b->chunks);
     if (done_total > b->done_cap) return bfail(b, TVS_ERR_CAPACITY, "batch tile counters");
     TVS_BCUDA(b, cudaMemcpy(b->d_dems, d.data(), d.size() * sizeof(tvs::QueueDem),
                             cudaMemcpyHostToDevice));
     b->dems_uploaded = true;
+    // the split sweep's surface planes (without memory for them it adds in turn)
+    uint32_t per = 0;
+    const size_t need = tvs::split_plane_bytes((int)b->precision, b->cfg, b->tiles_per_sector,
+                                               tvs::kSectorSteps, &per);
+    if (need > b->planes_cap) {
+        if (b->d_planes) cudaFree(b->d_planes);
+        b->device_bytes -= b->planes_cap;
+        b->d_planes = nullptr;
+        b->planes_cap = 0;
+        if (cudaMalloc(&b->d_planes, need) == cudaSuccess) {
+            b->planes_cap = need;
+            b->device_bytes += need;
+        } else {
+            cudaGetLastError();
+            b->d_planes = nullptr;
+        }
+    }
     return TVS_OK;
 }
 
@@ -84,6 +104,7 @@ tvs::QueueArgs queue_args(const tvs_batch *b, uint32_t first, uint32_t count) {
     q.first_sector = first;
     q.n_sectors = count;
     q.tiles_per_sector = b->tiles_per_sector;
+    q.chunks = b->chunks;
     q.max_step_cap = b->max_step_cap;
     q.queue = b->d_queue;
     q.done = b->d_done;
@@ -112,8 +133,16 @@ int enqueue_run(tvs_batch *b, uint32_t count) {
     if (cfg.layout == tvs::kQuadLayout)
         for (const tvs_context *c : b->dems)
             if (!c->d_quad) cfg.layout = tvs::kQuadFallback;
-    TVS_BCUDA(b, tvs::launch_sweep_queue(queue_args(b, 0, count), (int)b->precision, cfg,
-                                         b->stream));
+    uint32_t per = count;  // sectors per launch
+    tvs::QueueArgs q = queue_args(b, 0, count);
+    const size_t planes = tvs::split_plane_bytes((int)b->precision, b->cfg, b->tiles_per_sector, count, &per);
+    if (planes != 0 && planes <= b->planes_cap) q.planes = b->d_planes;
+    else per = count;
+    for (uint32_t s = 0; s < count; s += per) {
+        q.first_sector = s;
+        q.n_sectors = std::min(per, count - s);
+        TVS_BCUDA(b, tvs::launch_sweep_queue(q, (int)b->precision, cfg, b->stream));
+    }
     return TVS_OK;
 }
 
@@ -162,8 +191,7 @@ int tvs_batch_create(const tvs_params *params, const float *const *elevations, u
     struct { void **p; size_t bytes; } allocs[] = {
         {(void **)&b->d_shape, n_dems * sizeof(tvs::ShapeArgs)},
         {(void **)&b->d_dems, n_dems * sizeof(tvs::QueueDem)},
-        {(void **)&b->d_queue, sizeof(uint32_t)},
-        {(void **)&b->d_done, (size_t)b->done_cap * sizeof(uint32_t)},
+        {(void **)&b->d_queue, ((size_t)b->done_cap + 1) * sizeof(uint32_t)},
         {(void **)&b->d_error, sizeof(int32_t)},
         {(void **)&b->d_rechecks, sizeof(unsigned long long)},
     };
@@ -171,6 +199,7 @@ int tvs_batch_create(const tvs_params *params, const float *const *elevations, u
         if (e == cudaSuccess) e = cudaMalloc(a.p, a.bytes);
         if (e == cudaSuccess) b->device_bytes += a.bytes;
     }
+    b->d_done = b->d_queue + 1;
     if (e == cudaSuccess)
         e = cudaMemcpy(b->d_shape, sa.data(), n_dems * sizeof(tvs::ShapeArgs), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(b->d_error, 0, sizeof(int32_t));
@@ -199,7 +228,8 @@ void tvs_batch_destroy(tvs_batch *b) {
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     drop_graph(b);
-    void *ptrs[] = {b->d_shape, b->d_dems, b->d_queue, b->d_done, b->d_error, b->d_rechecks};
+    void *ptrs[] = {b->d_shape, b->d_dems, b->d_queue, b->d_error, b->d_rechecks,
+                    b->d_planes};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (b->stream) cudaStreamDestroy(b->stream);

@@ -142,12 +142,12 @@ void drop_tvs_graph(tvs_context *c) {
 
 void free_all(tvs_context *c) {
     void *ptrs[] = {c->d_elev, c->d_cum, c->d_total, c->d_cum64, c->d_trig, c->d_hdr,
-                    c->d_steps, c->d_offs, c->d_dtab, c->d_queue, c->d_done, c->d_error, c->d_hmax,
+                    c->d_steps, c->d_offs, c->d_dtab, c->d_quads, c->d_segs, c->d_queue, c->d_error, c->d_hmax,
                     c->d_rechecks, c->d_qdem,
                     c->d_deltas, c->d_dists, c->d_rings, c->d_spill, c->d_counters, c->d_sf,
                     c->d_sb, c->d_tab_deltas, c->d_tab_dists, c->d_installed,
                     c->d_rc_blocks, c->d_rc_offsets, c->d_rc_ids, c->d_bmax, c->d_qdem_rings,
-                    c->d_diag, c->d_quad};
+                    c->d_diag, c->d_quad, c->d_planes};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     drop_tvs_graph(c);
@@ -178,6 +178,10 @@ tvs::ShapeArgs shape_args(tvs_context *c, uint32_t first_slot) {
     a.dtab = c->d_dtab + (uint64_t)first_slot * c->step_cap;
     a.deltas = c->d_deltas + (uint64_t)first_slot * c->g.band_deltas_size;
     a.dists = c->d_dists + (uint64_t)first_slot * c->g.band_deltas_size;
+    a.quads = c->d_quads + (uint64_t)first_slot * c->step_cap;
+    a.segs = c->d_segs + (uint64_t)first_slot * tvs::seg_count(c->step_cap);
+    a.rho = (c->row_begin + c->g.max_los_as_points) & 3u;
+    a.quad_copy = tvs::quad_copy_elems(c->g.width, c->g.height);
     return a;
 }
 
@@ -327,6 +331,8 @@ tvs::QueueDem queue_dem(const tvs_context *c) {
     d.steps = c->d_steps;
     d.offs = c->d_offs;
     d.dtab = c->d_dtab;
+    d.quads = c->d_quads;
+    d.segs = c->d_segs;
     d.cumulative = c->d_cum;
     d.total = c->d_total;
     d.cumulative64 = c->d_cum64;
@@ -348,7 +354,7 @@ int upload_queue_dem(tvs_context *c) {
     if (q.px == u.px && q.py == u.py && q.layout == u.layout) return TVS_OK;
     tvs::QueueDem d = queue_dem(c);
     uint32_t done_total = 0;
-    tvs::queue_tile(&d, 1, q, &c->q_tiles_per_sector, &done_total);
+    tvs::queue_tile(&d, 1, q, &c->q_tiles_per_sector, &done_total, &c->q_chunks);
     TVS_CUDA(c, cudaMemcpyAsync(c->d_qdem, &d, sizeof d, cudaMemcpyHostToDevice, c->stream));
     c->qcfg_uploaded = q;
     return TVS_OK;
@@ -357,12 +363,14 @@ int upload_queue_dem(tvs_context *c) {
 // The queue descriptor of this context tiled for the ring sweep's split
 // layout: the context's own when its configuration is a split layout, else
 // one for the precision's default split layout.
-int ring_queue_dem(tvs_context *c, const tvs::QueueDem **dem, uint32_t *tiles, int *layout) {
+int ring_queue_dem(tvs_context *c, const tvs::QueueDem **dem, uint32_t *tiles, uint32_t *chunks,
+                   int *layout) {
     if (c->qcfg.layout != 0) {
         int rc = upload_queue_dem(c);
         if (rc) return rc;
         *dem = c->d_qdem;
         *tiles = c->q_tiles_per_sector;
+        *chunks = c->q_chunks;
         *layout = c->qcfg.layout;
         return TVS_OK;
     }
@@ -372,14 +380,40 @@ int ring_queue_dem(tvs_context *c, const tvs::QueueDem **dem, uint32_t *tiles, i
         c->device_bytes += sizeof(tvs::QueueDem);
         tvs::QueueDem d = queue_dem(c);
         uint32_t done_total = 0;
-        tvs::queue_tile(&d, 1, q, &c->q_ring_tiles, &done_total);
+        tvs::queue_tile(&d, 1, q, &c->q_ring_tiles, &done_total, &c->q_ring_chunks);
         TVS_CUDA(c, cudaMemcpy(c->d_qdem_rings, &d, sizeof d, cudaMemcpyHostToDevice));
         c->ring_layout = (uint32_t)q.layout;
     }
     *dem = c->d_qdem_rings;
     *tiles = c->q_ring_tiles;
+    *chunks = c->q_ring_chunks;
     *layout = (int)c->ring_layout;
     return TVS_OK;
+}
+
+// The split sweep's surface planes for a sweep of n_sectors and the sectors that
+// each of its launches takes; null (and every sector) where it adds the surfaces
+// in turn: a held tile of the failure test, or no memory for the planes.
+void *ensure_planes(tvs_context *c, const tvs::QueueConfig &q, uint32_t tiles, uint32_t n_sectors,
+                    uint32_t *sectors) {
+    const size_t need = tvs::split_plane_bytes((int)c->p.precision, q, tiles, n_sectors, sectors);
+    if (need != 0 && c->held_tile == 0xFFFFFFFFu) {
+        if (need <= c->planes_cap) return c->d_planes;
+        if (c->d_planes) cudaFree(c->d_planes);
+        c->device_bytes -= c->planes_cap;
+        c->d_planes = nullptr;
+        c->planes_cap = 0;
+        drop_tvs_graph(c);  // a captured sweep holds the old planes
+        if (cudaMalloc(&c->d_planes, need) == cudaSuccess) {
+            c->planes_cap = need;
+            c->device_bytes += need;
+            return c->d_planes;
+        }
+        cudaGetLastError();
+        c->d_planes = nullptr;
+    }
+    *sectors = n_sectors;
+    return nullptr;
 }
 
 // Sweep sectors [first, first+count) (slots == angles).  ring_slots != 0:
@@ -429,16 +463,20 @@ int enqueue_sweep(tvs_context *c, uint32_t first, uint32_t count, uint32_t ring_
     if (rings && c->p.precision != TVS_PRECISION_FP64 && impl == SweepImpl::Queue) {
         // ring records from the direction-split sweep itself
         const tvs::QueueDem *dem = nullptr;
-        uint32_t tiles = 0;
+        uint32_t tiles = 0, chunks = 0;
         int layout = 0;
-        int rc = ring_queue_dem(c, &dem, &tiles, &layout);
+        int rc = ring_queue_dem(c, &dem, &tiles, &chunks, &layout);
         if (rc) return rc;
+        const tvs::QueueConfig cfg{tvs::kSplitPoints, 1, 0, 0, layout};
         tvs::QueueArgs q{};
         q.dems = dem;
         q.n_dems = 1;
         q.first_sector = first;
         q.n_sectors = count;
         q.tiles_per_sector = tiles;
+        q.chunks = chunks;
+        uint32_t per = count;  // sectors per launch
+        q.planes = ensure_planes(c, cfg, tiles, count, &per);
         q.max_step_cap = c->step_cap;
         q.queue = c->d_queue;
         q.done = c->d_done;
@@ -456,9 +494,14 @@ int enqueue_sweep(tvs_context *c, uint32_t first, uint32_t count, uint32_t ring_
         q.spill = c->d_spill;
         q.spill_cap = c->spill_cap;
         q.ring_counters = c->d_counters;
-        TVS_CUDA(c, tvs::launch_sweep_split(q, (int)c->p.precision, runnable_layout(c, layout),
-                                            c->stream));
-        c->launches++;
+        q.first_record_sector = first;
+        for (uint32_t s = first; s < first + count; s += per) {
+            q.first_sector = s;
+            q.n_sectors = std::min(per, first + count - s);
+            TVS_CUDA(c, tvs::launch_sweep_split(q, (int)c->p.precision, runnable_layout(c, layout),
+                                                c->stream));
+            c->launches++;
+        }
         return TVS_OK;
     }
     if (!rings && impl == SweepImpl::Queue) {
@@ -470,6 +513,9 @@ int enqueue_sweep(tvs_context *c, uint32_t first, uint32_t count, uint32_t ring_
         q.first_sector = first;
         q.n_sectors = count;
         q.tiles_per_sector = c->q_tiles_per_sector;
+        q.chunks = c->q_chunks;
+        uint32_t per = count;  // sectors per launch
+        q.planes = ensure_planes(c, c->qcfg, c->q_tiles_per_sector, count, &per);
         q.max_step_cap = c->step_cap;
         q.queue = c->d_queue;
         q.done = c->d_done;
@@ -482,8 +528,12 @@ int enqueue_sweep(tvs_context *c, uint32_t first, uint32_t count, uint32_t ring_
         q.diag = c->diag_on ? c->d_diag : nullptr;
         tvs::QueueConfig cfg = c->qcfg;
         cfg.layout = runnable_layout(c, cfg.layout);
-        TVS_CUDA(c, tvs::launch_sweep_queue(q, (int)c->p.precision, cfg, c->stream));
-        c->launches++;
+        for (uint32_t s = first; s < first + count; s += per) {
+            q.first_sector = s;
+            q.n_sectors = std::min(per, first + count - s);
+            TVS_CUDA(c, tvs::launch_sweep_queue(q, (int)c->p.precision, cfg, c->stream));
+            c->launches++;
+        }
         return TVS_OK;
     }
     if (!rings && impl == SweepImpl::Const && c->p.precision == TVS_PRECISION_EXACT32 &&
@@ -708,8 +758,9 @@ int tvs_create(const tvs_params *params, const float *elevations, uint64_t n_ele
         {(void **)&c->d_steps, (size_t)slots * c->step_cap * sizeof(float4)},
         {(void **)&c->d_offs, (size_t)slots * c->step_cap * sizeof(int2)},
         {(void **)&c->d_dtab, (size_t)slots * c->step_cap * sizeof(double4)},
-        {(void **)&c->d_queue, sizeof(uint32_t)},
-        {(void **)&c->d_done, (size_t)std::max<uint32_t>(c->done_cap, 1) * sizeof(uint32_t)},
+        {(void **)&c->d_quads, (size_t)slots * c->step_cap * sizeof(int2)},
+        {(void **)&c->d_segs, (size_t)slots * tvs::seg_count(c->step_cap) * sizeof(int4)},
+        {(void **)&c->d_queue, ((size_t)c->done_cap + 1) * sizeof(uint32_t)},
         {(void **)&c->d_error, sizeof(int32_t)},
         {(void **)&c->d_hmax, sizeof(float)},
         {(void **)&c->d_bmax, (size_t)std::max<uint64_t>((uint64_t)c->bmax_w * c->bmax_h, 1) * sizeof(float)},
@@ -723,6 +774,7 @@ int tvs_create(const tvs_params *params, const float *elevations, uint64_t n_ele
         if ((e = cudaMalloc(a.p, a.bytes)) != cudaSuccess) return bail(e, "cudaMalloc");
         c->device_bytes += a.bytes;
     }
+    c->d_done = c->d_queue + 1;
     if (params->precision == TVS_PRECISION_MIXED64 || params->precision == TVS_PRECISION_FP64) {
         if ((e = cudaMalloc(&c->d_cum64, count * sizeof(double))) != cudaSuccess)
             return bail(e, "cudaMalloc");

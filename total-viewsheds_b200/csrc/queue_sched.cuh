@@ -26,40 +26,36 @@ constexpr int kQueueTileX = 32;
 constexpr int kQueueTileY = TVS_QUEUE_WARPS;
 constexpr int kQueueThreads = kQueueTileX * kQueueTileY;
 
+// Warps per CTA of the split sweep and warp tiles per chunk of its queue.
+constexpr int kSplitWarps = 16;
+constexpr uint32_t kSplitChunk = kSplitWarps;
+// The split sweep's launches take as many sectors as have planes of surfaces
+// (one per sector and direction) of about this size.
+constexpr size_t kPlaneBytes = (size_t)256 << 20;
+
 // Direction-split layouts 1-9: a warp holds LX columns x 32/LX rows of lanes;
 // each lane sweeps four points of view, LX columns apart (layouts 1-3: LX = 8,
 // 16, 32), 2 x 2 of them, LX columns and 32/LX rows apart (layouts 4-6), or
 // four rows 32/LX apart in one column (layouts 7, 8: LX = 32, 16), so that one
-// load of the warp reads whole 128- or 64-byte rows.  Layout 9 (quad) is
-// layout 7's tiling with the four rows read as one float4 from the DEM's
-// row-interleaved copies: a warp's load is 512 contiguous bytes.
+// load of the warp reads whole 128- or 64-byte rows.  Layout 9 (quad) is layout
+// 8's 16 x 8 tile, a lane's four rows consecutive and read as one float4 from the
+// DEM's row-interleaved copies: a warp's load is two runs of 256 bytes.  (Against
+// a 32 x 4 tile the runs of one step meet the next one's again: 8.1 in place of
+// 12.3 new sectors a step, and a small grid wastes fewer lanes at its edges; 1201^2
+// exact f32 3.95 -> 3.72 ms.)  The tile of the split sweep's queue is one warp's
+// 128 points of view.
 constexpr int kSplitCols = 4;  // points of view per lane
 constexpr int kSplitLayouts = 9;
 __host__ __device__ constexpr int split_lx(int layout) {
-    return layout == 7 || layout == 9 ? 32 : layout == 8 ? 16 : 4 << ((layout - 1) % 3 + 1);
+    return layout == 7 ? 32 : layout >= 8 ? 16 : 4 << ((layout - 1) % 3 + 1);
 }
 __host__ __device__ constexpr int split_ky(int layout) { return layout > 6 ? 4 : layout > 3 ? 2 : 1; }
 __host__ __device__ constexpr int split_tile_w(int layout) {
     return kSplitCols / split_ky(layout) * split_lx(layout);
 }
 __host__ __device__ constexpr int split_tile_h(int layout) {
-    return kQueueTileY * (32 / split_lx(layout)) * split_ky(layout);
+    return 32 / split_lx(layout) * split_ky(layout);
 }
-
-// Segments of the direction-split fast loop: kSegSteps steps whose samples are
-// bounded together.  Per segment: the range of the forward DEM offsets (x, y)
-// over its steps, the largest and smallest 1/d and the largest first-test
-// offset.
-#ifndef TVS_SEG_STEPS
-#define TVS_SEG_STEPS 32
-#endif
-constexpr uint32_t kSegSteps = TVS_SEG_STEPS;
-static_assert(kSegSteps >= 1 && kSegSteps <= 32,
-              "the staging reduces one segment per warp, one step per lane");
-struct __align__(16) SegBound {
-    int dx0, dx1, dy0, dy1;
-    float ymax, ymin, zmax, pad;
-};
 
 struct QueueCtl {
     QueueDem dem;           // the current item's DEM (copied from the descriptor array)
@@ -72,9 +68,7 @@ struct QueueCtl {
     uint32_t n_steps;
     uint32_t n_fast;
     bool restage;
-    bool plain;             // quad layout: the staged sector reads the plain DEM
     float hmax;             // the staged DEM's elevation range (estimate windows)
-    unsigned long long diag[4];  // per-item counters (sweep_split.cu), flushed per item
 };
 
 #ifdef __CUDACC__
@@ -148,9 +142,11 @@ __device__ __forceinline__ void queue_done(const QueueArgs &a, const QueueDem &D
 }
 #endif
 
-// Host: grid-wide launch of a persistent queue kernel: the shared-memory
-// attribute (only ever raised) and the occupancy are kept per (kernel, device)
-// under a lock; the queue and tile counters are reset on the stream first.
-cudaError_t launch_persistent(const void *fn, const QueueArgs &a, size_t smem, cudaStream_t s);
+// Host: launch of a persistent queue kernel over `items` work items: the
+// shared-memory attribute (only ever raised) and the occupancy are kept per
+// (kernel, device) under a lock; the queue and tile counters are reset on the
+// stream first.
+cudaError_t launch_persistent(const void *fn, const QueueArgs &a, uint64_t items, dim3 block,
+                              size_t smem, cudaStream_t s, uint32_t n_slots = 0);
 
 }  // namespace tvs

@@ -22,6 +22,8 @@
 //
 // Every projection is rounded op by op (__dmul_rn/__dsub_rn), with host glibc
 // sin/cos, so keys are bitwise those of the reference.
+#include <climits>
+
 #include "tvs.h"
 #include "tvs_internal.cuh"
 
@@ -131,11 +133,22 @@ __device__ void block_inclusive_scan(long long *v, uint32_t n, long long *scratc
     __syncthreads();
 }
 
+// The forward and backward offset of a step in the quad copies, in float4, from
+// a lane's base (copy 0, the group of its first row, its column): rows r0 + y ..
+// +3 sit in copy (rho + y) mod 4, rho = r0 mod 4 (r0 = the lane's first row).
+__device__ __forceinline__ int2 quad_offsets(long long dx, long long dy, long long W, long long rho,
+                                             long long copy) {
+    const long long cf = (rho + dy) & 3, cb = (rho - dy) & 3;
+    return make_int2((int)(cf * copy + (rho + dy - cf) / 4 * W + dx),
+                     (int)(cb * copy + (rho - dy - cb) / 4 * W - dx));
+}
+
 struct ShapeSmem {
     unsigned long long red[64];
     long long scan[kShapeThreads];
     uint32_t n_cand;
     int32_t status;
+    uint32_t n_surf, wide;
 };
 
 }  // namespace
@@ -150,6 +163,8 @@ __device__ void finish_shape(const ShapeArgs &a, uint32_t sector, uint32_t n_fil
     ShapeHeader *hdr = a.hdr + sector;
     long long mn = 0, mx = 0;
     uint32_t first_slow = n_steps;
+    if (threadIdx.x == 0) sm.n_surf = sm.wide = 0;
+    __syncthreads();
     float4 *gsteps = a.steps + (uint64_t)sector * a.step_cap;
     int2 *goffs = a.offs + (uint64_t)sector * a.step_cap;
     for (uint32_t i = threadIdx.x; i < n_steps; i += blockDim.x) {
@@ -168,6 +183,15 @@ __device__ void finish_shape(const ShapeArgs &a, uint32_t sector, uint32_t n_fil
         mn = min(mn, off);
         mx = max(mx, off);
         if (flags) first_slow = min(first_slow, i);
+        if (d != 0.0f) atomicMax(&sm.n_surf, i + 1);
+        if (a.quads) {
+            long long dx, dy;
+            step_xy(off, a.width, dx, dy);
+            a.quads[(uint64_t)sector * a.step_cap + i] =
+                quad_offsets(dx, dy, a.width, a.rho, (long long)a.quad_copy);
+            const long long los = (long long)a.band_size - 1;
+            if (dx > los || dx < -los) sm.wide = 1;
+        }
     }
     __syncthreads();
     sm.scan[threadIdx.x] = first_slow;
@@ -178,6 +202,22 @@ __device__ void finish_shape(const ShapeArgs &a, uint32_t sector, uint32_t n_fil
     }
     const uint32_t n_fast = (uint32_t)sm.scan[0];
     __syncthreads();
+    // the offset range of each segment of fast steps, one warp per segment
+    if (a.segs) {
+        const uint32_t lane = threadIdx.x & 31u;
+        for (uint32_t sg = threadIdx.x >> 5; sg * kSegSteps < n_fast; sg += blockDim.x >> 5) {
+            const uint32_t i = sg * kSegSteps + lane;
+            const bool v = lane < kSegSteps && i < n_fast;
+            long long dx, dy;
+            step_xy(v ? (i < n_filled ? soff[i] : soff[n_filled - 1]) : 0, a.width, dx, dy);
+            const int x0 = __reduce_min_sync(0xffffffffu, v ? (int)dx : INT_MAX);
+            const int x1 = __reduce_max_sync(0xffffffffu, v ? (int)dx : INT_MIN);
+            const int y0 = __reduce_min_sync(0xffffffffu, v ? (int)dy : INT_MAX);
+            const int y1 = __reduce_max_sync(0xffffffffu, v ? (int)dy : INT_MIN);
+            if (lane == 0)
+                a.segs[(uint64_t)sector * seg_count(a.step_cap) + sg] = make_int4(x0, x1, y0, y1);
+        }
+    }
     // block min / max through the scan scratch
     sm.scan[threadIdx.x] = mn;
     __syncthreads();
@@ -207,7 +247,10 @@ __device__ void finish_shape(const ShapeArgs &a, uint32_t sector, uint32_t n_fil
         hdr->min_off = min_off;
         hdr->max_off = max_off;
         hdr->n_fast = n_fast;
-    }}
+        hdr->n_surf = sm.n_surf;
+        hdr->wide = sm.wide;
+    }
+}
 
 // One sector of one DEM (the whole CTA).
 __device__ __forceinline__ void shape_sector(const ShapeArgs &a, const uint32_t sector,

@@ -577,15 +577,15 @@ k_sweep_queue(QueueArgs a) {
 template <int kPrec, int kPx, int kPy, int kVar>
 cudaError_t launch_queue_t(const QueueArgs &a, size_t smem, cudaStream_t s) {
     return launch_persistent(reinterpret_cast<const void *>(&k_sweep_queue<kPrec, kPx, kPy, kVar>),
-                             a, smem, s);
+                             a, (uint64_t)a.tiles_per_sector * a.n_sectors,
+                             dim3(kTileX, kTileY), smem, s);
 }
 
 }  // namespace
 
 uint32_t queue_tiles_bound(uint32_t tvs_width, uint32_t rows) {
     // the most tiles any configuration cuts: the row layouts' smallest tile is
-    // 32 x 8, but a split layout's tile can be narrower (16 x 64), which on a
-    // thin row shard gives more tiles
+    // 32 x 8, a split layout's is one warp's (128 points in one of several shapes)
     auto tiles = [&](uint32_t w, uint32_t h) { return ((tvs_width + w - 1) / w) * ((rows + h - 1) / h); };
     uint32_t n = tiles(kTileX, kTileY);
     for (int l = 1; l <= kSplitLayouts; l++) n = std::max(n, tiles(split_tile_w(l), split_tile_h(l)));
@@ -630,7 +630,7 @@ QueueConfig default_split_config(int precision) {
         const int v = l ? atoi(l) : d;
         return v >= 1 && v <= kSplitLayouts ? v : d;
     };
-    static const int mix = env_layout("TVS_SWEEP_LAYOUT", 1);
+    static const int mix = env_layout("TVS_SWEEP_LAYOUT", kQuadLayout);
     static const int exact = env_layout("TVS_SWEEP_LAYOUT32", kQuadLayout);
     static const int fp32 = env_layout("TVS_SWEEP_LAYOUT_FP32", kQuadLayout);
     const int l = precision == TVS_PRECISION_MIXED64 ? mix
@@ -640,8 +640,8 @@ QueueConfig default_split_config(int precision) {
 }
 
 void queue_tile(QueueDem *dems, uint32_t n_dems, const QueueConfig &c, uint32_t *tiles_per_sector,
-                uint32_t *done_total) {
-    uint32_t base = 0;
+                uint32_t *done_total, uint32_t *chunks) {
+    uint32_t base = 0, chunk_base = 0;
     for (uint32_t i = 0; i < n_dems; i++) {
         QueueDem &d = dems[i];
         const uint32_t rows = d.row_end - d.row_begin;
@@ -651,10 +651,17 @@ void queue_tile(QueueDem *dems, uint32_t n_dems, const QueueConfig &c, uint32_t 
         d.tiles_y = (rows + th - 1) / th;
         d.tile_base = base;
         d.done_base = base;
-        base += d.tiles_x * d.tiles_y;
+        const uint32_t tiles = d.tiles_x * d.tiles_y;
+        base += tiles;
+        // chunks of at most kSplitChunk tiles, of even size
+        const uint32_t n = (tiles + kSplitChunk - 1) / kSplitChunk;
+        d.chunk_base = chunk_base;
+        d.chunk = n ? (tiles + n - 1) / n : 1;
+        chunk_base += (tiles + d.chunk - 1) / d.chunk;
     }
     *tiles_per_sector = base;
     *done_total = base;
+    *chunks = chunk_base;
 }
 
 cudaError_t launch_sweep_queue(const QueueArgs &a, int precision, const QueueConfig &c,

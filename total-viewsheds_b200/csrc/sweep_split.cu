@@ -5,29 +5,51 @@
 // when its angle is above the maximum, visible samples add d*tan(1 deg) to
 // the band's surface and changes of visibility are ring events.
 //
-// Mapping.  A CTA sweeps one (sector, tile) item of the work queue
-// (queue_sched.cuh).  A warp holds LX columns x 32/LX rows of lanes and each
-// lane four points of view (chains), so a warp's 128 chains cover a compact
-// patch; the lane sweeps its four forward bands over every step, then its four
-// backward bands (the forward surfaces wait in shared memory).  Per step the
-// chains of a lane share one table entry and one address (the four samples
-// are load immediates apart).
+// Mapping.  A work item is one warp tile of one sector in one direction: a
+// warp holds LX columns x 32/LX rows of lanes and each lane four points of
+// view (chains), so a warp's 128 chains cover a compact patch.  Per step the
+// chains of a lane share one table entry and one address (in the quad layout
+// one 16-byte load gives all four samples).
+//
+// Scheduling.  The grid is the resident capacity of the GPU.  CTAs take chunks
+// of up to kSplitChunk tiles of one (sector, direction) from a global counter
+// in sector-major order; the warps of a CTA take the chunk's tiles one by one
+// and go on to the next chunk without waiting for each other: a ring of two or
+// three chunks with their step tables sits in shared memory, and the warp that
+// takes a chunk's last tile brings in the next chunk.  Segment skipping makes the
+// tiles' work uneven; with a barrier after every 8 tiles, as before, warps waited
+// for the slowest of their CTA and small DEMs for each other (301^2 exact f32:
+// 0.94 ms a sweep, now 0.18).
+//
+// Order.  Every point's surfaces are added sector by sector, forward before
+// backward (kernel.rs:254).  An item writes its surfaces to a plane of its own
+// (one per sector and direction of the launch; a launch takes as many sectors as
+// kPlaneBytes hold), and the last item of a tile adds the planes up in order.  So
+// no item waits, and only that last one needs an acquiring fence, which empties
+// the SM's L1.  (When every item added its surfaces in turn, behind a fence and
+// a wait for the tile's previous item, 37-48 % of the sectors hit L1 in place of
+// 72 %, and at 1201^2, where several sectors are under way at once, warps spent
+// half their time waiting.)  That way remains for a launch without planes (no
+// memory for them, or the failure test's held tile): a counter per tile, and a
+// bounded wait.
 //
 // Arithmetic.  Every step first forms the FP32 estimate of the angle from
-// the step's tables, a^ = e*y - c (e = RN(h - h_pov), y = RN(1/d),
-// c = RN(d/R)), with a per-step window G >= 4 x the estimate's error bound
-// (apart from its 2^-22 |a^| part, which the chain's window carries):
+// the step's tables, a^ = e*y - c (y = RN(1/d), c = RN(d/R)), with a per-step
+// window G above the estimate's error bound (apart from its part relative to
+// |a|, which the chain's window carries):
 //  * FP32 (the comparison form): the estimate is the angle, fma(e, y, -c).
-//  * EXACT32 / MIXED64: each chain keeps a window [lo, hi] around its running
-//    maximum's estimate and the step j of its maximum.  fma(e, y, -c + G) < lo
-//    proves the sample is not visible; fma(e, y, -c - G) > hi proves it is.
-//    Only between the two is the comparison re-decided exactly -- in the
-//    reference's f32 arithmetic (EXACT32, Markstein division from the table
-//    reciprocal) or in FP64 (MIXED64) -- against the exact maximum recomputed
-//    from step j.  So every decision is the exact one, and surfaces add the
-//    reference's w = RN(d*tan1) in f32 (EXACT32) or RN64(d*0.0174533) in
-//    double (MIXED64) in step order: bit for bit the reference f32 sweep and
-//    the all-FP64 sweep.
+//  * EXACT32: the running maximum is held exactly; fma(e, y, -c + G) < lo
+//    proves that a sample is not visible, and where a chain of the warp passes
+//    that test the reference's own f32 angle is evaluated (Markstein division
+//    from the table reciprocal).
+//  * MIXED64: each chain keeps the estimate mid of its running maximum, the half
+//    width hw of the band around it and the step j of the maximum.  f < mid - hw
+//    proves the sample is not visible, f > mid + hw that it is.  Only between the
+//    two is the comparison re-decided in FP64, against the exact maximum
+//    recomputed from step j.
+// So every decision is the exact one, and surfaces add the reference's
+// w = RN(d*tan1) in f32 (EXACT32) or RN64(d*0.0174533) in double (MIXED64) in
+// step order: bit for bit the reference f32 sweep and the all-FP64 sweep.
 // A warp skips a step when no chain can change state (the vote on the first
 // test), and a 32-step segment when the DEM's 16x16 block maxima over the
 // warp's patch, moved by the segment's offsets, bound every sample below
@@ -53,7 +75,9 @@ namespace tvs {
 namespace {
 
 constexpr int K = kSplitCols;     // chains per lane
-constexpr float kRel = 0x1p-19f;  // the chain window's part relative to |max|
+// Iterations of a wait for a chunk of the CTA's own ring (at least 64 ns each:
+// seconds, against a real wait of at most a few work items).
+constexpr uint32_t kRingSpinLimit = 1u << 26;
 
 __device__ __forceinline__ float div_table32(float e, float y, float d) {
     const float q = __fmul_rn(e, y);
@@ -67,366 +91,529 @@ __device__ __forceinline__ double div_table64(double e, double y, double d) {
     return __fma_rn(r, y, q);
 }
 
-// A step's forward DEM offset (cells) as (x, y): |x| < W/2 on every band of
-// sight, and |y| <= the line of sight (the shape stage's path check).
-__device__ __forceinline__ void step_xy(long long off, long long W, long long &dx, long long &dy) {
-    const long long q = off + W / 2;
-    dy = q >= 0 ? q / W : -((W - 1 - q) / W);
-    dx = off - dy * W;
+// Pairs of floats in one 64-bit register: sm_100's add.f32x2 rounds each half as
+// the scalar instruction does and takes one issue slot.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pk(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
 }
-
-// The quad layout's forward and backward byte offsets of a step from a lane's
-// base (copy 0, the group of its first row, its column): rows r0 + y .. +3
-// sit in copy (rho + y) mod 4, rho = r0 mod 4 (r0 = the lane's first row).
-__device__ __forceinline__ int2 quad_offsets(long long off, long long W, long long rho,
-                                             long long copy_bytes) {
-    long long dx, dy;
-    step_xy(off, W, dx, dy);
-    const long long cf = (rho + dy) & 3, cb = (rho - dy) & 3;
-    const long long fwd = cf * copy_bytes + (rho + dy - cf) / 4 * W * 16 + dx * 16;
-    const long long bwd = cb * copy_bytes + (rho - dy - cb) / 4 * W * 16 - dx * 16;
-    return make_int2((int)fwd, (int)bwd);
+__device__ __forceinline__ void upk(f32x2 v, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
-
-// The per-step window of exact f32: 2^-20 (d/R + hmax/d) plus a floor, as the
-// shape of the estimate's error bound 2^-22 (|a| + d/R + hmax/d) demands (the
-// |a| part travels with the chain's maximum).
-__device__ __forceinline__ float step_window(float y, float c, float hmax) {
-    return __fadd_rn(__fmul_rn(0x1p-20f, __fadd_rn(c, __fmul_rn(hmax, y))), 0x1p-90f);
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
 }
-
-// MIXED64's per-step window.  Its estimate takes e = RN(h - h_pov) and folds the
-// observer height o into the step's offset -(d/R + o/d), so that no rounding of
-// it is relative to the elevations themselves: against the real angle a,
-// |estimate - a| <= 2^-24 (3 |a| + 5 d/R + 6 |o|/d) from the roundings of e, 1/d,
-// the offset and the fma, and the FP64 angle adds 2^-53 (hmax/d + ...).  The
-// window 2^-20 (d/R + |o|/d) + 2^-44 hmax/d holds 2.6 x the absolute part of
-// that; kRelMix = 2^-20 of the maximum holds the 3 |a| of both the maximum and a
-// sample near it 2.6 x.  With h_pov + o rounded to f32 first the window was
-// 2^-20 hmax/d: on the sea of a 3601^2 tile with 4500 m peaks every sample past
-// 330 cells fell into it, 7.6e-4 of all samples were re-decided in FP64 and the
-// sweep took 141.8 ms.
-constexpr float kRelMix = 0x1p-20f;
-__device__ __forceinline__ float mix_window(float y, float c, float o, float hmax) {
+// MIXED64's guard band.  A sample's estimate f and the maximum's estimate mid (f at
+// the step j of the maximum) decide a comparison when they differ by more than
+//   hw = 2^-20 |mid| + W_j,   W_j = G_j + the largest G of the steps from j on,
+// where G is a step's bound on |f - angle| apart from its part relative to the
+// angle.  e = RN(h - h_pov), and the observer height o sits in the step's offset
+// z = -(d/R + o/d), so that no rounding is relative to the elevations themselves:
+// |f - a| <= 2^-24 (3 |a| + 5 d/R + 6 |o|/d) from the roundings of e, 1/d, z and
+// the fma, and the FP64 angle adds 2^-53 (hmax/d + ...).  G = 2^-20 (d/R + |o|/d) +
+// 2^-44 hmax/d + 2^-90 holds 2.6 x the absolute part, 2^-20 |mid| the 3 |a| of the
+// maximum and of a sample near it 2.6 x; the rounding of f - mid is 2^-24 of a
+// value that matters only near hw.  A NaN estimate decides nothing and is not
+// visible, as a > m is false for a NaN angle.  (With h_pov + o rounded to f32
+// first, the band was 2^-20 hmax/d: on the sea of a 3601^2 tile with 4500 m peaks
+// every sample past 330 cells fell into it and was re-decided, 7.6e-4 of all.)
+constexpr float kRel = 0x1p-20f;
+__device__ __forceinline__ float band_mix(float y, float c, float o, float hmax) {
     return __fadd_rn(__fadd_rn(__fmul_rn(0x1p-20f, __fadd_rn(c, __fmul_rn(fabsf(o), y))),
                                __fmul_rn(0x1p-44f, __fmul_rn(hmax, y))),
                      0x1p-90f);
 }
+// EXACT32's first test fma(e, y, -d/R + G) >= m - 2^-19 |m| passes every step where
+// a chain may change state: e is the reference's own RN(h - RN(h_pov + o)), and
+// |e y - d/R - a| <= 2^-24 (4 |a| + 3 d/R) from the roundings of 1/d, the fma and
+// the reference's division and subtraction.
+constexpr float kRelExact = 0x1p-19f;
+__device__ __forceinline__ float window_exact(float c) { return __fmaf_rn(0x1p-20f, c, 0x1p-90f); }
 
-template <int kPrec> struct SplitTypes;
-template <> struct SplitTypes<TVS_PRECISION_EXACT32> {
-    using S = float;   // surfaces
-    using X = float2;  // {d, RN(d/R)}: the exact re-decision
+// A step's entry of the table in shared memory: step i's constants are in entry
+// i + kAhead, and entry i holds where step i's samples are (next: of the step
+// kAhead steps later; the point of view itself past the last step), in floats of
+// the DEM or bytes of the quad copies.  One 16-byte read so gives a step its
+// constants and the address of the loads that run two steps ahead.
+constexpr uint32_t kAhead = 2;
+template <int kPrec> struct Step;
+template <> struct __align__(16) Step<TVS_PRECISION_EXACT32> {
+    float y, z, w;  // 1/d, -d/R + G, the surface addend
+    int next;
+    float d, c;     // the exact angle's d and d/R
+    float2 pad;
 };
-template <> struct SplitTypes<TVS_PRECISION_MIXED64> {
-    using S = double;
-    using X = double2;  // {RN64(d/R), RN64(d*0.0174533)}
+template <> struct __align__(16) Step<TVS_PRECISION_MIXED64> {
+    float y, z, band;  // 1/d, -(d/R + o/d), W
+    int next;
+    double w, pad;  // RN64(d*0.0174533)
 };
-template <> struct SplitTypes<TVS_PRECISION_FP32> {
-    using S = float;
-    using X = float2;  // unused
+template <> struct __align__(16) Step<TVS_PRECISION_FP32> {
+    float y, z, w;  // 1/d, -d/R, the surface addend
+    int next;
+};
+template <int kPrec>
+using Surface = typename std::conditional<kPrec == TVS_PRECISION_MIXED64, double, float>::type;
+
+// A segment's bounds in this direction: the range of the offsets and the
+// extremes of 1/d and of the first test's offset.
+struct __align__(16) SegBound {
+    int x0, x1, y0, y1;
+    float ymax, ymin, zmax, pad;
 };
 
-// MIXED64 comes in two forms (kLean).  Both keep the step of each chain's
-// maximum in registers, two 16-bit steps per register (TVS_MIX_JREG; written
-// at every raise, read only by the rare re-decisions).  The default stages
-// {RN64(d/R), RN64(d*0.0174533)} per step.  The lean form, for lines of sight
-// whose tables would leave fewer than three CTAs per SM, recomputes the
-// surface addend from the staged f32 d (one DMUL, the shape stage's own
-// operation) and reads RN64(d/R) for the rare exact re-decisions from the FP64
-// table in global memory.  Exact f32 holds its running maximum exactly, in
-// registers, and evaluates the reference's angle wherever the first test
-// passes.
-#ifndef TVS_EXACT_INLINE
-#define TVS_EXACT_INLINE 1
-#endif
-// MIXED64 re-decisions read RN64(1/d) from the shape stage's FP64 table
-// instead of recomputing it.
-#ifndef TVS_MIX_RCP_TABLE
-#define TVS_MIX_RCP_TABLE 0
-#endif
-// MIXED64 keeps the step of each chain's maximum in registers, two 16-bit
-// steps per register (band tables of up to 65535 steps; 0 keeps it in shared
-// memory instead, 4 B per chain).
-#ifndef TVS_MIX_JREG
-#define TVS_MIX_JREG 1
-#endif
+struct SplitSlot {
+    QueueDem dem;          // the chunk's DEM (copied from the descriptor array)
+    uint32_t group;        // 2 * sector of the launch + direction
+    uint32_t tile0, n_tiles;
+    uint32_t next;         // next tile of the chunk
+    uint32_t left;         // warps that have gone on to the next chunk
+    uint32_t end;          // the queue is empty: no chunk
+    uint32_t n, n_fast;    // steps, and steps of the table-division loop
+    int32_t status;        // the sector's shape status
+    uint32_t plain;        // quad layout: the sector reads the plain DEM
+};
 
-// Shared-memory layout of one CTA.  Every array starts on 16 bytes.
+struct SplitCtl {
+    uint32_t ready;              // chunks brought in so far
+    unsigned long long diag[4];  // counters, flushed at the end
+};
+
+// Shared memory of one CTA: the control block, then the slots of {chunk, step
+// table, segment bounds}.
 __host__ __device__ constexpr size_t align16(size_t n) { return (n + 15) & ~(size_t)15; }
 
-template <int kPrec, bool kLean = false> struct SplitSmem {
-    using S = typename SplitTypes<kPrec>::S;
-    using X = typename SplitTypes<kPrec>::X;
-    static constexpr bool kExactTab =
-        kPrec == TVS_PRECISION_EXACT32 || (kPrec == TVS_PRECISION_MIXED64 && !kLean);
-    __host__ __device__ static size_t ctl() { return 0; }
-    __host__ __device__ static size_t steps(uint32_t) { return align16(sizeof(QueueCtl)); }
-    __host__ __device__ static size_t boff(uint32_t cap) { return steps(cap) + align16((size_t)cap * 16); }
-    __host__ __device__ static size_t xtab(uint32_t cap) { return boff(cap) + align16((size_t)cap * 8); }
+template <int kPrec> struct SplitSmem {
+    __host__ __device__ static size_t slots() { return align16(sizeof(SplitCtl)); }
+    __host__ __device__ static size_t table() { return align16(sizeof(SplitSlot)); }
     __host__ __device__ static size_t seg(uint32_t cap) {
-        return xtab(cap) + (kExactTab ? align16((size_t)cap * sizeof(X)) : 0);
+        return table() + (size_t)(cap + kAhead) * sizeof(Step<kPrec>);
     }
-    __host__ __device__ static size_t fwd(uint32_t cap) {
-        return seg(cap) + align16((size_t)((cap + kSegSteps - 1) / kSegSteps) * sizeof(SegBound));
+    __host__ __device__ static size_t slot(uint32_t cap) {
+        return seg(cap) + (size_t)seg_count(cap) * sizeof(SegBound);
     }
-    __host__ __device__ static size_t jtab(uint32_t cap) {
-        return fwd(cap) + (size_t)K * kQueueThreads * sizeof(S);
-    }
-    __host__ __device__ static size_t total(uint32_t cap) {
-        return jtab(cap) + (kPrec == TVS_PRECISION_MIXED64 && !kLean && !TVS_MIX_JREG
-                                ? (size_t)K * kQueueThreads * sizeof(int32_t) : 0);
+    __host__ __device__ static size_t total(uint32_t cap, uint32_t n_slots) {
+        return slots() + n_slots * slot(cap);
     }
 };
 
-// Occupancy target: 4 CTAs of 256 threads per SM (64 registers a thread)
-// for the surface sweeps; ring output keeps more state and takes 3.
-#ifndef TVS_SPLIT_MIX_BLOCKS
-#define TVS_SPLIT_MIX_BLOCKS 4
-#endif
-#ifndef TVS_SPLIT_BLOCKS32
-#define TVS_SPLIT_BLOCKS32 4
-#endif
-#ifndef TVS_SPLIT_RING_BLOCKS
-#define TVS_SPLIT_RING_BLOCKS 3
-#endif
-#ifndef TVS_SPLIT_RING_BLOCKS32
-#define TVS_SPLIT_RING_BLOCKS32 3
-#endif
-template <int kPrec, bool kRings>
-constexpr int split_min_blocks() {
-    return (kPrec == TVS_PRECISION_MIXED64 ? (kRings ? TVS_SPLIT_RING_BLOCKS : TVS_SPLIT_MIX_BLOCKS)
-                                           : (kRings ? TVS_SPLIT_RING_BLOCKS32 : TVS_SPLIT_BLOCKS32)) *
-           8 / kQueueTileY;
+// Warps per CTA and CTAs per SM: 32 warps of 64 registers a thread for the surface
+// sweeps; ring output keeps more state (24 warps of 80 registers).  24 warps of 80
+// registers measured slower for the surfaces too (1201^2 exact f32 5.03 against
+// 4.38 ms): the step loop hides its loads with warps.
+constexpr int kRingWarps = 8;
+template <bool kRings> __host__ __device__ constexpr int split_warps() {
+    return kRings ? kRingWarps : kSplitWarps;
+}
+template <bool kRings> __host__ __device__ constexpr int split_min_blocks() {
+    return (kRings ? 24 : 32) / split_warps<kRings>();
 }
 
-// Unroll factors of the step loops (FP32 4, exact f32 4, MIXED64 1: the
-// fastest on one B200 at 3601^2 within the register budget).
-#ifndef TVS_SPLIT_UNROLL32
-#define TVS_SPLIT_UNROLL32 4
-#endif
-#ifndef TVS_SPLIT_UNROLL_EXACT
-#define TVS_SPLIT_UNROLL_EXACT 4
-#endif
-#ifndef TVS_SPLIT_UNROLL_MIX
-#define TVS_SPLIT_UNROLL_MIX 1
-#endif
-#define TVS_PRAGMA(x) _Pragma(#x)
-#define TVS_UNROLL(n) TVS_PRAGMA(unroll n)
+__device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
+    uint32_t v;
+    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];"
+                 : "=r"(v) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release(uint32_t *p, uint32_t v) {
+    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;"
+                 :: "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t add_release(uint32_t *p, uint32_t v) {
+    uint32_t old;
+    asm volatile("atom.release.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+    return old;
+}
+__device__ __forceinline__ void red_release(uint32_t *p, uint32_t v) {
+    asm volatile("red.release.cta.shared::cta.add.u32 [%0], %1;"
+                 :: "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(v) : "memory");
+}
 
-template <int kPrec, int kLayout, bool kRings, bool kLean>
-__global__ void __launch_bounds__(kQueueThreads, (split_min_blocks<kPrec, kRings>()))
-k_sweep_split(QueueArgs a) {
+// A visible sample's state change, spelled with predicates: the compiler would
+// turn it into a branch and its reconvergence.  The FP32 form: the surface gains
+// w, the maximum moves to the angle (false for a NaN: the maximum stays, as
+// f32::max has it).
+__device__ __forceinline__ void raise_fp32(float ang, float &m, float &s, float w) {
+    asm("{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.gt.f32 p, %2, %0;\n\t"
+        "@p add.rn.f32 %1, %1, %3;\n\t"
+        "@p mov.f32 %0, %2;\n\t"
+        "}"
+        : "+f"(m), "+f"(s)
+        : "f"(ang), "f"(w));
+}
+// EXACT32: also the first test's threshold lo = m - 2^-19 |m|.
+__device__ __forceinline__ void raise_exact(float ang, float &m, float &s, float &lo, float w) {
+    asm("{\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .f32 t;\n\t"
+        "setp.gt.f32 p, %3, %0;\n\t"
+        "abs.f32 t, %3;\n\t"
+        "@p add.rn.f32 %1, %1, %4;\n\t"
+        "@p fma.rn.f32 %2, t, %5, %3;\n\t"
+        "@p mov.f32 %0, %3;\n\t"
+        "}"
+        : "+f"(m), "+f"(s), "+f"(lo)
+        : "f"(ang), "f"(w), "f"(-kRelExact));
+}
+// MIXED64, where x = f - mid >= -hw: mid = f (kept negated; computed again, for a
+// predicated multiply-add goes to the FMA pipe and a predicated move to the busier
+// ALU), hw = 2^-20 |f| + band, the surface gains w, and j's half kHi becomes step.
+template <int kHi>
+__device__ __forceinline__ void raise_mix(float x, float f, float e, float y, float z, float band,
+                                          uint32_t step, double w, float &nmid, float &hw,
+                                          uint32_t &j, double &acc) {
+    asm("{\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .f32 a, n;\n\t"
+        "neg.f32 n, %1;\n\t"
+        "setp.ge.f32 p, %4, n;\n\t"
+        "abs.f32 a, %5;\n\t"
+        "neg.f32 n, %6;\n\t"
+        "@p fma.rn.f32 %1, a, %12, %9;\n\t"
+        "neg.f32 a, %8;\n\t"
+        "@p fma.rn.f32 %0, n, %7, a;\n\t"
+        "@p add.rn.f64 %3, %3, %11;\n\t"
+        "@p prmt.b32 %2, %2, %10, %13;\n\t"
+        "}"
+        : "+f"(nmid), "+f"(hw), "+r"(j), "+d"(acc)
+        : "f"(x), "f"(f), "f"(e), "f"(y), "f"(z), "f"(band), "r"(step), "d"(w), "f"(kRel),
+          "n"(kHi ? 0x5410 : 0x3254));
+}
+
+// A value that every lane holds, in a uniform register: the branches and shared
+// memory addresses that follow from it need no per-lane registers.
+__device__ __forceinline__ uint32_t uni(uint32_t v) { return __reduce_max_sync(0xffffffffu, v); }
+
+// MIXED64's exact decision (kernel.rs:175-190 in double, from the shape stage's
+// table): is the angle of the sample h at step i above the one of hj at step j
+// (-2000 while j < 0)?  Kept out of line: it runs for about one sample in 10^5 and
+// its registers would crowd the loop.
+__device__ __forceinline__ double mix_angle(float h, float pov, float observer, const double4 *dtab,
+                                            uint32_t i) {
+    const double y = __ldg(&dtab[i].x), c = __ldg(&dtab[i].y), d = __ldg(&dtab[i].w);
+    const double hp = __dadd_rn((double)pov, (double)observer);
+    return __dsub_rn(div_table64(__dsub_rn((double)h, hp), y, d), c);
+}
+__device__ __noinline__ bool mix_visible(float h, float hj, float pov, float observer,
+                                         const double4 *dtab, uint32_t i, int32_t j) {
+    const double m = j < 0 ? (double)kMaxAngle : mix_angle(hj, pov, observer, dtab, (uint32_t)j);
+    return mix_angle(h, pov, observer, dtab, i) > m;
+}
+template <int kPrec, int kLayout, bool kRings>
+__global__ void __launch_bounds__(32 * split_warps<kRings>(), (split_min_blocks<kRings>()))
+k_sweep_split(QueueArgs a, uint32_t n_slots) {
     constexpr int LX = split_lx(kLayout), KY = split_ky(kLayout), KX = K / KY, LY = 32 / LX;
+    // rows between a lane's chains: the quad layout reads four consecutive ones
+    constexpr int RS = kLayout == kQuadLayout ? 1 : LY, LS = kLayout == kQuadLayout ? KY : 1;
+    constexpr int kWarps = split_warps<kRings>();
     constexpr bool kFp32 = kPrec == TVS_PRECISION_FP32;
     constexpr bool kMix = kPrec == TVS_PRECISION_MIXED64;
     constexpr bool kQuad = kLayout == kQuadLayout;
-    using L = SplitSmem<kPrec, kLean>;
-    using S = typename L::S;
-    using X = typename L::X;
+    using L = SplitSmem<kPrec>;
+    using S = Surface<kPrec>;
     extern __shared__ __align__(16) unsigned char smem[];
     const uint32_t cap = a.max_step_cap;
-    QueueCtl &ctl = *reinterpret_cast<QueueCtl *>(smem + L::ctl());
-    float4 *s_t = reinterpret_cast<float4 *>(smem + L::steps(cap));
-    long long *s_boff = reinterpret_cast<long long *>(smem + L::boff(cap));
-    int2 *s_q = reinterpret_cast<int2 *>(smem + L::boff(cap));  // quad: {forward, backward}
-    X *s_x = reinterpret_cast<X *>(smem + L::xtab(cap));
-    SegBound *s_seg = reinterpret_cast<SegBound *>(smem + L::seg(cap));
-    S *s_fwd = reinterpret_cast<S *>(smem + L::fwd(cap));
-    int32_t *s_j = reinterpret_cast<int32_t *>(smem + L::jtab(cap));  // MIXED64, not lean
-    const uint32_t tid = threadIdx.y * kQueueTileX + threadIdx.x;
-    const uint32_t lane = threadIdx.x;
-    queue_init(ctl, tid);
+    SplitCtl &ctl = *reinterpret_cast<SplitCtl *>(smem);
+    const uint32_t slot_bytes = (uint32_t)L::slot(cap);
+    auto slot_of = [&](uint32_t c) -> unsigned char * {
+        return smem + ((uint32_t)L::slots() + c % n_slots * slot_bytes);
+    };
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t warp = uni(threadIdx.x >> 5);
+    const uint32_t n_items = a.chunks * a.n_sectors * 2;
+    if (threadIdx.x < 4) ctl.diag[threadIdx.x] = 0;
+    if (threadIdx.x == 0) ctl.ready = 0;
+    __syncthreads();
 
-    while (queue_next(a, ctl, tid)) {
-        const QueueDem &D = ctl.dem;
-        const uint32_t s = ctl.sector, tile = ctl.tile;
-        if (tid < 4) ctl.diag[tid] = 0;
-        if (ctl.restage) {
-            // ---- stage this DEM's sector tables -----------------------------
-            const uint32_t slot = a.first_sector + s;
+    // Brings chunk c into its slot (one warp): the next item of the queue and
+    // its step tables.
+    auto bring = [&](uint32_t c) {
+        unsigned char *base = slot_of(c);
+        SplitSlot &sl = *reinterpret_cast<SplitSlot *>(base);
+        Step<kPrec> *s_t = reinterpret_cast<Step<kPrec> *>(base + L::table());
+        SegBound *s_seg = reinterpret_cast<SegBound *>(base + L::seg(cap));
+        uint32_t item = 0;
+        if (lane == 0) item = atomicAdd(a.queue, 1u);
+        item = uni(item);
+        if (item < n_items) {
+            const uint32_t group = item / a.chunks, r = item - group * a.chunks;
+            const uint32_t dir = group & 1u, slot = a.first_sector + (group >> 1);
+            // the DEM whose chunks hold r (chunk_base ascends)
+            uint32_t lo = 0, hi = a.n_dems - 1;
+            while (lo < hi) {
+                const uint32_t mid = (lo + hi + 1) >> 1;
+                if (uni(__ldg(&a.dems[mid].chunk_base)) <= r) lo = mid; else hi = mid - 1;
+            }
+            const uint32_t *src = reinterpret_cast<const uint32_t *>(a.dems + lo);
+            uint32_t *dst = reinterpret_cast<uint32_t *>(&sl.dem);
+#pragma unroll
+            for (uint32_t q = 0; q < sizeof(QueueDem) / 4; q += 32)
+                if (q + lane < sizeof(QueueDem) / 4) dst[q + lane] = __ldg(src + q + lane);
+            __syncwarp();
+            const QueueDem &D = sl.dem;
             const ShapeHeader *h = D.hdr + slot;
-            const uint32_t n = h->n_steps;
+            const uint32_t nf = uni(h->n_fast);
+            // surfaces stop at the last step that adds to them
+            const uint32_t n = uni(kRings ? h->n_steps : max(nf, min(h->n_surf, h->n_steps)));
+            const bool plain = !kQuad || uni(h->wide) != 0;
             const float4 *gs = D.steps + (uint64_t)slot * D.step_cap;
             const int2 *go = D.offs + (uint64_t)slot * D.step_cap;
+            const int2 *gq = D.quads + (uint64_t)slot * D.step_cap;
+            const int4 *gseg = D.segs + (uint64_t)slot * seg_count(D.step_cap);
             const double4 *gd = D.dtab + (uint64_t)slot * D.step_cap;
-            const float hmax = kFp32 ? 0.0f : *D.hmax;
-            // The quad copies hold a lane's four rows at one column.  The
-            // reference's sample ids are linear (kernel.rs:259-292), so a step
-            // that moves more than the line of sight sideways wraps a point of
-            // view's row; such a sector reads the plain DEM.  Otherwise every
-            // point of view's samples stay on its own rows, inside the DEM, and
-            // every quad address inside the copies.
-            bool plain = !kQuad;
-            if constexpr (kQuad) {
-                bool wide = false;
-                for (uint32_t i = tid; i < n; i += kQueueThreads) {
-                    long long dx, dy;
-                    step_xy(go[i].x, D.width, dx, dy);
-                    wide |= dx > (long long)D.los || dx < -(long long)D.los;
-                }
-                plain = __syncthreads_or(wide) != 0;
-                if (tid == 0) ctl.plain = plain;
-            }
-            for (uint32_t i = tid; i < n; i += kQueueThreads) {
-                const float4 t = gs[i];  // {RN(1/d), d, RN(d/R), RN(d*tan1)}
-                if (!plain)
-                    s_q[i] = quad_offsets(go[i].x, D.width, (D.row_begin + D.los) & 3u,
-                                          (long long)D.quad_copy * 16);
-                else
-                    s_boff[i] = (long long)go[i].x * (long long)sizeof(float);
-                if constexpr (kFp32) {
-                    s_t[i] = make_float4(t.x, -t.z, t.w, 0.0f);
-                } else {
-                    const float o = D.observer_height;
-                    const float off = kMix ? -__fadd_rn(t.z, __fmul_rn(o, t.x)) : -t.z;
-                    const float g = kMix ? mix_window(t.x, t.z, o, hmax) : step_window(t.x, t.z, hmax);
-                    const float zhi = __fadd_rn(off, g), zlo = __fsub_rn(off, g);
+            (void)gd;
+            const float hmax = kMix ? *D.hmax : 0.0f;
+            // from the last 32 steps to the first: the band needs the largest G of
+            // the later steps
+            float later = 0.0f;
+            for (uint32_t b = seg_count(n); b-- > 0;) {
+                const uint32_t i0 = b * kSegSteps, i = i0 + lane;
+                const bool v = i < n;
+                float4 t = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                float z = 0.0f, g = 0.0f;
+                if (v) {
+                    t = gs[i];  // {RN(1/d), d, RN(d/R), RN(d*tan1)}
+                    z = -t.z;
                     if constexpr (kMix) {
-                        s_t[i] = make_float4(t.x, zhi, zlo, t.y);
-                        const double4 dt = gd[i];  // {1/d, d/R, d*tan1, d} in double
-                        if constexpr (L::kExactTab) s_x[i] = make_double2(dt.y, dt.z);
+                        z = -__fadd_rn(t.z, __fmul_rn(D.observer_height, t.x));
+                        if (i < nf) g = band_mix(t.x, t.z, D.observer_height, hmax);
+                    } else if constexpr (!kFp32) {
+                        z = __fadd_rn(z, window_exact(t.z));
+                    }
+                }
+                if constexpr (kMix) {
+                    float most = g;  // of this step and the later ones
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const float q = __shfl_down_sync(0xffffffffu, most, o);
+                        if (lane + o < 32) most = fmaxf(most, q);
+                    }
+                    most = fmaxf(most, later);
+                    later = __shfl_sync(0xffffffffu, most, 0);
+                    g = __fadd_rn(g, most);
+                }
+                if (v) {
+                    int off;
+                    if (plain) {
+                        off = go[i].x;
+                        off = dir ? -off : off;
                     } else {
-                        s_t[i] = make_float4(t.x, zhi, zlo, t.w);
-                        s_x[i] = make_float2(t.y, t.z);
+                        const int2 q = gq[i];
+                        off = (dir ? q.y : q.x) * (int)sizeof(float4);
+                    }
+                    s_t[i].next = off;
+                    Step<kPrec> &e = s_t[i + kAhead];
+                    e.y = t.x;
+                    e.z = z;
+                    if constexpr (kMix) {
+                        e.band = g;
+                        e.w = gd[i].z;
+                    } else {
+                        e.w = t.w;
+                        if constexpr (!kFp32) {
+                            e.d = t.y;
+                            e.c = t.z;
+                        }
+                    }
+                }
+                if (i0 < nf) {  // these 32 steps are segment b
+                    const bool f = i < nf;
+                    float ymax = f ? t.x : -INFINITY, ymin = f ? t.x : INFINITY;
+                    float zmax = f ? z : -INFINITY;
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        ymax = fmaxf(ymax, __shfl_xor_sync(0xffffffffu, ymax, o));
+                        ymin = fminf(ymin, __shfl_xor_sync(0xffffffffu, ymin, o));
+                        zmax = fmaxf(zmax, __shfl_xor_sync(0xffffffffu, zmax, o));
+                    }
+                    if (lane == 0) {
+                        const int4 q = gseg[b];
+                        s_seg[b] = dir ? SegBound{-q.y, -q.x, -q.w, -q.z, ymax, ymin, zmax, 0.0f}
+                                                    : SegBound{q.x, q.y, q.z, q.w, ymax, ymin, zmax, 0.0f};
                     }
                 }
             }
-            __syncthreads();
-            // segment bounds of the fast steps, one warp per segment
-            const uint32_t nf = h->n_fast;
-            const long long W = D.width;
-            for (uint32_t sg = threadIdx.y; sg * kSegSteps < nf; sg += kQueueTileY) {
-                const uint32_t i = sg * kSegSteps + lane;
-                const bool v = lane < kSegSteps && i < nf;
-                long long dxl, dy;
-                step_xy(v ? (long long)go[i].x : 0, W, dxl, dy);
-                const int dx = (int)dxl;
-                int dx0 = v ? dx : INT_MAX, dx1 = v ? dx : INT_MIN;
-                int dy0 = v ? (int)dy : INT_MAX, dy1 = v ? (int)dy : INT_MIN;
-                float ymax = v ? s_t[i].x : -INFINITY, ymin = v ? s_t[i].x : INFINITY;
-                float zmax = v ? s_t[i].y : -INFINITY;
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    dx0 = min(dx0, __shfl_xor_sync(0xffffffffu, dx0, o));
-                    dx1 = max(dx1, __shfl_xor_sync(0xffffffffu, dx1, o));
-                    dy0 = min(dy0, __shfl_xor_sync(0xffffffffu, dy0, o));
-                    dy1 = max(dy1, __shfl_xor_sync(0xffffffffu, dy1, o));
-                    ymax = fmaxf(ymax, __shfl_xor_sync(0xffffffffu, ymax, o));
-                    ymin = fminf(ymin, __shfl_xor_sync(0xffffffffu, ymin, o));
-                    zmax = fmaxf(zmax, __shfl_xor_sync(0xffffffffu, zmax, o));
-                }
-                if (lane == 0) s_seg[sg] = SegBound{dx0, dx1, dy0, dy1, ymax, ymin, zmax, 0.0f};
-            }
-            if (tid == 0) {
-                ctl.sector_status = h->status;
-                ctl.n_steps = n;
-                ctl.n_fast = nf;
+            if (lane == 0) {
+                for (uint32_t q = 0; q < kAhead; q++) s_t[n + q].next = 0;  // the point of view itself
+                const uint32_t tiles = D.tiles_x * D.tiles_y;
+                sl.tile0 = (r - D.chunk_base) * D.chunk;
+                sl.n_tiles = min(D.chunk, tiles - sl.tile0);
+                sl.group = group;
+                sl.n = n;
+                sl.n_fast = nf;
+                sl.status = h->status;
+                sl.plain = plain;
             }
         }
-        __syncthreads();  // the staged tables
+        __syncwarp();
+        if (lane == 0) {
+            sl.next = 0;
+            sl.left = 0;
+            sl.end = item >= n_items;
+            st_release(&ctl.ready, c + 1);
+        }
+        __syncwarp();
+    };
+    static_assert(kSegSteps == 32, "a segment's bounds are reduced in one warp, a step per lane");
+    // All lanes: waits (bounded) until *p >= v; false: gave up.  The exits are
+    // votes, here and below: a loop of one lane would split the warp, and the
+    // step loop would then run once for each part.
+    auto wait_for = [&](const uint32_t *p, uint32_t v) -> bool {
+        uint32_t spins = 0;
+        while (!__all_sync(0xffffffffu, ld_acquire(p) >= v)) {
+            if (++spins > kRingSpinLimit) {
+                if (lane == 0) atomicExch(a.error, (int32_t)TVS_ERR_TIMEOUT);
+                __syncwarp();
+                return false;
+            }
+            __nanosleep(64);
+        }
+        return true;
+    };
+    // Chunk c can be brought in when every warp has left the chunk whose slot
+    // it takes.
+    auto slot_free = [&](uint32_t c) -> bool {
+        if (c < n_slots) return true;
+        return uni(ld_acquire(&reinterpret_cast<SplitSlot *>(slot_of(c))->left)) == kWarps;
+    };
 
-        if (ctl.sector_status == TVS_OK) {
-            const uint32_t n = ctl.n_steps, n_fast = ctl.n_fast;
-            const uint32_t bx = tile % D.tiles_x, by = tile / D.tiles_x;
-            // chain k: column tx + LX (k % KX), row ty + LY (k / KX)
+    uint32_t n_swept = 0, n_passed = 0, n_all = 0;  // counters of this warp
+    if (warp == 0) bring(0);
+    for (uint32_t chunk = 0; wait_for(&ctl.ready, chunk + 1);) {
+        unsigned char *base = slot_of(chunk);
+        SplitSlot &sl = *reinterpret_cast<SplitSlot *>(base);
+        if (uni(sl.end)) break;
+        uint32_t idx = 0;
+        if (lane == 0) idx = atomicAdd(&sl.next, 1u);
+        idx = uni(idx);
+        if (idx >= uni(sl.n_tiles)) {
+            __syncwarp();
+            if (lane == 0) red_release(&sl.left, 1u);
+            __syncwarp();
+            chunk++;
+            continue;
+        }
+        bool owe = idx == sl.n_tiles - 1;  // this warp brings the next chunk
+        if (owe && slot_free(chunk + 1)) {
+            bring(chunk + 1);
+            owe = false;
+        }
+        const QueueDem &D = sl.dem;
+        const Step<kPrec> *s_t = reinterpret_cast<const Step<kPrec> *>(base + L::table());
+        const SegBound *s_seg = reinterpret_cast<const SegBound *>(base + L::seg(cap));
+        const uint32_t tile = uni(sl.tile0) + idx;
+        const uint32_t group = uni(sl.group), dir = group & 1u;
+
+        if (uni((uint32_t)(sl.status == TVS_OK))) {
+            const uint32_t n = uni(sl.n), n_fast = uni(sl.n_fast);
+            // tiles run down stripes of 8 tile rows, so that a chunk is a compact
+            // block of the DEM
+            const uint32_t per = 8 * D.tiles_x, stripe = tile / per, in = tile - stripe * per;
+            const uint32_t rows = min(8u, D.tiles_y - 8 * stripe);
+            const uint32_t bx = in / rows, by = 8 * stripe + in - bx * rows;
+            // chain k: column tx + LX (k % KX), row ty + RS (k / KX)
             const uint32_t lx = lane % LX, ly = lane / LX;
             const uint32_t tx = bx * (KX * LX) + lx;
-            const uint32_t ty = D.row_begin + by * (kQueueTileY * LY * KY) + threadIdx.y * LY * KY + ly;
+            const uint32_t ty = D.row_begin + by * (LY * KY) + ly * LS;
             // rows past the grid are clamped, columns past it read the padding
             // after the elevations; both are discarded (and record no rings)
             auto row_ptr = [&](int r) -> const float * {
-                return D.elev + (int64_t)(min(ty + LY * r, D.row_end - 1) + D.los) * D.width + tx + D.los;
+                return D.elev + (int64_t)(min(ty + RS * r, D.row_end - 1) + D.los) * D.width + tx + D.los;
             };
-            // the quad layout reads the plain DEM only on a few sectors: there
-            // the row pointers are recomputed instead of held in registers
-            const float *ep[kQuad ? 1 : KY];
+            uint32_t active = 0;  // chains on the grid
 #pragma unroll
-            for (int r = 0; r < (kQuad ? 1 : KY); r++) ep[r] = row_ptr(r);
-            // quad: the lane's base in the row-interleaved copies (rows past the
-            // grid are not clamped: the copies hold zero rows for them)
-            const char *qbase = nullptr;
-            if constexpr (kQuad)
-                qbase = reinterpret_cast<const char *>(
-                    D.quad + (uint64_t)((ty + D.los - ((D.row_begin + D.los) & 3u)) / 4) * D.width +
-                    tx + D.los);
-            const int2 *goff = D.offs + (uint64_t)(a.first_sector + s) * D.step_cap;
-            const double4 *gdt = D.dtab + (uint64_t)(a.first_sector + s) * D.step_cap;  // MIXED64
-            (void)qbase;
-            (void)goff;
-            (void)gdt;
+            for (int k = 0; k < K; k++)
+                if (tx + LX * (k % KX) < D.tvs_width && ty + RS * (k / KX) < D.row_end) active |= 1u << k;
             // kernel.rs:134, the f32 observer elevation (MIXED64: the point of
             // view's own elevation; the observer height is in the step's offset)
-            float hp32[K];
+            float hp[K];
 #pragma unroll
             for (int k = 0; k < K; k++) {
                 const float h = __ldg(row_ptr(k / KX) + LX * (k % KX));
-                hp32[k] = kMix ? h : __fadd_rn(h, D.observer_height);
+                hp[k] = kMix ? h : __fadd_rn(h, D.observer_height);
             }
-            // chain k's point-of-view elevation, re-read by the rare exact
-            // re-decisions (the address is recomputed rather than kept live)
-            auto pov_h = [&](int k) -> float {
-                const uint32_t r = min(ty + LY * (k / KX), D.row_end - 1);
-                return __ldg(D.elev + (int64_t)(r + D.los) * D.width + tx + LX * (k % KX) + D.los);
-            };
-            uint32_t active = 0;  // chains on the grid (ring records)
+            f32x2 nhp[K / 2];  // negated, for the packed subtraction
 #pragma unroll
-            for (int k = 0; k < K; k++)
-                if (tx + LX * (k % KX) < D.tvs_width && ty + LY * (k / KX) < D.row_end) active |= 1u << k;
-            uint32_t n_swept = 0, n_passed = 0;  // diagnostics (re-decisions count in ctl.diag[3])
-            S sb[K];
+            for (int q = 0; q < K / 2; q++) nhp[q] = pk(-hp[2 * q], -hp[2 * q + 1]);
+            S out[K];
 
-            // one direction's sweep; PLAIN: a quad-layout sector that reads the
+            // the sweep of this tile; PLAIN: a quad-layout sector that reads the
             // plain DEM (a separate instantiation, so that the quad loop is as
             // lean as without it)
-            auto pass = [&](auto DIR, auto PLAIN) {
-                constexpr int dir = decltype(DIR)::value;
-                constexpr bool qplain = decltype(PLAIN)::value;
-                auto at = [&](long long b, int k) -> const float * {
+            auto pass = [&](auto PLAIN) {
+                constexpr bool quad = kQuad && !decltype(PLAIN)::value;
+                // plain: the rows of the lane's chains (recomputed in the quad
+                // layout's few plain sectors)
+                const float *ep[kQuad ? 1 : KY] = {};
+                if constexpr (!quad) {
+#pragma unroll
+                    for (int r = 0; r < (kQuad ? 1 : KY); r++) ep[r] = row_ptr(r);
+                }
+                // quad: the copies' base and the lane's offset in them, in bytes (rows
+                // past the grid are not clamped: the copies hold zero rows for
+                // them).  The copies lie within 2^31 bytes (quad_fits): a sample's
+                // address is a uniform base and one 32-bit add.
+                const char *qbase = nullptr;
+                uint32_t qlane = 0;
+                if constexpr (quad) {
+                    const uint64_t q = reinterpret_cast<uint64_t>(D.quad);
+                    qbase = reinterpret_cast<const char *>((uint64_t)uni((uint32_t)(q >> 32)) << 32 |
+                                                           uni((uint32_t)q));
+                    qlane = (((ty + D.los - ((D.row_begin + D.los) & 3u)) / 4) * D.width + tx + D.los) * 16u;
+                }
+                (void)qbase;
+                (void)qlane;
+                auto at = [&](int off, int k) -> const float * {
                     const float *row = kQuad ? row_ptr(k / KX) : ep[k / KX];
-                    return (const float *)((const char *)row + (dir ? -b : b)) + LX * (k % KX);
+                    return row + off + LX * (k % KX);
                 };
-                // ring records of chain k: kernel id and the DEM id of a sample
-                // the four chains' samples at step st
-                auto load = [&](uint32_t st, float (&h)[K]) {
-                    if constexpr (kQuad && !qplain) {
-                        const int2 o = s_q[st];
-                        const float4 v = __ldg(reinterpret_cast<const float4 *>(qbase + (dir ? o.y : o.x)));
+                auto quad_at = [&](int off) -> const float4 * {
+                    return reinterpret_cast<const float4 *>(qbase + (qlane + (uint32_t)off));
+                };
+                // the four chains' samples at a step's offset
+                auto load = [&](int off, float (&h)[K]) {
+                    if constexpr (quad) {
+                        const float4 v = __ldg(quad_at(off));
                         h[0] = v.x;
                         h[1] = v.y;
                         h[2] = v.z;
                         h[3] = v.w;
                     } else {
-                        const long long b = s_boff[st];
 #pragma unroll
-                        for (int k = 0; k < K; k++) h[k] = __ldg(at(b, k));
+                        for (int k = 0; k < K; k++) h[k] = __ldg(at(off, k));
                     }
                 };
-                auto load1 = [&](uint32_t st, int k) -> float {
-                    if constexpr (kQuad && !qplain) {
-                        const int2 o = s_q[st];
-                        return __ldg(reinterpret_cast<const float *>(qbase + (dir ? o.y : o.x)) + k);
-                    } else {
-                        return __ldg(at(s_boff[st], k));
-                    }
+                auto load1 = [&](int off, int k) -> float {
+                    if constexpr (quad) return __ldg(reinterpret_cast<const float *>(quad_at(off)) + k);
+                    else return __ldg(at(off, k));
                 };
-                // the step's forward offset in bytes in the DEM (ring ids)
+                // ring records of chain k: kernel id and the DEM id of a sample;
+                // a call over several sectors keeps each sector's records apart: its
+                // sector s owns records s * total_bands ..
                 auto orig = [&](uint32_t st) -> long long {
-                    if constexpr (kQuad && !qplain)
-                        return (long long)__ldg(&goff[st].x) * (long long)sizeof(float);
-                    else
-                        return s_boff[st];
+                    if constexpr (quad) {
+                        const long long o =
+                            __ldg(&D.offs[(uint64_t)(a.first_sector + (group >> 1)) * D.step_cap + st].x);
+                        return dir ? -o : o;
+                    } else {
+                        return s_t[st].next;
+                    }
                 };
-                // a launch over several sectors keeps each sector's records
-                // apart: sector s of the launch owns records s * total_bands ..
                 auto kid = [&](int k) -> uint64_t {
-                    return (uint64_t)(ty + LY * (k / KX)) * D.tvs_width + tx + LX * (k % KX) +
-                           (dir ? a.half_bands : 0) + (uint64_t)s * 2 * a.half_bands;
+                    return (uint64_t)(ty + RS * (k / KX)) * D.tvs_width + tx + LX * (k % KX) +
+                           (dir ? a.half_bands : 0) +
+                           (uint64_t)(a.first_sector - a.first_record_sector + (group >> 1)) * 2 * a.half_bands;
                 };
-                auto dem_id = [&](int k, long long b) -> uint32_t {
-                    const long long pov = (long long)(ty + LY * (k / KX) + D.los) * D.width +
+                auto dem_id = [&](int k, long long o) -> uint32_t {
+                    const long long pov = (long long)(ty + RS * (k / KX) + D.los) * D.width +
                                           tx + LX * (k % KX) + D.los;
-                    return (uint32_t)(pov + (dir ? -b : b) / (long long)sizeof(float));
+                    return (uint32_t)(pov + o);
                 };
                 auto ring_put = [&](uint64_t band, uint32_t slot, uint32_t value) {
                     if (slot < a.ring_reserved) {
@@ -451,10 +638,10 @@ k_sweep_split(QueueArgs a) {
                 auto events = [&](uint32_t vis, uint32_t st) {
                     const uint32_t ev = (vis ^ prev) & active;
                     if (__any_sync(0xffffffffu, ev != 0)) {
-                        const long long b = orig(st);
+                        const long long o = orig(st);
 #pragma unroll
                         for (int k = 0; k < K; k++)
-                            if (ev >> k & 1u) ring_put(kid(k), ++nr[k], dem_id(k, b));
+                            if (ev >> k & 1u) ring_put(kid(k), ++nr[k], dem_id(k, o));
                     }
                     prev = vis;
                 };
@@ -463,19 +650,19 @@ k_sweep_split(QueueArgs a) {
                 // view moved by the segment's offset range (warp-uniform).
                 auto segment_max = [&](const SegBound &b) -> float {
                     const int px0 = (int)(bx * (KX * LX) + D.los), px1 = px0 + KX * LX - 1;
-                    const int py0 = (int)(D.row_begin + by * (kQueueTileY * LY * KY) +
-                                          threadIdx.y * LY * KY + D.los);
-                    const int py1 = py0 + LY * KY - 1;
-                    const int x0 = dir ? px0 - b.dx1 : px0 + b.dx0, x1 = dir ? px1 - b.dx0 : px1 + b.dx1;
-                    const int y0 = dir ? py0 - b.dy1 : py0 + b.dy0, y1 = dir ? py1 - b.dy0 : py1 + b.dy1;
-                    const int bx0 = max(x0, 0) / (int)kBlockMax;
-                    const int bx1 = min(max(x1, 0) / (int)kBlockMax, (int)D.bmax_w - 1);
-                    const int by0 = max(y0, 0) / (int)kBlockMax;
-                    const int by1 = min(max(y1, 0) / (int)kBlockMax, (int)D.bmax_h - 1);
-                    const int nx = bx1 - bx0 + 1, cells = nx > 0 && by1 >= by0 ? nx * (by1 - by0 + 1) : 0;
+                    const int py0 = (int)(D.row_begin + by * (LY * KY) + D.los), py1 = py0 + LY * KY - 1;
+                    const int bx0 = max(px0 + b.x0, 0) / (int)kBlockMax;
+                    const int bx1 = min(max(px1 + b.x1, 0) / (int)kBlockMax, (int)D.bmax_w - 1);
+                    const int by0 = max(py0 + b.y0, 0) / (int)kBlockMax;
+                    const int by1 = min(max(py1 + b.y1, 0) / (int)kBlockMax, (int)D.bmax_h - 1);
                     float m = -INFINITY;
-                    for (int q = (int)lane; q < cells; q += 32)
-                        m = fmaxf(m, __ldg(D.bmax + (size_t)(by0 + q / nx) * D.bmax_w + bx0 + q % nx));
+                    // 8 x 4 blocks at a time
+                    for (int y0 = by0; y0 <= by1; y0 += 4)
+                        for (int x0 = bx0; x0 <= bx1; x0 += 8) {
+                            const int y = y0 + (int)(lane >> 3), x = x0 + (int)(lane & 7u);
+                            if (y <= by1 && x <= bx1)
+                                m = fmaxf(m, __ldg(D.bmax + (uint32_t)y * D.bmax_w + x));
+                        }
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
                     return m;
@@ -492,110 +679,137 @@ k_sweep_split(QueueArgs a) {
                     bool skip = prev == 0;
 #pragma unroll
                     for (int k = 0; k < K; k++) {
-                        const float E = __fsub_rn(B, hp32[k]);
+                        const float E = __fsub_rn(B, hp[k]);
                         skip &= below(k, __fmaf_rn(E, E >= 0.0f ? b.ymax : b.ymin, b.zmax));
                     }
                     return __all_sync(0xffffffffu, skip);
                 };
-                S out[K];
+                // e = h - h_pov and the estimate fma(e, y, z) of the four chains (the
+                // subtraction packed; the multiply-adds not, for they would need
+                // y and z in pairs)
+                auto estimate = [&](const float (&h)[K], float y, float z, float (&e)[K], float (&f)[K]) {
+#pragma unroll
+                    for (int q = 0; q < K / 2; q++)
+                        upk(add2(pk(h[2 * q], h[2 * q + 1]), nhp[q]), e[2 * q], e[2 * q + 1]);
+#pragma unroll
+                    for (int k = 0; k < K; k++) f[k] = __fmaf_rn(e[k], y, z);
+                };
                 uint32_t i = 0;
+                // The segments of fast steps, two steps an iteration: the samples of
+                // step i + 2 take the registers of step i's as soon as its estimates
+                // are formed, so two loads are under way at every step (one step
+                // ahead: 1201^2 exact f32 4.47 ms, two: 3.74 ms).
+                auto sweep_fast = [&](auto &&below, auto &&step) {
+                    for (uint32_t seg = 0; i < n_fast; seg++) {
+                        const uint32_t i1 = min(i + kSegSteps, n_fast);
+                        if (skippable(seg, below)) {
+                            i = i1;
+                            continue;
+                        }
+                        n_swept += i1 - i;
+                        float h0[K], h1[K];
+                        load(s_t[i].next, h0);
+                        load(s_t[i + 1].next, h1);
+                        const Step<kPrec> *p = s_t + i + kAhead;
+                        if constexpr (kFp32) {  // its short steps gain from four an iteration
+                            for (; i + 4 <= i1; i += 4, p += 4) {
+                                step(i, p, h0);
+                                step(i + 1, p + 1, h1);
+                                step(i + 2, p + 2, h0);
+                                step(i + 3, p + 3, h1);
+                            }
+                        }
+#pragma unroll 1
+                        for (; i + 2 <= i1; i += 2, p += 2) {
+                            step(i, p, h0);
+                            step(i + 1, p + 1, h1);
+                        }
+                        if (i < i1) {
+                            step(i, p, h0);
+                            i++;
+                        }
+                    }
+                };
                 if constexpr (kFp32) {
                     // ---- the reciprocal-table form: the estimate is the angle --
                     float m[K], sf[K];
 #pragma unroll
                     for (int k = 0; k < K; k++) {
-                        m[k] = kMaxAngle;
+                        m[k] = active >> k & 1u ? kMaxAngle : INFINITY;  // off the grid: never visible
                         sf[k] = 0.0f;
                     }
-                    auto step = [&](uint32_t st) {
-                        const float4 t = s_t[st];  // {y, -c, w, 0}
-                        float h[K];
-                        load(st, h);
-                        uint32_t vis = 0;
+                    // step i from its samples h, which then hold step i + kAhead's
+                    auto step = [&](uint32_t st, const Step<kPrec> *p, float (&h)[K]) {
+                        const Step<kPrec> t = *p;
+                        float e[K], ang[K];
+                        estimate(h, t.y, t.z, e, ang);
+                        load(t.next, h);
+                        [[maybe_unused]] uint32_t vis = 0;
 #pragma unroll
                         for (int k = 0; k < K; k++) {
-                            const float ang = __fmaf_rn(__fsub_rn(h[k], hp32[k]), t.x, t.y);
-                            const bool v = ang > m[k];
-                            if (v) sf[k] = __fadd_rn(sf[k], t.z);
-                            m[k] = fmaxf(ang, m[k]);  // NaN yields the other operand
-                            vis |= (uint32_t)v << k;
+                            if constexpr (kRings) vis |= (uint32_t)(ang[k] > m[k]) << k;
+                            raise_fp32(ang[k], m[k], sf[k], t.w);
                         }
                         if constexpr (kRings) events(vis, st);
                     };
-                    for (uint32_t seg = 0; i < n_fast; seg++) {
-                        const uint32_t i1 = min(i + kSegSteps, n_fast);
-                        if (skippable(seg, [&](int k, float bound) { return bound <= m[k]; })) {
-                            i = i1;
-                            continue;
-                        }
-                        n_swept += i1 - i;
-                        TVS_UNROLL(TVS_SPLIT_UNROLL32)
-                        for (; i < i1; i++) step(i);
+                    sweep_fast([&](int k, float bound) { return bound <= m[k]; }, step);
+                    for (; i < n; i++) {  // zero distances: y = inf, the same form
+                        float h[K];
+                        load(s_t[i].next, h);
+                        step(i, s_t + i + kAhead, h);
                     }
-                    for (; i < n; i++) step(i);  // zero distances: y = inf, the same form
 #pragma unroll
                     for (int k = 0; k < K; k++) out[k] = sf[k];
-                } else if constexpr (!kMix && TVS_EXACT_INLINE) {
+                } else if constexpr (!kMix) {
                     // ---- exact f32, the running maximum held exactly ----------
-                    // The first test fma(e, y, -c + G) >= m - |m| 2^-19 passes
-                    // every step where a chain may change state (|a - (e y - c)|
-                    // <= 2^-22 |a| + 2^-23 c); there the reference's angle is
-                    // computed for every chain (kernel.rs:175-233).
+                    // where the first test passes the reference's angle is computed
+                    // for every chain (kernel.rs:175-233)
                     float m[K], lo[K], sf[K];
 #pragma unroll
                     for (int k = 0; k < K; k++) {
-                        m[k] = kMaxAngle;
-                        lo[k] = __fmaf_rn(fabsf(m[k]), -kRel, m[k]);
+                        m[k] = active >> k & 1u ? kMaxAngle : INFINITY;  // off the grid: never visible
+                        lo[k] = active >> k & 1u ? __fmaf_rn(fabsf(m[k]), -kRelExact, m[k]) : INFINITY;
                         sf[k] = 0.0f;
                     }
-                    for (uint32_t seg = 0; i < n_fast; seg++) {
-                        const uint32_t i1 = min(i + kSegSteps, n_fast);
-                        if (skippable(seg, [&](int k, float bound) { return bound < lo[k]; })) {
-                            i = i1;
-                            continue;
-                        }
-                        n_swept += i1 - i;
-                        TVS_UNROLL(TVS_SPLIT_UNROLL_EXACT)
-                        for (; i < i1; i++) {
-                            const float4 t = s_t[i];  // {y, -c + G, -c - G, w}
-                            float e[K];
-                            load(i, e);
-                            bool hit = false;
+                    auto step = [&](uint32_t st, const Step<kPrec> *p, float (&h)[K]) {
+                        const float y = p->y, z = p->z, w = p->w;
+                        const int next = p->next;
+                        float e[K], f[K];
+                        estimate(h, y, z, e, f);  // kernel.rs:164
+                        load(next, h);
+                        bool hit = false;
 #pragma unroll
-                            for (int k = 0; k < K; k++) {
-                                e[k] = __fsub_rn(e[k], hp32[k]);  // kernel.rs:164
-                                hit |= __fmaf_rn(e[k], t.x, t.y) >= lo[k];
-                            }
-                            if (!__any_sync(0xffffffffu, hit || prev != 0)) continue;
+                        for (int k = 0; k < K; k++) hit |= f[k] >= lo[k];
+                        if (__any_sync(0xffffffffu, hit || prev != 0)) {
                             n_passed++;
-                            const float2 x = s_x[i];  // {d, c}
-                            uint32_t vis = 0;
+                            const float d = p->d, c = p->c;
+                            [[maybe_unused]] uint32_t vis = 0;
 #pragma unroll
                             for (int k = 0; k < K; k++) {
-                                const float ang = __fsub_rn(div_table32(e[k], t.x, x.x), x.y);
-                                const bool v = ang > m[k];
-                                if (v) sf[k] = __fadd_rn(sf[k], t.w);
-                                m[k] = fmaxf(ang, m[k]);  // f32::max: NaN yields the other
-                                lo[k] = __fmaf_rn(fabsf(m[k]), -kRel, m[k]);
-                                vis |= (uint32_t)v << k;
+                                const float ang = __fsub_rn(div_table32(e[k], y, d), c);
+                                if constexpr (kRings) vis |= (uint32_t)(ang > m[k]) << k;
+                                raise_exact(ang, m[k], sf[k], lo[k], w);
                             }
-                            if constexpr (kRings) events(vis, i);
+                            if constexpr (kRings) events(vis, st);
                         }
-                    }
-                    for (; i < n; i++) {  // the zero-distance tail, IEEE division
-                        const float2 x = s_x[i];
-                        const bool fast = x.x >= 0x1p-20f && x.x <= 0x1p20f;
+                    };
+                    sweep_fast([&](int k, float bound) { return bound < lo[k]; }, step);
+                    for (; i < n; i++) {  // past the table division's domain: IEEE division
+                        const Step<kPrec> &t = s_t[i + kAhead];
+                        const bool fast = t.d >= 0x1p-20f && t.d <= 0x1p20f;
                         float h[K];
-                        load(i, h);
+                        load(s_t[i].next, h);
                         uint32_t vis = 0;
 #pragma unroll
                         for (int k = 0; k < K; k++) {
-                            const float e = __fsub_rn(h[k], hp32[k]);
+                            const float e = __fsub_rn(h[k], hp[k]);
                             const float ang =
-                                __fsub_rn(fast ? div_table32(e, s_t[i].x, x.x) : __fdiv_rn(e, x.x), x.y);
+                                __fsub_rn(fast ? div_table32(e, t.y, t.d) : __fdiv_rn(e, t.d), t.c);
                             const bool v = ang > m[k];
-                            if (v) sf[k] = __fadd_rn(sf[k], s_t[i].w);
-                            m[k] = fmaxf(ang, m[k]);
+                            if (v) {
+                                sf[k] = __fadd_rn(sf[k], t.w);
+                                m[k] = ang;
+                            }
                             vis |= (uint32_t)v << k;
                         }
                         if constexpr (kRings) events(vis, i);
@@ -603,174 +817,104 @@ k_sweep_split(QueueArgs a) {
 #pragma unroll
                     for (int k = 0; k < K; k++) out[k] = sf[k];
                 } else {
-                    // ---- guard band with exact re-decisions (MIXED64) ----------
-                    constexpr bool kJSmem = kMix && !kLean && !TVS_MIX_JREG;
-                    constexpr bool kJPack = kMix && TVS_MIX_JREG;
-                    float hi[K], lo[K];
-                    // step of the running maximum (-1: the initial one)
-                    int32_t jreg[kJSmem ? 1 : K] = {};
-                    int32_t *sj = s_j + tid;
-                    (void)jreg;
-                    (void)sj;
-                    // packed: two chains' steps per register, 16 bits each
+                    // ---- MIXED64: the guard band ------------------------------
+                    float nmid[K], hw[K];  // -(the maximum's estimate), the band's half width
+                    // step of the running maximum, 16 bits, two chains per register
                     // (0xffff: the initial maximum)
-                    uint32_t jpk[K / 2] = {};
-                    (void)jpk;
-                    auto getj = [&](int k) -> int32_t {
-                        if constexpr (kJSmem) return sj[k * kQueueThreads];
-                        else if constexpr (kJPack) {
-                            const uint32_t v = (jpk[k / 2] >> (16 * (k & 1))) & 0xffffu;
-                            return v == 0xffffu ? -1 : (int32_t)v;
-                        } else return jreg[k];
-                    };
-                    auto setj = [&](int k, int32_t v) {
-                        if constexpr (kJSmem) sj[k * kQueueThreads] = v;
-                        else if constexpr (kJPack)
-                            jpk[k / 2] = __byte_perm(jpk[k / 2], (uint32_t)v, (k & 1) ? 0x5410 : 0x3254);
-                        else jreg[k] = v;
-                    };
-                    S acc[K];
+                    uint32_t jpk[K / 2];
+                    double acc[K];
+                    const float first = s_t[kAhead].band;
 #pragma unroll
                     for (int k = 0; k < K; k++) {
-                        // the initial maximum (-2000, exact) carries the relative part
-                        hi[k] = __fmaf_rn(2000.0f, kRelMix, -2000.0f);
-                        lo[k] = __fmaf_rn(2000.0f, -kRelMix, -2000.0f);
-                        setj(k, -1);
-                        acc[k] = (S)0;
+                        // the initial maximum is -2000; chains off the grid are never
+                        // visible
+                        nmid[k] = active >> k & 1u ? -kMaxAngle : -INFINITY;
+                        hw[k] = active >> k & 1u ? __fmaf_rn(2000.0f, kRel, first) : 0.0f;
+                        jpk[k / 2] = 0xffffffffu;
+                        acc[k] = 0.0;
                     }
-                    // the exact angle of chain k at step st, in the precision's arithmetic
-                    // MIXED64's per-step FP64 values (fp64_step of the staged d):
-                    // the surface addend RN64(d*0.0174533) and RN64(d/R)
-                    auto mix_w = [&](uint32_t st) -> double {
-                        if constexpr (L::kExactTab) return (double)s_x[st].y;
-                        else return __dmul_rn((double)s_t[st].w, 0.0174533);
+                    auto getj = [&](int k) -> int32_t {
+                        const uint32_t v = (jpk[k / 2] >> (16 * (k & 1))) & 0xffffu;
+                        return v == 0xffffu ? -1 : (int32_t)v;
                     };
-                    auto mix_c = [&](uint32_t st) -> double {
-                        if constexpr (L::kExactTab) return (double)s_x[st].x;
-                        else return __ldg(&gdt[st].y);
-                    };
-                    auto exact_at = [&](int k, uint32_t st, float h) -> S {
-                        if constexpr (kMix) {
-                            const double d = (double)s_t[st].w;
-                            const double hp64 = __dadd_rn((double)pov_h(k),
-                                                          (double)D.observer_height);
-                            const double e = __dsub_rn((double)h, hp64);
-#if TVS_MIX_RCP_TABLE
-                            // the shape stage's RN64(1/d), read instead of recomputed
-                            const double y = __ldg(&gdt[st].x);
-#else
-                            const double y = __drcp_rn(d);
-#endif
-                            return __dsub_rn(div_table64(e, y, d), mix_c(st));
-                        } else {
-                            const float e = __fsub_rn(h, hp32[k]);
-                            const float2 x = s_x[st];
-                            return __fsub_rn(div_table32(e, s_t[st].x, x.x), x.y);
-                        }
-                    };
-                    auto exact_max = [&](int k) -> S {
-                        const int32_t j = getj(k);
-                        return j < 0 ? (S)kMaxAngle : exact_at(k, (uint32_t)j, load1((uint32_t)j, k));
-                    };
-                    auto raise = [&](int k, uint32_t st, float fh, float fl, const float4 &t) {
-                        hi[k] = __fmaf_rn(fabsf(fh), kRelMix, fh);
-                        lo[k] = __fmaf_rn(fabsf(fl), -kRelMix, fl);
-                        setj(k, (int32_t)st);
-                        if constexpr (kMix) acc[k] = __dadd_rn(acc[k], mix_w(st));
-                        else acc[k] = __fadd_rn(acc[k], t.w);
-                    };
-                    for (uint32_t seg = 0; i < n_fast; seg++) {
-                        const uint32_t i1 = min(i + kSegSteps, n_fast);
-                        if (skippable(seg, [&](int k, float bound) { return bound < lo[k]; })) {
-                            i = i1;
-                            continue;
-                        }
-                        n_swept += i1 - i;
-                        constexpr int kUnroll = kMix ? TVS_SPLIT_UNROLL_MIX : TVS_SPLIT_UNROLL_EXACT;
-#pragma unroll kUnroll
-                        for (; i < i1; i++) {
-                            const float4 t = s_t[i];  // {y, -c + G, -c - G, w or d}
-                            float e[K], fh[K];
-                            load(i, e);
-                            bool hit = false;
+                    const double4 *gdt = D.dtab + (uint64_t)(a.first_sector + (group >> 1)) * D.step_cap;
+                    auto step = [&](uint32_t st, const Step<kPrec> *p, float (&h)[K]) {
+                        const float y = p->y, z = p->z, band = p->band;
+                        const int next = p->next;
+                        float e[K], f[K], x[K];
+                        estimate(h, y, z, e, f);
+                        load(next, h);
 #pragma unroll
-                            for (int k = 0; k < K; k++) {
-                                e[k] = __fsub_rn(e[k], hp32[k]);  // kernel.rs:164
-                                fh[k] = __fmaf_rn(e[k], t.x, t.y);
-                                hit |= fh[k] >= lo[k];
-                            }
-                            if (!__any_sync(0xffffffffu, hit || prev != 0)) continue;
+                        for (int q = 0; q < K / 2; q++)
+                            upk(add2(pk(f[2 * q], f[2 * q + 1]), pk(nmid[2 * q], nmid[2 * q + 1])),
+                                x[2 * q], x[2 * q + 1]);
+                        bool hit = false;
+#pragma unroll
+                        for (int k = 0; k < K; k++) hit |= x[k] >= -hw[k];
+                        if (__any_sync(0xffffffffu, hit || prev != 0)) {
                             n_passed++;
-                            uint32_t vis = 0, amb = 0;
-                            // the surface addend of this step, read once for the four chains
-                            S w;
-                            if constexpr (kMix) w = mix_w(i);
-                            else w = t.w;
+                            const double w = p->w;
+                            bool amb = false;  // inside the band
 #pragma unroll
-                            for (int k = 0; k < K; k++) {
-                                const bool maybe = fh[k] >= lo[k];
-                                // surely visible: raise the window
-                                const float fl = __fmaf_rn(e[k], t.x, t.z);
-                                const bool sure = fl > hi[k];
-                                if (sure) {
-                                    hi[k] = __fmaf_rn(fabsf(fh[k]), kRelMix, fh[k]);
-                                    lo[k] = __fmaf_rn(fabsf(fl), -kRelMix, fl);
-                                    setj(k, (int32_t)i);
-                                    if constexpr (kMix) acc[k] = __dadd_rn(acc[k], w);
-                                    else acc[k] = __fadd_rn(acc[k], w);
-                                }
-                                vis |= (uint32_t)sure << k;
-                                amb |= (uint32_t)(!sure && maybe) << k;
-                            }
-                            if (__any_sync(0xffffffffu, amb != 0)) {
-                                if (amb) atomicAdd(&ctl.diag[3], (unsigned long long)__popc(amb));
+                            for (int k = 0; k < K; k++) amb |= fabsf(x[k]) <= hw[k];
+                            if (__any_sync(0xffffffffu, amb)) {
+                                uint32_t n_amb = 0;
 #pragma unroll
                                 for (int k = 0; k < K; k++) {
-                                    if (!(amb >> k & 1u)) continue;
-                                    // kernel.rs:190, decided exactly
-                                    if (exact_at(k, i, load1(i, k)) > exact_max(k)) {
-                                        raise(k, i, fh[k], __fmaf_rn(e[k], t.x, t.z), t);
-                                        vis |= 1u << k;
-                                    }
+                                    if (!(fabsf(x[k]) <= hw[k])) continue;
+                                    n_amb++;
+                                    const int32_t j = getj(k);
+                                    if (!mix_visible(load1(s_t[st].next, k), load1(s_t[max(j, 0)].next, k),
+                                                     hp[k], D.observer_height, gdt, st, j))
+                                        x[k] = -INFINITY;
                                 }
+                                if (n_amb) atomicAdd(&ctl.diag[3], (unsigned long long)n_amb);
+                                __syncwarp();
+                            }
+                            // now every chain at or above its band is visible
+                            [[maybe_unused]] uint32_t vis = 0;
+                            if constexpr (kRings) {
+#pragma unroll
+                                for (int k = 0; k < K; k++) vis |= (uint32_t)(x[k] >= -hw[k]) << k;
+                            }
+                            raise_mix<0>(x[0], f[0], e[0], y, z, band, st, w, nmid[0], hw[0], jpk[0], acc[0]);
+                            raise_mix<1>(x[1], f[1], e[1], y, z, band, st, w, nmid[1], hw[1], jpk[0], acc[1]);
+                            raise_mix<0>(x[2], f[2], e[2], y, z, band, st, w, nmid[2], hw[2], jpk[1], acc[2]);
+                            raise_mix<1>(x[3], f[3], e[3], y, z, band, st, w, nmid[3], hw[3], jpk[1], acc[3]);
+                            if constexpr (kRings) events(vis, st);
+                        }
+                    };
+                    sweep_fast([&](int k, float bound) { return __fadd_rn(bound, nmid[k]) < -hw[k]; }, step);
+                    // the steps past the table-division domain (the zero
+                    // distances): exact arithmetic from the exact maximum
+                    if (i < n) {
+                        double m[K];
+#pragma unroll
+                        for (int k = 0; k < K; k++) {
+                            const int32_t j = getj(k);
+                            m[k] = kMaxAngle;
+                            if (j >= 0)
+                                m[k] = mix_angle(load1(s_t[j].next, k), hp[k], D.observer_height, gdt,
+                                                 (uint32_t)j);
+                        }
+                        __syncwarp();
+                        for (; i < n; i++) {
+                            const double4 q = gdt[i];
+                            float hk[K];
+                            load(s_t[i].next, hk);
+                            uint32_t vis = 0;
+#pragma unroll
+                            for (int k = 0; k < K; k++) {
+                                const double hp64 = __dadd_rn((double)hp[k], (double)D.observer_height);
+                                const double ang =
+                                    __dsub_rn(__ddiv_rn(__dsub_rn((double)hk[k], hp64), q.w), q.y);
+                                const bool v = ang > m[k];
+                                if (v) acc[k] = __dadd_rn(acc[k], q.z);
+                                m[k] = fmax(ang, m[k]);
+                                vis |= (uint32_t)v << k;
                             }
                             if constexpr (kRings) events(vis, i);
                         }
-                    }
-                    // the steps past the table-division domain (the zero
-                    // distances): exact arithmetic from the exact maximum
-                    S m[K];
-#pragma unroll
-                    for (int k = 0; k < K; k++) m[k] = exact_max(k);
-                    for (; i < n; i++) {
-                        float hk[K];
-                        load(i, hk);
-                        uint32_t vis = 0;
-#pragma unroll
-                        for (int k = 0; k < K; k++) {
-                            const float h = hk[k];
-                            S ang;
-                            if constexpr (kMix) {
-                                const double d = (double)s_t[i].w;
-                                const double hp64 = __dadd_rn((double)pov_h(k),
-                                                              (double)D.observer_height);
-                                ang = __dsub_rn(__ddiv_rn(__dsub_rn((double)h, hp64), d), mix_c(i));
-                            } else {
-                                const float2 x = s_x[i];
-                                const bool fast = x.x >= 0x1p-20f && x.x <= 0x1p20f;
-                                const float e = __fsub_rn(h, hp32[k]);
-                                ang = __fsub_rn(fast ? div_table32(e, s_t[i].x, x.x) : __fdiv_rn(e, x.x), x.y);
-                            }
-                            const bool v = ang > m[k];
-                            if (v) {
-                                if constexpr (kMix) acc[k] = __dadd_rn(acc[k], mix_w(i));
-                                else acc[k] = __fadd_rn(acc[k], s_t[i].w);
-                            }
-                            if constexpr (kMix) m[k] = fmax(ang, m[k]);
-                            else m[k] = fmaxf(ang, m[k]);  // f32::max: NaN yields the other
-                            vis |= (uint32_t)v << k;
-                        }
-                        if constexpr (kRings) events(vis, i);
                     }
 #pragma unroll
                     for (int k = 0; k < K; k++) out[k] = acc[k];
@@ -778,12 +922,12 @@ k_sweep_split(QueueArgs a) {
                 if constexpr (kRings) {
                     // kernel.rs:237-243: close a ring cut off by the line of
                     // sight, then the count in slot 0
-                    const long long b_last = n ? orig(n - 1) : 0;
+                    const long long o_last = n ? orig(n - 1) : 0;
                     uint32_t most = 0, over = 0;
 #pragma unroll
                     for (int k = 0; k < K; k++) {
                         if (!(active >> k & 1u)) continue;
-                        if (prev >> k & 1u) ring_put(kid(k), ++nr[k], dem_id(k, b_last));
+                        if (prev >> k & 1u) ring_put(kid(k), ++nr[k], dem_id(k, o_last));
                         ring_put(kid(k), 0, nr[k]);
                         most = max(most, nr[k]);
                         over += nr[k] >= a.ref_reserved;
@@ -795,116 +939,211 @@ k_sweep_split(QueueArgs a) {
                         if (most) atomicMax(&a.ring_counters[2], most);
                     }
                 }
-#pragma unroll
-                for (int k = 0; k < K; k++) {
-                    if (dir == 0) s_fwd[k * kQueueThreads + tid] = out[k];
-                    else sb[k] = out[k];
-                }
             };
-            using Fwd = std::integral_constant<int, 0>;
-            using Bwd = std::integral_constant<int, 1>;
-            using Quad = std::false_type;
             if constexpr (kQuad) {
-                if (ctl.plain) {
-                    pass(Fwd{}, std::true_type{});
-                    pass(Bwd{}, std::true_type{});
-                } else {
-                    pass(Fwd{}, Quad{});
-                    pass(Bwd{}, Quad{});
-                }
+                if (uni(sl.plain)) pass(std::true_type{});
+                else pass(std::false_type{});
             } else {
-                pass(Fwd{}, Quad{});
-                pass(Bwd{}, Quad{});
+                pass(std::false_type{});
             }
-            if (a.diag || a.rechecks) {
-                if (lane == 0) {
-                    atomicAdd(&ctl.diag[0], (unsigned long long)n_swept);
-                    atomicAdd(&ctl.diag[1], (unsigned long long)n_passed);
-                    atomicAdd(&ctl.diag[2], 2ull * n_fast);
+            n_all += n_fast;
+
+            // ---- the surfaces, in order ---------------------------------------
+            auto point = [&](int k) -> uint64_t {
+                return (uint64_t)(ty + RS * (k / KX)) * D.tvs_width + tx + LX * (k % KX);
+            };
+            if (a.planes) {
+                S *plane = reinterpret_cast<S *>(a.planes) +
+                           ((size_t)group * a.tiles_per_sector + D.done_base + tile) * (32 * K) + lane;
+#pragma unroll
+                for (int k = 0; k < K; k++) __stcg(plane + 32 * k, out[k]);
+            } else {
+                // the tile's previous item must be complete
+                bool ok = true;
+                if (group > 0) {
+                    const volatile uint32_t *d = a.done + D.done_base + tile;
+                    const volatile int32_t *err = a.error;
+                    uint32_t spins = 0;
+                    while (!__all_sync(0xffffffffu, *d >= group)) {
+                        // give up at the limit, or soon when another wait already did
+                        spins++;
+                        if (spins > a.spin_limit ||
+                            ((spins & 15u) == 0 && __any_sync(0xffffffffu, *err != 0))) {
+                            if (lane == 0) atomicExch(a.error, (int32_t)TVS_ERR_TIMEOUT);
+                            ok = false;
+                            break;
+                        }
+                        __nanosleep(256);
+                    }
+                    __threadfence();
+                    __syncwarp();
                 }
-            }
-            const bool write = queue_wait_prev(a, ctl, D, s, tile, tid);  // every thread
-            if (write) {
 #pragma unroll
                 for (int k = 0; k < K; k++) {
-                    const uint32_t col = tx + LX * (k % KX), row = ty + LY * (k / KX);
-                    if (col >= D.tvs_width || row >= D.row_end) continue;
-                    const uint64_t p = (uint64_t)row * D.tvs_width + col;
-                    // forward surface first (kernel.rs:254); in L2: another SM
-                    // wrote the previous sector's values
+                    if (!ok || !(active >> k & 1u)) continue;
+                    const uint64_t p = point(k);
+                    // in L2: another SM wrote the previous item's values
                     if constexpr (kMix) {
-                        const double cum = __dadd_rn(
-                            __dadd_rn(__ldcg(D.cumulative64 + p), s_fwd[k * kQueueThreads + tid]), sb[k]);
+                        const double cum = __dadd_rn(__ldcg(D.cumulative64 + p), out[k]);
                         __stcg(D.cumulative64 + p, cum);
-                        const float c32 = __double2float_rn(cum);
-                        __stcg(D.cumulative + p, c32);
-                        if (D.total) __stcg(D.total + p, __fadd_rn(__ldcg(D.total + p), c32));
+                        if (dir) {
+                            const float c32 = __double2float_rn(cum);
+                            __stcg(D.cumulative + p, c32);
+                            if (D.total) __stcg(D.total + p, __fadd_rn(__ldcg(D.total + p), c32));
+                        }
                     } else {
-                        const float cum = __fadd_rn(
-                            __fadd_rn(__ldcg(D.cumulative + p), s_fwd[k * kQueueThreads + tid]), sb[k]);
+                        const float cum = __fadd_rn(__ldcg(D.cumulative + p), out[k]);
                         __stcg(D.cumulative + p, cum);
-                        if (D.total) __stcg(D.total + p, __fadd_rn(__ldcg(D.total + p), cum));  // compute.rs:206-214
+                        if (dir && D.total)  // compute.rs:206-214
+                            __stcg(D.total + p, __fadd_rn(__ldcg(D.total + p), cum));
                     }
                 }
             }
-            if (tid == 0 && (a.diag || a.rechecks)) {
-                if (a.diag) {
-                    atomicAdd(&a.diag[0], ctl.diag[0]);
-                    atomicAdd(&a.diag[1], ctl.diag[1]);
-                    atomicAdd(&a.diag[2], ctl.diag[2]);
+        }
+        if (!a.planes) {
+            __threadfence();  // this lane's surface writes before the tile's counter
+            __syncwarp();
+            if (lane == 0 && D.done_base + tile != a.held_tile)
+                atomicAdd(a.done + D.done_base + tile, 1u);
+        } else {
+            // Release only: an acquiring fence invalidates the SM's L1, which holds
+            // the DEM for 32 warps; one per tile and launch (the last item's below)
+            // does, one per item left 37-48 % of the sectors hitting.
+            __syncwarp();
+            uint32_t before = 0;
+            if (lane == 0) before = add_release(a.done + D.done_base + tile, 1u);
+            before = uni(before);
+            if (before == 2 * a.n_sectors - 1) {
+                // the tile's last item: its planes of every sector, in order
+                __threadfence();
+                __syncwarp();
+                const uint32_t per = 8 * D.tiles_x, stripe = tile / per, in = tile - stripe * per;
+                const uint32_t rows = min(8u, D.tiles_y - 8 * stripe);
+                const uint32_t bx = in / rows, by = 8 * stripe + in - bx * rows;
+                const uint32_t tx = bx * (KX * LX) + lane % LX;
+                const uint32_t ty = D.row_begin + by * (LY * KY) + lane / LX * LS;
+                const size_t stride = (size_t)a.tiles_per_sector * (32 * K);  // between groups
+                const S *plane = reinterpret_cast<const S *>(a.planes) +
+                                 (size_t)(D.done_base + tile) * (32 * K) + lane;
+                bool on[K];
+                uint64_t p[K];
+                S cum[K];
+                float total[K], c32[K];
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    const uint32_t col = tx + LX * (k % KX), row = ty + RS * (k / KX);
+                    on[k] = col < D.tvs_width && row < D.row_end;
+                    p[k] = on[k] ? (uint64_t)row * D.tvs_width + col : 0;
+                    if constexpr (kMix) cum[k] = on[k] ? __ldcg(D.cumulative64 + p[k]) : 0.0;
+                    else cum[k] = on[k] ? __ldcg(D.cumulative + p[k]) : 0.0f;
+                    total[k] = on[k] && D.total ? __ldcg(D.total + p[k]) : 0.0f;
+                    c32[k] = 0.0f;
                 }
-                if (a.rechecks && ctl.diag[3]) atomicAdd(a.rechecks, ctl.diag[3]);
+                bool any = false;
+                constexpr int kAhead = 2;  // sectors whose planes are read together
+                for (uint32_t s0 = 0; s0 < a.n_sectors; s0 += kAhead) {
+                    S f[kAhead][K], b[kAhead][K];
+                    bool ok[kAhead];
+#pragma unroll
+                    for (int q = 0; q < kAhead; q++) {
+                        const uint32_t s = s0 + q;
+                        ok[q] = s < a.n_sectors && __ldg(&D.hdr[a.first_sector + s].status) == TVS_OK;
+#pragma unroll
+                        for (int k = 0; k < K; k++) {
+                            f[q][k] = ok[q] ? __ldcg(plane + (size_t)(2 * s) * stride + 32 * k) : (S)0;
+                            b[q][k] = ok[q] ? __ldcg(plane + (size_t)(2 * s + 1) * stride + 32 * k) : (S)0;
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < kAhead; q++) {
+                        if (!ok[q]) continue;
+                        any = true;
+#pragma unroll
+                        for (int k = 0; k < K; k++) {
+                            if constexpr (kMix) {
+                                cum[k] = __dadd_rn(__dadd_rn(cum[k], f[q][k]), b[q][k]);
+                                c32[k] = __double2float_rn(cum[k]);
+                            } else {
+                                cum[k] = __fadd_rn(__fadd_rn(cum[k], f[q][k]), b[q][k]);
+                                c32[k] = cum[k];
+                            }
+                            total[k] = __fadd_rn(total[k], c32[k]);  // compute.rs:206-214
+                        }
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    if (!on[k] || !any) continue;
+                    if constexpr (kMix) __stcg(D.cumulative64 + p[k], cum[k]);
+                    __stcg(D.cumulative + p[k], c32[k]);
+                    if (D.total) __stcg(D.total + p[k], total[k]);
+                }
             }
         }
-        queue_done(a, D, tile, tid);
+        if (owe) {  // the next chunk's slot was still in use
+            bool ok = true;
+            if (chunk + 1 >= n_slots)
+                ok = wait_for(&reinterpret_cast<SplitSlot *>(slot_of(chunk + 1))->left, kWarps);
+            if (!ok) break;
+            bring(chunk + 1);
+        }
+    }
+    if (a.diag && lane == 0) {
+        atomicAdd(&ctl.diag[0], (unsigned long long)n_swept);
+        atomicAdd(&ctl.diag[1], (unsigned long long)n_passed);
+        atomicAdd(&ctl.diag[2], (unsigned long long)n_all);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (a.diag)
+            for (int q = 0; q < 3; q++) atomicAdd(&a.diag[q], ctl.diag[q]);
+        if (a.rechecks && ctl.diag[3]) atomicAdd(a.rechecks, ctl.diag[3]);
     }
 }
 
-template <int kPrec, int kLayout, bool kRings, bool kLean>
-cudaError_t launch_split_t(const QueueArgs &a, cudaStream_t s) {
-    const size_t smem = SplitSmem<kPrec, kLean>::total(a.max_step_cap);
-    return launch_persistent(
-        reinterpret_cast<const void *>(&k_sweep_split<kPrec, kLayout, kRings, kLean>), a, smem, s);
+// Chunks in the ring: three where they leave the SM's CTAs room, else two.
+template <int kPrec, bool kRings>
+cudaError_t ring_slots(uint32_t step_cap, uint32_t *n_slots) {
+    int dev = 0, per_sm = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+    const size_t three = SplitSmem<kPrec>::total(step_cap, 3) * split_min_blocks<kRings>();
+    *n_slots = three <= (size_t)per_sm / 2 ? 3 : 2;
+    return e;
 }
 
-template <int kPrec, bool kRings, bool kLean = false>
+template <int kPrec, int kLayout, bool kRings>
+cudaError_t launch_split_t(const QueueArgs &a, cudaStream_t s) {
+    uint32_t n_slots = 2;
+    const cudaError_t e = ring_slots<kPrec, kRings>(a.max_step_cap, &n_slots);
+    if (e != cudaSuccess) return e;
+    const size_t smem = SplitSmem<kPrec>::total(a.max_step_cap, n_slots);
+    return launch_persistent(
+        reinterpret_cast<const void *>(&k_sweep_split<kPrec, kLayout, kRings>), a,
+        (uint64_t)a.chunks * a.n_sectors * 2, dim3(32 * split_warps<kRings>()), smem, s, n_slots);
+}
+
+template <int kPrec, bool kRings>
 cudaError_t launch_split_layout(const QueueArgs &a, int layout, cudaStream_t s) {
     switch (layout) {
-    case 1: return launch_split_t<kPrec, 1, kRings, kLean>(a, s);
-    case 2: return launch_split_t<kPrec, 2, kRings, kLean>(a, s);
-    case 3: return launch_split_t<kPrec, 3, kRings, kLean>(a, s);
-    case 4: return launch_split_t<kPrec, 4, kRings, kLean>(a, s);
-    case 5: return launch_split_t<kPrec, 5, kRings, kLean>(a, s);
-    case 6: return launch_split_t<kPrec, 6, kRings, kLean>(a, s);
-    case 7: return launch_split_t<kPrec, 7, kRings, kLean>(a, s);
-    case 8: return launch_split_t<kPrec, 8, kRings, kLean>(a, s);
-    case 9: return launch_split_t<kPrec, 9, kRings, kLean>(a, s);
+    case 1: return launch_split_t<kPrec, 1, kRings>(a, s);
+    case 2: return launch_split_t<kPrec, 2, kRings>(a, s);
+    case 3: return launch_split_t<kPrec, 3, kRings>(a, s);
+    case 4: return launch_split_t<kPrec, 4, kRings>(a, s);
+    case 5: return launch_split_t<kPrec, 5, kRings>(a, s);
+    case 6: return launch_split_t<kPrec, 6, kRings>(a, s);
+    case 7: return launch_split_t<kPrec, 7, kRings>(a, s);
+    case 8: return launch_split_t<kPrec, 8, kRings>(a, s);
+    case 9: return launch_split_t<kPrec, 9, kRings>(a, s);
     default: return cudaErrorInvalidValue;
     }
 }
 
-// MIXED64 surfaces run the lean form when it keeps more CTAs per SM (up to
-// the register limit) than the default form's tables allow.
-cudaError_t mix_lean(uint32_t step_cap, bool *lean) {
-    int dev = 0, per_sm = 0, reserved = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess)
-        e = cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-    if (e == cudaSuccess)
-        e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
-    if (e != cudaSuccess) return e;
-    auto ctas = [&](size_t smem) {
-        return std::min<size_t>(split_min_blocks<TVS_PRECISION_MIXED64, false>(),
-                                (size_t)per_sm / (smem + (size_t)reserved));
-    };
-    *lean = ctas(SplitSmem<TVS_PRECISION_MIXED64, true>::total(step_cap)) >
-            ctas(SplitSmem<TVS_PRECISION_MIXED64>::total(step_cap));
-    return cudaSuccess;
-}
-
 }  // namespace
 
-cudaError_t launch_persistent(const void *fn, const QueueArgs &a, size_t smem, cudaStream_t s) {
+cudaError_t launch_persistent(const void *fn, const QueueArgs &a, uint64_t items, dim3 block,
+                              size_t smem, cudaStream_t s, uint32_t n_slots) {
     struct Occ {
         size_t attr = 0, smem = 0;
         int blocks = -1;
@@ -935,7 +1174,7 @@ cudaError_t launch_persistent(const void *fn, const QueueArgs &a, size_t smem, c
             int b = 0, per_sm = 0, reserved = 0;
             e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
             if (e == cudaSuccess)
-                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, kQueueThreads, smem);
+                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, (int)(block.x * block.y), smem);
             if (e == cudaSuccess)
                 e = cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
             if (e == cudaSuccess)
@@ -948,7 +1187,7 @@ cudaError_t launch_persistent(const void *fn, const QueueArgs &a, size_t smem, c
                 int b2 = 0;
                 e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
                 if (e == cudaSuccess)
-                    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, fn, kQueueThreads, smem);
+                    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, fn, (int)(block.x * block.y), smem);
                 if (e != cudaSuccess) return e;
                 if (b2 < b) {  // the rounding lost a CTA: keep the largest carveout
                     e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
@@ -960,26 +1199,38 @@ cudaError_t launch_persistent(const void *fn, const QueueArgs &a, size_t smem, c
         }
         blocks_per_sm = o.blocks;
     }
-    if (a.done_total > a.done_cap) return cudaErrorInvalidValue;
-    e = cudaMemsetAsync(a.queue, 0, sizeof(uint32_t), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(a.done, 0, (size_t)a.done_total * sizeof(uint32_t), s);
+    if (a.done_total > a.done_cap || a.done != a.queue + 1) return cudaErrorInvalidValue;
+    // the tile counters follow the queue counter in memory
+    e = cudaMemsetAsync(a.queue, 0, ((size_t)a.done_total + 1) * sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    const uint64_t items = (uint64_t)a.tiles_per_sector * a.n_sectors;
     const uint32_t grid = (uint32_t)std::min<uint64_t>((uint64_t)blocks_per_sm * sms, items);
     QueueArgs args = a;
-    void *params[] = {&args};
-    e = cudaLaunchKernel(fn, dim3(grid), dim3(kQueueTileX, kQueueTileY), params, smem, s);
+    void *params[] = {&args, &n_slots};  // (the row kernels take the first only)
+    e = cudaLaunchKernel(fn, dim3(grid), block, params, smem, s);
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
 }
 
 size_t split_smem_bytes(int precision, uint32_t step_cap) {
     switch (precision) {
-    case TVS_PRECISION_EXACT32: return SplitSmem<TVS_PRECISION_EXACT32>::total(step_cap);
-    case TVS_PRECISION_MIXED64: return SplitSmem<TVS_PRECISION_MIXED64>::total(step_cap);
-    case TVS_PRECISION_FP32: return SplitSmem<TVS_PRECISION_FP32>::total(step_cap);
+    case TVS_PRECISION_EXACT32: return SplitSmem<TVS_PRECISION_EXACT32>::total(step_cap, 2);
+    case TVS_PRECISION_MIXED64: return SplitSmem<TVS_PRECISION_MIXED64>::total(step_cap, 2);
+    case TVS_PRECISION_FP32: return SplitSmem<TVS_PRECISION_FP32>::total(step_cap, 2);
     default: return 0;
     }
+}
+
+size_t split_plane_bytes(int precision, const QueueConfig &c, uint32_t tiles_per_sector,
+                         uint32_t n_sectors, uint32_t *sectors) {
+    *sectors = 0;
+    if (c.layout == 0 || tiles_per_sector == 0) return 0;
+    const size_t one = precision == TVS_PRECISION_MIXED64 ? sizeof(double) : sizeof(float);
+    const size_t sector = (size_t)2 * tiles_per_sector * 32 * K * one;
+    // launches of about even size
+    const size_t fit = std::min<size_t>(n_sectors, std::max<size_t>(kPlaneBytes / sector, 1));
+    const uint32_t launches = (uint32_t)((n_sectors + fit - 1) / fit);
+    *sectors = (n_sectors + launches - 1) / launches;
+    return *sectors * sector;
 }
 
 cudaError_t launch_sweep_split(const QueueArgs &a, int precision, int layout, cudaStream_t s) {
@@ -991,17 +1242,12 @@ cudaError_t launch_sweep_split(const QueueArgs &a, int precision, int layout, cu
     case TVS_PRECISION_EXACT32:
         return rings ? launch_split_layout<TVS_PRECISION_EXACT32, true>(a, layout, s)
                      : launch_split_layout<TVS_PRECISION_EXACT32, false>(a, layout, s);
-    case TVS_PRECISION_MIXED64: {
+    case TVS_PRECISION_MIXED64:
         // 16-bit steps (0xffff marks the initial maximum): at most 65535 steps,
         // a step table of at most 65536 entries (its length rounds up to 4)
-        if (TVS_MIX_JREG && a.max_step_cap > 0x10000u) return cudaErrorInvalidValue;
-        if (rings) return launch_split_layout<TVS_PRECISION_MIXED64, true>(a, layout, s);
-        bool lean = false;
-        const cudaError_t e = mix_lean(a.max_step_cap, &lean);
-        if (e != cudaSuccess) return e;
-        return lean ? launch_split_layout<TVS_PRECISION_MIXED64, false, true>(a, layout, s)
-                    : launch_split_layout<TVS_PRECISION_MIXED64, false>(a, layout, s);
-    }
+        if (a.max_step_cap > 0x10000u) return cudaErrorInvalidValue;
+        return rings ? launch_split_layout<TVS_PRECISION_MIXED64, true>(a, layout, s)
+                     : launch_split_layout<TVS_PRECISION_MIXED64, false>(a, layout, s);
     case TVS_PRECISION_FP32:
         return rings ? launch_split_layout<TVS_PRECISION_FP32, true>(a, layout, s)
                      : launch_split_layout<TVS_PRECISION_FP32, false>(a, layout, s);

@@ -26,8 +26,10 @@ struct tvs_context {
     float4 *d_steps = nullptr;
     int2 *d_offs = nullptr;
     double4 *d_dtab = nullptr;
+    int2 *d_quads = nullptr;             // split sweep: quad-copy offsets per step
+    int4 *d_segs = nullptr;              // split sweep: offset ranges per segment
     // persistent-sweep work queue
-    uint32_t *d_queue = nullptr;
+    uint32_t *d_queue = nullptr;  // the queue counter, then the tile counters (d_done)
     uint32_t *d_done = nullptr;
     uint32_t done_cap = 0;
     int32_t *d_error = nullptr;
@@ -39,7 +41,9 @@ struct tvs_context {
     tvs::QueueDem *d_qdem = nullptr;           // this context as a one-DEM queue
     tvs::QueueConfig qcfg{0, 0, 0, 0, 0};            // sweep configuration (autotuned or default)
     tvs::QueueConfig qcfg_uploaded{0, 0, 0, 0, 0};   // the tiling currently in d_qdem
-    uint32_t q_tiles_per_sector = 0;
+    uint32_t q_tiles_per_sector = 0, q_chunks = 0;
+    void *d_planes = nullptr;                  // split_plane_bytes (grown on use)
+    size_t planes_cap = 0;
     uint32_t spin_limit = tvs::kDefaultSpinLimit;  // dependency-wait iteration limit
     uint32_t held_tile = 0xFFFFFFFFu;               // failure-detection test hook
     int32_t *d_deltas = nullptr;
@@ -53,7 +57,7 @@ struct tvs_context {
     uint32_t compact_slots = 64;               // slots per band behind the compact stream
     tvs::QueueDem *d_qdem_rings = nullptr;     // this context tiled for the ring sweep
     uint32_t ring_layout = 0;                  // the ring sweep's split layout
-    uint32_t q_ring_tiles = 0;
+    uint32_t q_ring_tiles = 0, q_ring_chunks = 0;
     // plain-kernel scratch (allocated on first use)
     float *d_sf = nullptr, *d_sb = nullptr;
     // band shapes installed as tables (the reference's shape cache), in place of

@@ -37,7 +37,7 @@ constexpr uint32_t kBlockMax = TVS_BLOCK_MAX;
 // row's end.  The sweep's step offsets are 32-bit byte offsets, so the four
 // copies must lie within 2^31 bytes (quad_fits).
 constexpr int kQuadLayout = 9;     // the split layout that reads them
-constexpr int kQuadFallback = 7;   // the same tiling from the plain DEM
+constexpr int kQuadFallback = 8;   // the same tiling from the plain DEM
 constexpr uint32_t kQuadPad = 64;
 __host__ __device__ constexpr uint32_t quad_groups(uint32_t height) { return (height + 48) / 4 + 2; }
 __host__ __device__ constexpr uint64_t quad_copy_elems(uint32_t width, uint32_t height) {
@@ -84,8 +84,26 @@ struct ShapeHeader {
     int64_t min_off;       // min over {0, offsets of evaluated steps}
     int64_t max_off;
     uint32_t n_fast;       // steps before the first kStepSlowDivide step
+    uint32_t n_surf;       // steps up to the last one whose distance is not zero: the
+                           // zero-distance steps after it add 0 to every surface
+    uint32_t wide;         // a step moves more than the line of sight sideways
     uint32_t pad;
 };
+
+// Steps per segment of the direction-split sweep: the samples of a segment are
+// bounded together.
+constexpr uint32_t kSegSteps = 32;
+__host__ __device__ constexpr uint32_t seg_count(uint32_t steps) {
+    return (steps + kSegSteps - 1) / kSegSteps;
+}
+
+// A step's forward DEM offset (cells) as (x, y): |x| < W/2 on every band of
+// sight, and |y| <= the line of sight (the shape stage's path check).
+__host__ __device__ inline void step_xy(long long off, long long W, long long &dx, long long &dy) {
+    const long long q = off + W / 2;
+    dy = q >= 0 ? q / W : -((W - 1 - q) / W);
+    dx = off - dy * W;
+}
 
 // Per-sector sweep launches read their step table from constant memory, so
 // every table value is a warp-uniform operand (no shared-memory loads, no
@@ -115,6 +133,13 @@ struct ShapeArgs {
     double4 *dtab;             // [sectors][step_cap] FP64 {1/d, d/R, d*tan1, d}
     int32_t *deltas;           // [sectors][band_deltas_size]
     float *dists;              // [sectors][band_deltas_size]
+    // For the direction-split sweep (nullable): each step's forward and backward
+    // offset in the quad copies, in float4, and each segment's range of forward
+    // (x, y) offsets {x0, x1, y0, y1}.
+    int2 *quads;               // [sectors][step_cap]
+    int4 *segs;                // [sectors][seg_count(step_cap)]
+    uint32_t rho;              // (first computed row + line of sight) mod 4
+    uint64_t quad_copy;        // float4 per quad copy
     // Optional debug outputs for sector 0 of the launch (tvs_axes):
     uint32_t *sector_ids_out;  // ranks [dbg_first, dbg_first + dbg_count)
     uint64_t dbg_first, dbg_count;
@@ -159,6 +184,8 @@ struct QueueDem {
     const float4 *steps;
     const int2 *offs;
     const double4 *dtab;               // FP64 tables {1/d, d/R, d*tan1, d} (double)
+    const int2 *quads;                 // quad-copy offsets {forward, backward}
+    const int4 *segs;                  // segment offset ranges {x0, x1, y0, y1}
     float *cumulative;
     float *total;                      // nullable
     double *cumulative64;              // FP64/MIXED64 only
@@ -168,6 +195,8 @@ struct QueueDem {
     uint32_t tiles_x, tiles_y;         // set by queue_tile
     uint32_t tile_base;                // first item of this DEM within a sector
     uint32_t done_base;                // this DEM's per-tile counters in `done`
+    uint32_t chunk_base;               // split sweep: first chunk within a sector and direction
+    uint32_t chunk;                    // split sweep: tiles per chunk
 };
 
 struct QueueArgs {
@@ -175,6 +204,9 @@ struct QueueArgs {
     uint32_t n_dems;
     uint32_t first_sector, n_sectors;  // absolute sector slots
     uint32_t tiles_per_sector;         // sum of tiles_x * tiles_y
+    uint32_t chunks;                   // split sweep: chunks of a sector and direction
+    void *planes;                      // split sweep: every tile's surfaces per sector and
+                                       // direction, summed by its last item (null: in turn)
     uint32_t max_step_cap;
     uint32_t *queue;                   // [1] next work item
     uint32_t *done;                    // [done_cap] sectors completed per tile
@@ -189,6 +221,7 @@ struct QueueArgs {
     // launch): band k's count at rings[k * ring_reserved], its ids in slots
     // 1 .. ring_reserved - 1, further ids as {k lo, k hi, slot, id} in spill.
     uint32_t *rings;
+    uint32_t first_record_sector;      // the sector whose records are the first in `rings`
     uint32_t ring_reserved;            // slots per band in `rings`
     uint32_t ref_reserved;             // the reference's slots per band (statistics)
     uint64_t half_bands;               // computable points of the whole grid
@@ -209,6 +242,7 @@ struct QueueArgs {
 struct QueueConfig {
     int px, py, packed, prefetch, layout;
 };
+constexpr int kSplitPoints = 4;  // points of view per lane of the split layouts
 
 struct PlainArgs {
     const float *elev;
@@ -286,7 +320,11 @@ QueueConfig default_queue_config(int precision);
 QueueConfig default_split_config(int precision);
 // Sets tiles_x/tiles_y/tile_base/done_base of every DEM for the configuration.
 void queue_tile(QueueDem *dems, uint32_t n_dems, const QueueConfig &c, uint32_t *tiles_per_sector,
-                uint32_t *done_total);
+                uint32_t *done_total, uint32_t *chunks);
+// Bytes of the surface planes that a split sweep over that many tiles per sector
+// wants, and the sectors that one of its launches then takes (at most n_sectors).
+size_t split_plane_bytes(int precision, const QueueConfig &c, uint32_t tiles_per_sector,
+                         uint32_t n_sectors, uint32_t *sectors);
 cudaError_t launch_shape_batch(const ShapeArgs *d_args, uint32_t n_dems, uint32_t n_sectors,
                                cudaStream_t s);
 cudaError_t launch_combine(float *cum, float *total, const float *sf, const float *sb,
