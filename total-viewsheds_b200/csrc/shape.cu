@@ -8,13 +8,16 @@
 //
 //  1. Along one DEM row the sector projection x*sin - y*cos is monotone in x,
 //     and so are its f32 cast and radix key.  The number of points with key < K
-//     is therefore a sum of per-row binary searches (H * log2(W) evaluations
-//     instead of W*H).
-//  2. A binary search over the 32-bit key space finds the keys K_lo, K_hi of
-//     the first and last window ranks, and count(key < K_lo).
-//  3. The points with K_lo <= key <= K_hi (the window plus key ties) are
-//     gathered into shared memory and sorted by (key, id): radsort is stable,
-//     so this is exactly the reference's sector order on those ranks.
+//     is therefore a sum over the rows of the place where the row crosses K: a
+//     guess from the projection solved for x, which two exact evaluations on
+//     either side of it confirm or move.
+//  2. A bisection over the keys brackets those of the first and last window
+//     ranks, from the keys that a uniform density over the square gives these
+//     ranks; it ends as soon as the points between the outer bounds fit the sort
+//     that the window needs anyway.
+//  3. The points between the bounds are gathered into shared memory and sorted
+//     by (key, id): radsort is stable, so this is exactly the reference's sector
+//     order on those ranks.
 //  4. The window is sorted by (sight key, id), which orders it by
 //     sight_ordered_map rank (band_of_sight.rs:135-145), and the delta and
 //     distance tables are derived from the strip (band_of_sight.rs:149-170).
@@ -43,69 +46,128 @@ __device__ __forceinline__ uint32_t key_at(uint32_t x, double right, double s) {
     return f32_radix_key(projection32(x, right, s));
 }
 
-// Number of x in [x0, x0 + S) whose key is < K.  Keys are non-decreasing in x
-// when s >= 0 and non-increasing when s < 0.
-__device__ uint32_t row_count_less(uint64_t K, double right, double s, uint32_t x0, uint32_t S) {
-    uint32_t lo = 0, hi = S;
-    if (!(s < 0.0)) {
-        while (lo < hi) {
-            uint32_t mid = (lo + hi) >> 1;
-            if ((uint64_t)key_at(x0 + mid, right, s) < K) lo = mid + 1; else hi = mid;
-        }
-        return lo;
-    }
-    while (lo < hi) {
-        uint32_t mid = (lo + hi) >> 1;
-        if ((uint64_t)key_at(x0 + mid, right, s) < K) hi = mid; else lo = mid + 1;
-    }
-    return S - lo;
+// The largest float below which no key < K lies, as the place where a projection
+// crosses from keys < K to keys >= K: halfway between the floats of K - 1 and K.
+__device__ __forceinline__ double key_threshold(uint64_t K) {
+    auto value = [](uint32_t k) -> double {
+        return (double)__uint_as_float((k & 0x80000000u) ? k ^ 0x80000000u : ~k);
+    };
+    if (K == 0 || K > 0xFFFFFFFFull) return K == 0 ? -INFINITY : INFINITY;
+    return 0.5 * (value((uint32_t)K) + value((uint32_t)K - 1u));
 }
 
-template <typename T>
-__device__ T block_sum(T v, T *scratch) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+// Number of x in [x0, x0 + S) whose key is < K (T = key_threshold(K), inv = 1 / s).
+// Keys are non-decreasing in x when s >= 0 and non-increasing when s < 0, so the
+// count is the first x of the other side.  The guess (T + right) / s is off by a
+// rounding at most; where it is not (an infinite T, s near 0) the search falls back
+// to bisection.
+__device__ uint32_t row_count_less(uint64_t K, double T, double right, double s, double inv,
+                                   uint32_t x0, uint32_t S) {
+    const bool up = !(s < 0.0);
+    auto past = [&](uint32_t x) -> bool {  // x is on the far side of the crossing
+        return ((uint64_t)key_at(x0 + x, right, s) < K) != up;
+    };
+    const double g = ceil((T + right) * inv - (double)x0);
+    uint32_t lo = 0, hi = S;  // the first x past the crossing is in [lo, hi]
+    uint32_t x = g >= (double)S ? S : g > 0.0 ? (uint32_t)g : 0u;  // (a NaN gives 0)
+    if (x < hi && !past(x)) {
+        lo = x + 1;
+        if (lo < hi && past(lo)) hi = lo;
+    } else {
+        hi = x;
+        if (hi > lo && !past(hi - 1)) lo = hi;
+    }
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (past(mid)) hi = mid; else lo = mid + 1;
+    }
+    return up ? lo : S - lo;
+}
+
+// Reduction of one value per thread over the CTA (op commutative; scratch holds a
+// value per warp).
+template <typename T, typename Op>
+__device__ T block_reduce(T v, T *scratch, Op op) {
+    for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     __syncthreads();
     if (lane == 0) scratch[warp] = v;
     __syncthreads();
-    T r = 0;
     const int nw = (blockDim.x + 31) >> 5;
-    for (int w = 0; w < nw; w++) r += scratch[w];
+    T r = scratch[lane < nw ? lane : 0];
+    for (int o = 16; o > 0; o >>= 1) r = op(r, __shfl_xor_sync(0xffffffffu, r, o));
     return r;
 }
+static_assert(kShapeThreads == 1024, "32 warps, one value per lane in the second round");
 
 // Sum over the rows of the window of count(key < K), two thresholds at once.
-__device__ void count_less2(uint64_t K0, uint64_t K1, double c, double s, uint32_t x0,
+__device__ void count_less2(uint64_t K0, uint64_t K1, double c, double s, double inv, uint32_t x0,
                             uint32_t y0, uint32_t S, uint64_t *out0, uint64_t *out1,
                             unsigned long long *scratch) {
+    const double T0 = key_threshold(K0), T1 = key_threshold(K1);
     unsigned long long a = 0, b = 0;
     for (uint32_t r = threadIdx.x; r < S; r += blockDim.x) {
         double right = row_term(y0 + r, c);
-        a += row_count_less(K0, right, s, x0, S);
-        b += row_count_less(K1, right, s, x0, S);
+        a += row_count_less(K0, T0, right, s, inv, x0, S);
+        b += row_count_less(K1, T1, right, s, inv, x0, S);
     }
-    *out0 = block_sum(a, scratch);
-    *out1 = block_sum(b, scratch + 32);
+    // both counts are at most 2^31 - 1: one 64-bit sum
+    const unsigned long long both =
+        block_reduce(a << 32 | b, scratch, [](unsigned long long p, unsigned long long q) { return p + q; });
+    *out0 = both >> 32;
+    *out1 = both & 0xFFFFFFFFull;
 }
 
+// Bitonic sort of n_pow2 values in shared memory (one CTA).  The exchanges over
+// less than a warp run in registers, all of a merge's in one pass.
 __device__ void bitonic_sort(unsigned long long *v, uint32_t n_pow2) {
     for (uint32_t k = 2; k <= n_pow2; k <<= 1) {
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = threadIdx.x; i < n_pow2; i += blockDim.x) {
-                uint32_t ixj = i ^ j;
-                if (ixj > i) {
-                    unsigned long long a = v[i], b = v[ixj];
-                    bool up = (i & k) == 0;
-                    if ((a > b) == up) { v[i] = b; v[ixj] = a; }
+        uint32_t j = k >> 1;
+        for (; j >= 32; j >>= 1) {
+            for (uint32_t t = threadIdx.x; t < n_pow2 / 2; t += blockDim.x) {
+                const uint32_t i = 2 * t - (t & (j - 1)), ixj = i + j;  // the t-th pair
+                const unsigned long long a = v[i], b = v[ixj];
+                const bool up = (i & k) == 0;
+                if ((a > b) == up) {
+                    v[i] = b;
+                    v[ixj] = a;
                 }
+            }
+            __syncthreads();
+        }
+        if (k >= 32) {  // j is 16 here
+            for (uint32_t i = threadIdx.x; i < n_pow2; i += blockDim.x) {
+                unsigned long long a = v[i];
+                const bool up = (i & k) == 0;
+                for (uint32_t q = j; q > 0; q >>= 1) {
+                    const unsigned long long b = __shfl_xor_sync(0xffffffffu, a, q);
+                    const bool low = (i & q) == 0;  // this lane keeps the smaller one
+                    if ((a > b) == (low == up)) a = b;
+                }
+                v[i] = a;
+            }
+            __syncthreads();
+        } else if (k == 16) {  // every merge of less than a warp at once
+            for (uint32_t i = threadIdx.x; i < n_pow2; i += blockDim.x) {
+                unsigned long long a = v[i];
+                for (uint32_t m = 2; m <= 16; m <<= 1) {
+                    const bool up = (i & m) == 0;
+                    for (uint32_t q = m >> 1; q > 0; q >>= 1) {
+                        const unsigned long long b = __shfl_xor_sync(0xffffffffu, a, q);
+                        const bool low = (i & q) == 0;
+                        if ((a > b) == (low == up)) a = b;
+                    }
+                }
+                v[i] = a;
             }
             __syncthreads();
         }
     }
 }
 
+// (at least a warp, which the sort's register passes need)
 __device__ __forceinline__ uint32_t next_pow2(uint32_t n) {
-    uint32_t p = 1;
+    uint32_t p = 32;
     while (p < n) p <<= 1;
     return p;
 }
@@ -118,17 +180,19 @@ __device__ void block_inclusive_scan(long long *v, uint32_t n, long long *scratc
     const uint32_t e = min(n, b + per);
     long long local = 0;
     for (uint32_t i = b; i < e; i++) local += v[i];
-    // exclusive scan of the per-thread sums through shared memory
-    __syncthreads();
-    scratch[threadIdx.x] = local;
-    __syncthreads();
-    for (uint32_t off = 1; off < T; off <<= 1) {
-        long long add = threadIdx.x >= off ? scratch[threadIdx.x - off] : 0;
-        __syncthreads();
-        scratch[threadIdx.x] += add;
-        __syncthreads();
+    // exclusive scan of the per-thread sums: in the warp, then over the warps
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    long long incl = local;
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
     }
-    long long run = scratch[threadIdx.x] - local;
+    __syncthreads();
+    if (lane == 31) scratch[warp] = incl;
+    __syncthreads();
+    long long before = lane < warp ? scratch[lane] : 0;
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    long long run = before + incl - local;
     for (uint32_t i = b; i < e; i++) { run += v[i]; v[i] = run; }
     __syncthreads();
 }
@@ -193,15 +257,9 @@ __device__ void finish_shape(const ShapeArgs &a, uint32_t sector, uint32_t n_fil
             if (dx > los || dx < -los) sm.wide = 1;
         }
     }
-    __syncthreads();
-    sm.scan[threadIdx.x] = first_slow;
-    __syncthreads();
-    for (uint32_t o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sm.scan[threadIdx.x] = min(sm.scan[threadIdx.x], sm.scan[threadIdx.x + o]);
-        __syncthreads();
-    }
-    const uint32_t n_fast = (uint32_t)sm.scan[0];
-    __syncthreads();
+    const auto least = [](long long p, long long q) { return p < q ? p : q; };
+    const auto most = [](long long p, long long q) { return p > q ? p : q; };
+    const uint32_t n_fast = (uint32_t)block_reduce((long long)first_slow, sm.scan, least);
     // the offset range of each segment of fast steps, one warp per segment
     if (a.segs) {
         const uint32_t lane = threadIdx.x & 31u;
@@ -218,22 +276,8 @@ __device__ void finish_shape(const ShapeArgs &a, uint32_t sector, uint32_t n_fil
                 a.segs[(uint64_t)sector * seg_count(a.step_cap) + sg] = make_int4(x0, x1, y0, y1);
         }
     }
-    // block min / max through the scan scratch
-    sm.scan[threadIdx.x] = mn;
-    __syncthreads();
-    for (uint32_t o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sm.scan[threadIdx.x] = min(sm.scan[threadIdx.x], sm.scan[threadIdx.x + o]);
-        __syncthreads();
-    }
-    const long long min_off = sm.scan[0];
-    __syncthreads();
-    sm.scan[threadIdx.x] = mx;
-    __syncthreads();
-    for (uint32_t o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sm.scan[threadIdx.x] = max(sm.scan[threadIdx.x], sm.scan[threadIdx.x + o]);
-        __syncthreads();
-    }
-    const long long max_off = sm.scan[0];
+    const long long min_off = block_reduce(mn, sm.scan, least);
+    const long long max_off = block_reduce(mx, sm.scan, most);
     if (threadIdx.x == 0) {
         // kernel.rs:157-164: every band of every point of view stays on the DEM.
         const long long size = (long long)a.size;
@@ -266,29 +310,52 @@ __device__ __forceinline__ void shape_sector(const ShapeArgs &a, const uint32_t 
     const uint32_t S = a.win, X0 = a.x0, Y0 = a.y0;
     const uint64_t rank_hi = rank_lo + rank_count - 1;
 
-    // 1-2. Keys of ranks rank_lo and rank_hi in the sector order.
-    uint64_t lo0 = 0, hi0 = 0xFFFFFFFFull, lo1 = 0, hi1 = 0xFFFFFFFFull;
-    for (int it = 0; it < 33 && (lo0 < hi0 || lo1 < hi1); it++) {
+    // 1-2. Keys around ranks rank_lo and rank_hi in the sector order.  The points
+    // have unit density, so a rank r lies (r - middle) / chord along the axis from
+    // the square's centre; rows and columns make that wrong by about a spacing.
+    // Bounds that do not hold are replaced by the whole key range.
+    const double sn = tr.sector_sin, cs = tr.sector_cos, inv = 1.0 / sn;
+    const double chord = (double)S / fmax(fabs(sn), fabs(cs));
+    const double mid_x = X0 + 0.5 * (S - 1), mid_y = Y0 + 0.5 * (S - 1);
+    const double centre = mid_x * sn + mid_y * cs, middle_rank = 0.5 * ((double)S * S - 1.0);
+    auto key_of = [](double v) -> uint64_t { return f32_radix_key(__double2float_rn(v)); };
+    const double est0 = centre + ((double)rank_lo - middle_rank) / chord;
+    const double est1 = centre + ((double)rank_hi - middle_rank) / chord;
+    constexpr double kSlack = 2.0;  // spacings
+    uint64_t lo0 = key_of(est0 - kSlack), hi0 = key_of(est0 + kSlack);
+    uint64_t lo1 = key_of(est1 - kSlack), hi1 = key_of(est1 + kSlack);
+    uint64_t less_lo, le_hi;  // points with key < lo0, with key <= hi1
+    uint64_t c0, c1;
+    count_less2(lo0, hi1 + 1, cs, sn, inv, X0, Y0, S, &less_lo, &le_hi, sm.red);
+    count_less2(hi0 + 1, lo1, cs, sn, inv, X0, Y0, S, &c0, &c1, sm.red);
+    if (less_lo > rank_lo || c0 <= rank_lo) {
+        lo0 = 0, hi0 = 0xFFFFFFFFull, less_lo = 0;
+    }
+    const uint64_t points = (uint64_t)S * S;
+    if (le_hi <= rank_hi || c1 > rank_hi) {
+        lo1 = 0, hi1 = 0xFFFFFFFFull, le_hi = points;
+    }
+    // Any bounds around the window serve; the sort takes a power of two.
+    const uint64_t enough = min(max(next_pow2((uint32_t)rank_count), 512u), kCandidateCap);
+    for (int it = 0; it < 33 && (lo0 < hi0 || lo1 < hi1) && le_hi - less_lo > enough; it++) {
         uint64_t mid0 = lo0 + ((hi0 - lo0) >> 1);
         uint64_t mid1 = lo1 + ((hi1 - lo1) >> 1);
-        uint64_t c0, c1;
-        count_less2(mid0 + 1, mid1 + 1, tr.sector_cos, tr.sector_sin, X0, Y0, S, &c0, &c1, sm.red);
-        if (lo0 < hi0) { if (c0 > rank_lo) hi0 = mid0; else lo0 = mid0 + 1; }
-        if (lo1 < hi1) { if (c1 > rank_hi) hi1 = mid1; else lo1 = mid1 + 1; }
+        count_less2(mid0 + 1, mid1 + 1, cs, sn, inv, X0, Y0, S, &c0, &c1, sm.red);
+        if (lo0 < hi0) { if (c0 > rank_lo) hi0 = mid0; else { lo0 = mid0 + 1; less_lo = c0; } }
+        if (lo1 < hi1) { if (c1 > rank_hi) { hi1 = mid1; le_hi = c1; } else lo1 = mid1 + 1; }
     }
-    const uint64_t K_lo = lo0, K_hi = lo1;
-    uint64_t less_lo, le_hi;
-    count_less2(K_lo, K_hi + 1, tr.sector_cos, tr.sector_sin, X0, Y0, S, &less_lo, &le_hi, sm.red);
+    const uint64_t K_lo = lo0, K_hi = hi1;
 
     // 3. Gather the candidates (every point with K_lo <= key <= K_hi).
     if (threadIdx.x == 0) { sm.n_cand = 0; sm.status = TVS_OK; }
     __syncthreads();
-    const bool inc = !(tr.sector_sin < 0.0);
+    const double T_lo = key_threshold(K_lo), T_hi = key_threshold(K_hi + 1);
+    const bool inc = !(sn < 0.0);
     for (uint32_t r = threadIdx.x; r < S; r += blockDim.x) {
         const uint32_t row = Y0 + r;
         double right = row_term(row, tr.sector_cos);
-        uint32_t b = row_count_less(K_lo, right, tr.sector_sin, X0, S);
-        uint32_t e = row_count_less(K_hi + 1, right, tr.sector_sin, X0, S);
+        uint32_t b = row_count_less(K_lo, T_lo, right, sn, inv, X0, S);
+        uint32_t e = row_count_less(K_hi + 1, T_hi, right, sn, inv, X0, S);
         if (e <= b) continue;
         uint32_t x0 = X0 + (inc ? b : S - e);
         uint32_t n = e - b;
@@ -297,7 +364,7 @@ __device__ __forceinline__ void shape_sector(const ShapeArgs &a, const uint32_t 
             if (at + k >= kCandidateCap) break;
             uint32_t x = x0 + k;
             uint32_t id = row * W + x;
-            cand[at + k] = ((unsigned long long)key_at(x, right, tr.sector_sin) << 32) | id;
+            cand[at + k] = ((unsigned long long)key_at(x, right, sn) << 32) | id;
         }
     }
     __syncthreads();
@@ -419,14 +486,8 @@ k_shape_tables(ShapeArgs a, const int32_t *tab_deltas, const float *tab_dists,
         sdist[i] = x;
         if (d != 0 || __float_as_uint(x) != 0u) last = (long long)i + 1;
     }
-    __syncthreads();
-    sm.scan[threadIdx.x] = last;
-    __syncthreads();
-    for (uint32_t o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sm.scan[threadIdx.x] = max(sm.scan[threadIdx.x], sm.scan[threadIdx.x + o]);
-        __syncthreads();
-    }
-    const uint32_t n_filled = (uint32_t)sm.scan[0];
+    const uint32_t n_filled = (uint32_t)block_reduce(
+        last, sm.scan, [](long long p, long long q) { return p > q ? p : q; });
     __syncthreads();
     const uint32_t n_steps = n_filled + min(bds - n_filled, 2u);
     block_inclusive_scan(soff, n_filled, sm.scan);
