@@ -69,3 +69,51 @@ def test_mixed64_guard_band_observer_heights(tvs, oracle, synth, observer):
                 cum = np.zeros(eng.count, np.float32)
                 eng.compute_sector(angle, cum)
                 assert np.array_equal(bits(cum), bits(want.astype(np.float32))), (observer, angle)
+
+
+@pytest.mark.parametrize("w,h,los,rows,observer,relief", [
+    (301, 301, 100, None, 1.65, 1500.0), (340, 262, 87, (11, 77), 0.0, 40.0),
+    (173, 173, 57, None, -3.0, 9000.0)])
+def test_fp64_split_form_equals_the_rows_and_the_oracle(tvs, oracle, synth, w, h, los, rows, observer,
+                                                        relief):
+    """FP64 by default evaluates angles where its first test passes; the row
+    kernel (a configuration set by hand) evaluates every step.  Whole metres and a
+    flat sea give exact ties."""
+    z = np.round(synth.fbm(w, h, 0.7, 9, 0.0, relief))
+    z[:h // 4] = 0.0
+    with tvs.Engine(z, w, 30.0, los * 30, height=h, observer_height=observer, precision="fp64",
+                    rows=rows) as eng:
+        c0 = eng.sweep_config()
+        assert (c0.points_x, c0.points_y, c0.layout) == (2, 1, 0)
+        split = eng.run()[:2]
+        eng.set_queue_wait(held_tile=IN_TURN)
+        turn = eng.run()[:2]
+        eng.set_queue_wait()
+        eng.set_sweep_config(2, 1)
+        row = eng.run()[:2]
+        cfg = eng.autotune(2)
+        assert cfg.layout == 0
+        tuned = eng.run()[:2]
+    for other in (turn, row, tuned):
+        for a, b in zip(split, other):
+            assert np.array_equal(bits(a), bits(b))
+    if rows is None:
+        g = oracle.geometry(w, 30.0, los * 30, height=h)
+        want = oracle.run_f64(g, z, observer)[0].astype(np.float32)
+        assert np.array_equal(bits(split[0]), bits(want))
+
+
+def test_fp64_batch_equals_engines(tvs, synth):
+    tiles = [(np.round(synth.fbm(w, h, 0.7, w, 0.0, 900.0)), 30.0, min(w, h) // 3 * 30)
+             for w, h in ((257, 261), (330, 258))]
+    with tvs.Batch(tiles, observer_height=1.65, precision="fp64") as b:
+        b.run()
+        b.finish()
+        got = [b.read(i) for i in range(2)]
+    for (z, s, los), g in zip(tiles, got):
+        with tvs.Engine(z, z.shape[1], s, los, height=z.shape[0], observer_height=1.65,
+                        precision="fp64") as eng:
+            eng.set_sweep_config(4, 1)
+            want = eng.run()[:2]
+        for a, b in zip(g, want):
+            assert np.array_equal(bits(a), bits(b))

@@ -248,15 +248,7 @@ int tvs_batch_geometry(const tvs_batch *b, uint32_t dem, tvs_geometry *out) {
     return tvs_get_geometry(b->dems[dem], out);
 }
 
-int tvs_batch_set_sweep_config(tvs_batch *b, const tvs_sweep_config *cfg) {
-    if (!b || !cfg) return TVS_ERR_INVALID_ARGUMENT;
-    tvs::QueueConfig c{cfg->points_x, cfg->points_y, cfg->packed != 0, cfg->prefetch != 0, cfg->layout};
-    if (!tvs::queue_config_valid(c))
-        return bfail(b, TVS_ERR_INVALID_ARGUMENT, "unsupported points-per-thread shape");
-    if (c.layout != 0 && b->precision == TVS_PRECISION_FP64)
-        return bfail(b, TVS_ERR_INVALID_ARGUMENT, "sweep layouts 1-9 are not available for FP64");
-    if (c.layout == 0 && b->precision == TVS_PRECISION_FP32)
-        return bfail(b, TVS_ERR_INVALID_ARGUMENT, "the FP32 form runs on sweep layouts 1-9 only");
+static int set_config(tvs_batch *b, const tvs::QueueConfig &c) {
     if (c.px != b->cfg.px || c.py != b->cfg.py || c.packed != b->cfg.packed ||
         c.prefetch != b->cfg.prefetch || c.layout != b->cfg.layout) {
         b->cfg = c;
@@ -266,13 +258,21 @@ int tvs_batch_set_sweep_config(tvs_batch *b, const tvs_sweep_config *cfg) {
     return upload_dems(b);
 }
 
+int tvs_batch_set_sweep_config(tvs_batch *b, const tvs_sweep_config *cfg) {
+    if (!b || !cfg) return TVS_ERR_INVALID_ARGUMENT;
+    tvs::QueueConfig c{cfg->points_x, cfg->points_y, cfg->packed != 0, cfg->prefetch != 0, cfg->layout};
+    if (!tvs::queue_config_valid(c))
+        return bfail(b, TVS_ERR_INVALID_ARGUMENT, "unsupported points-per-thread shape");
+    if (c.layout != 0 && b->precision == TVS_PRECISION_FP64)
+        return bfail(b, TVS_ERR_INVALID_ARGUMENT, "sweep layouts 1-9 are not available for FP64");
+    if (c.layout == 0 && b->precision == TVS_PRECISION_FP32)
+        return bfail(b, TVS_ERR_INVALID_ARGUMENT, "the FP32 form runs on sweep layouts 1-9 only");
+    return set_config(b, c);
+}
+
 int tvs_batch_get_sweep_config(const tvs_batch *b, tvs_sweep_config *cfg) {
     if (!b || !cfg) return TVS_ERR_INVALID_ARGUMENT;
-    cfg->points_x = b->cfg.px;
-    cfg->points_y = b->cfg.py;
-    cfg->packed = b->cfg.packed;
-    cfg->prefetch = b->cfg.prefetch;
-    cfg->layout = b->cfg.layout;
+    *cfg = tvs_host::public_config((int)b->precision, b->cfg);
     return TVS_OK;
 }
 
@@ -298,9 +298,11 @@ int tvs_batch_autotune(tvs_batch *b, uint32_t sample_sectors, tvs_sweep_config *
     tvs::QueueConfig best_cfg = b->cfg;
     int rc = TVS_OK;
     for (const tvs::QueueConfig &c : cands) {
-        if ((c.packed && !exact) || (c.layout != 0 && f64) || (c.layout == 0 && fp32)) continue;
-        tvs_sweep_config sc{c.px, c.py, c.packed, c.prefetch, c.layout};
-        if ((rc = tvs_batch_set_sweep_config(b, &sc))) break;
+        // (FP64's split form is tiled as layout 9 and not selected by name)
+        if ((c.packed && !exact) || (c.layout != 0 && c.layout != tvs::kQuadLayout && f64) ||
+            (c.layout == 0 && fp32))
+            continue;
+        if ((rc = set_config(b, c))) break;
         float ms = 0.0f;
         for (int rep = 0; rep < 2 && rc == TVS_OK; rep++) {  // the first run warms up
             cudaEventRecord(t0, b->stream);
@@ -319,9 +321,8 @@ int tvs_batch_autotune(tvs_batch *b, uint32_t sample_sectors, tvs_sweep_config *
     cudaEventDestroy(t0);
     cudaEventDestroy(t1);
     if (rc) return rc;
-    tvs_sweep_config sc{best_cfg.px, best_cfg.py, best_cfg.packed, best_cfg.prefetch, best_cfg.layout};
-    rc = tvs_batch_set_sweep_config(b, &sc);
-    if (rc == TVS_OK && chosen) *chosen = sc;
+    rc = set_config(b, best_cfg);
+    if (rc == TVS_OK && chosen) *chosen = tvs_host::public_config((int)b->precision, b->cfg);
     return rc;
 }
 

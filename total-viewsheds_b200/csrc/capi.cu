@@ -661,6 +661,11 @@ int collect_rings(tvs_context *c, uint32_t *rings, uint64_t rings_len, tvs_secto
 void tvs_set_create_error(const std::string &msg) { g_create_error = msg; }
 
 namespace tvs_host {
+// A sweep configuration as callers see it: FP64's split form is its rows 2x1.
+tvs_sweep_config public_config(int precision, const tvs::QueueConfig &c) {
+    if (precision == TVS_PRECISION_FP64 && c.layout != 0) return tvs_sweep_config{2, 1, 0, 0, 0};
+    return tvs_sweep_config{c.px, c.py, c.packed, c.prefetch, c.layout};
+}
 tvs::ShapeArgs shape_args_of(tvs_context *c, uint32_t first_slot) { return shape_args(c, first_slot); }
 tvs::QueueDem queue_dem_of(const tvs_context *c) { return queue_dem(c); }
 int header_status_of(tvs_context *c, uint32_t first, uint32_t count) {
@@ -780,11 +785,9 @@ int tvs_create(const tvs_params *params, const float *elevations, uint64_t n_ele
             return bail(e, "cudaMalloc");
         c->device_bytes += count * sizeof(double);
     }
-    // the quad layout's copies (4x the DEM); without them (FP64, the plain
-    // kernel, a DEM past the 32-bit offsets, or no memory for them) the quad
+    // the quad layout's copies (4x the DEM); without them (the plain kernel, a DEM past the 32-bit offsets, or no memory for them) the quad
     // layout's tiling runs from the plain DEM
-    if (params->precision != TVS_PRECISION_FP64 && params->sweep_kernel == TVS_SWEEP_ENGINE &&
-        tvs::quad_fits(g.width, g.height)) {
+    if (params->sweep_kernel == TVS_SWEEP_ENGINE && tvs::quad_fits(g.width, g.height)) {
         const size_t qb = 4 * tvs::quad_copy_elems(g.width, g.height) * sizeof(float4);
         if (cudaMalloc(&c->d_quad, qb) == cudaSuccess) {
             c->device_bytes += qb;
@@ -1219,11 +1222,7 @@ int tvs_set_sweep_config(tvs_context *ctx, const tvs_sweep_config *cfg) {
 
 int tvs_get_sweep_config(const tvs_context *ctx, tvs_sweep_config *cfg) {
     if (!ctx || !cfg) return TVS_ERR_INVALID_ARGUMENT;
-    cfg->points_x = ctx->qcfg.px;
-    cfg->points_y = ctx->qcfg.py;
-    cfg->packed = ctx->qcfg.packed;
-    cfg->prefetch = ctx->qcfg.prefetch;
-    cfg->layout = ctx->qcfg.layout;
+    *cfg = tvs_host::public_config((int)ctx->p.precision, ctx->qcfg);
     return TVS_OK;
 }
 
@@ -1250,7 +1249,10 @@ int tvs_autotune(tvs_context *ctx, uint32_t sample_sectors, tvs_sweep_config *ch
     int rc = enqueue_shape(ctx, 0, sample_sectors);
     for (const tvs::QueueConfig &c : cands) {
         if (rc) break;
-        if ((c.packed && !exact) || (c.layout != 0 && f64) || (c.layout == 0 && fp32)) continue;
+        // (FP64's split form is tiled as layout 9 and not selected by name)
+        if ((c.packed && !exact) || (c.layout != 0 && c.layout != tvs::kQuadLayout && f64) ||
+            (c.layout == 0 && fp32))
+            continue;
         ctx->qcfg = c;
         float ms = 0.0f;
         for (int rep = 0; rep < 2 && rc == TVS_OK; rep++) {  // the first run warms up

@@ -603,7 +603,9 @@ bool queue_config_valid(const QueueConfig &c) {
 }
 
 QueueConfig default_queue_config(int precision) {
+    static bool rows = false;  // the environment asks for a row layout
     static QueueConfig v = [] {
+        rows = getenv("TVS_SWEEP_SHAPE") || getenv("TVS_SWEEP_PACKED") || getenv("TVS_SWEEP_PREFETCH");
         QueueConfig d{2, 1, 0, 0, 0};
         const char *e = getenv("TVS_SWEEP_SHAPE");
         int x = 0, y = 0;
@@ -617,7 +619,11 @@ QueueConfig default_queue_config(int precision) {
         if (f) d.prefetch = atoi(f) != 0;
         return d;
     }();
-    if (precision == TVS_PRECISION_FP64) return v;
+    // FP64's split form takes the quad layout's tiling and no other; callers see it
+    // as rows 2x1, the one configuration that FP64 always had by default, and get
+    // the row kernel, which evaluates every step in double, by setting one (1201^2,
+    // 180 sectors: rows 13.5 ms).
+    if (precision == TVS_PRECISION_FP64) return rows ? v : QueueConfig{kSplitCols, 1, 0, 0, kQuadLayout};
     return default_split_config(precision);
 }
 
@@ -669,7 +675,6 @@ cudaError_t launch_sweep_queue(const QueueArgs &a, int precision, const QueueCon
     if (a.n_dems == 0 || a.tiles_per_sector == 0 || a.n_sectors == 0) return cudaSuccess;
     if (!queue_config_valid(c)) return cudaErrorInvalidValue;
     if (c.layout != 0) {  // direction-split layouts (sweep_split.cu)
-        if (precision == TVS_PRECISION_FP64) return cudaErrorInvalidValue;
         return launch_sweep_split(a, precision, c.layout, s);
     }
     const bool mix = precision == TVS_PRECISION_MIXED64;

@@ -47,6 +47,9 @@
 //    proves the sample is not visible, f > mid + hw that it is.  Only between the
 //    two is the comparison re-decided in FP64, against the exact maximum
 //    recomputed from step j.
+//  * FP64: the running maximum is held in double; where the MIXED64 estimate,
+//    raised by its bound, does not prove every chain's sample below the maximum,
+//    the angles are evaluated in double.
 // So every decision is the exact one, and surfaces add the reference's
 // w = RN(d*tan1) in f32 (EXACT32) or RN64(d*0.0174533) in double (MIXED64) in
 // step order: bit for bit the reference f32 sweep and the all-FP64 sweep.
@@ -152,12 +155,18 @@ template <> struct __align__(16) Step<TVS_PRECISION_MIXED64> {
     int next;
     double w, pad;  // RN64(d*0.0174533)
 };
+template <> struct __align__(16) Step<TVS_PRECISION_FP64> {
+    float y, z, d;  // 1/d, -(d/R + o/d) + G, d
+    int next;
+    double y64, c64;  // RN64(1/d), RN64(d/R)
+};
 template <> struct __align__(16) Step<TVS_PRECISION_FP32> {
     float y, z, w;  // 1/d, -d/R, the surface addend
     int next;
 };
 template <int kPrec>
-using Surface = typename std::conditional<kPrec == TVS_PRECISION_MIXED64, double, float>::type;
+using Surface = typename std::conditional<kPrec == TVS_PRECISION_MIXED64 || kPrec == TVS_PRECISION_FP64,
+                                          double, float>::type;
 
 // A segment's bounds in this direction: the range of the offsets and the
 // extremes of 1/d and of the first test's offset.
@@ -202,15 +211,17 @@ template <int kPrec> struct SplitSmem {
 };
 
 // Warps per CTA and CTAs per SM: 32 warps of 64 registers a thread for the surface
-// sweeps; ring output keeps more state (24 warps of 80 registers).  24 warps of 80
-// registers measured slower for the surfaces too (1201^2 exact f32 5.03 against
-// 4.38 ms): the step loop hides its loads with warps.
-constexpr int kRingWarps = 8;
-template <bool kRings> __host__ __device__ constexpr int split_warps() {
-    return kRings ? kRingWarps : kSplitWarps;
+// sweeps; ring output and FP64 keep more state (24 warps of 80 registers).  24 warps
+// of 80 registers measured slower for the other surfaces (1201^2 exact f32 5.03
+// against 4.38 ms): the step loop hides its loads with warps.
+template <int kPrec, bool kRings> __host__ __device__ constexpr int split_sm_warps() {
+    return kRings || kPrec == TVS_PRECISION_FP64 ? 24 : 32;
 }
-template <bool kRings> __host__ __device__ constexpr int split_min_blocks() {
-    return (kRings ? 24 : 32) / split_warps<kRings>();
+template <int kPrec, bool kRings> __host__ __device__ constexpr int split_warps() {
+    return split_sm_warps<kPrec, kRings>() == 32 ? kSplitWarps : 8;
+}
+template <int kPrec, bool kRings> __host__ __device__ constexpr int split_min_blocks() {
+    return split_sm_warps<kPrec, kRings>() / split_warps<kPrec, kRings>();
 }
 
 __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
@@ -306,14 +317,16 @@ __device__ __noinline__ bool mix_visible(float h, float hj, float pov, float obs
     return mix_angle(h, pov, observer, dtab, i) > m;
 }
 template <int kPrec, int kLayout, bool kRings>
-__global__ void __launch_bounds__(32 * split_warps<kRings>(), (split_min_blocks<kRings>()))
+__global__ void __launch_bounds__(32 * split_warps<kPrec, kRings>(), (split_min_blocks<kPrec, kRings>()))
 k_sweep_split(QueueArgs a, uint32_t n_slots) {
     constexpr int LX = split_lx(kLayout), KY = split_ky(kLayout), KX = K / KY, LY = 32 / LX;
     // rows between a lane's chains: the quad layout reads four consecutive ones
     constexpr int RS = kLayout == kQuadLayout ? 1 : LY, LS = kLayout == kQuadLayout ? KY : 1;
-    constexpr int kWarps = split_warps<kRings>();
+    constexpr int kWarps = split_warps<kPrec, kRings>();
     constexpr bool kFp32 = kPrec == TVS_PRECISION_FP32;
     constexpr bool kMix = kPrec == TVS_PRECISION_MIXED64;
+    constexpr bool kF64 = kPrec == TVS_PRECISION_FP64;
+    constexpr bool kWide = kMix || kF64;  // surfaces in double
     constexpr bool kQuad = kLayout == kQuadLayout;
     using L = SplitSmem<kPrec>;
     using S = Surface<kPrec>;
@@ -368,7 +381,7 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
             const int4 *gseg = D.segs + (uint64_t)slot * seg_count(D.step_cap);
             const double4 *gd = D.dtab + (uint64_t)slot * D.step_cap;
             (void)gd;
-            const float hmax = kMix ? *D.hmax : 0.0f;
+            const float hmax = kWide ? *D.hmax : 0.0f;
             // from the last 32 steps to the first: the band needs the largest G of
             // the later steps
             float later = 0.0f;
@@ -380,9 +393,10 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                 if (v) {
                     t = gs[i];  // {RN(1/d), d, RN(d/R), RN(d*tan1)}
                     z = -t.z;
-                    if constexpr (kMix) {
+                    if constexpr (kWide) {
                         z = -__fadd_rn(t.z, __fmul_rn(D.observer_height, t.x));
                         if (i < nf) g = band_mix(t.x, t.z, D.observer_height, hmax);
+                        if constexpr (kF64) z = __fadd_rn(z, g);
                     } else if constexpr (!kFp32) {
                         z = __fadd_rn(z, window_exact(t.z));
                     }
@@ -414,6 +428,10 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                     if constexpr (kMix) {
                         e.band = g;
                         e.w = gd[i].z;
+                    } else if constexpr (kF64) {
+                        e.d = t.y;
+                        e.y64 = gd[i].x;
+                        e.c64 = gd[i].y;
                     } else {
                         e.w = t.w;
                         if constexpr (!kFp32) {
@@ -530,13 +548,13 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
 #pragma unroll
             for (int k = 0; k < K; k++)
                 if (tx + LX * (k % KX) < D.tvs_width && ty + RS * (k / KX) < D.row_end) active |= 1u << k;
-            // kernel.rs:134, the f32 observer elevation (MIXED64: the point of
+            // kernel.rs:134, the f32 observer elevation (MIXED64, FP64: the point of
             // view's own elevation; the observer height is in the step's offset)
             float hp[K];
 #pragma unroll
             for (int k = 0; k < K; k++) {
                 const float h = __ldg(row_ptr(k / KX) + LX * (k % KX));
-                hp[k] = kMix ? h : __fadd_rn(h, D.observer_height);
+                hp[k] = kWide ? h : __fadd_rn(h, D.observer_height);
             }
             f32x2 nhp[K / 2];  // negated, for the packed subtraction
 #pragma unroll
@@ -760,6 +778,66 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                     }
 #pragma unroll
                     for (int k = 0; k < K; k++) out[k] = sf[k];
+                } else if constexpr (kF64) {
+                    // ---- FP64: angles in double where the first test passes -----
+                    // its threshold lo = RN(m) - 2^-20 |RN(m)| leaves 2.6 x the
+                    // estimate's error relative to the angle, as the guard band does
+                    double m[K], acc[K];
+                    float lo[K];
+#pragma unroll
+                    for (int k = 0; k < K; k++) {
+                        const bool on = active >> k & 1u;  // off the grid: never visible
+                        m[k] = on ? (double)kMaxAngle : (double)INFINITY;
+                        lo[k] = on ? __fmaf_rn(2000.0f, -kRel, kMaxAngle) : INFINITY;
+                        acc[k] = 0.0;
+                    }
+                    const double o64 = (double)D.observer_height;
+                    auto step = [&](uint32_t st, const Step<kPrec> *p, float (&h)[K]) {
+                        const float y = p->y, z = p->z;
+                        const int next = p->next;
+                        float e[K], f[K], hs[K];
+                        estimate(h, y, z, e, f);
+#pragma unroll
+                        for (int k = 0; k < K; k++) hs[k] = h[k];
+                        load(next, h);
+                        bool hit = false;
+#pragma unroll
+                        for (int k = 0; k < K; k++) hit |= f[k] >= lo[k];
+                        if (__any_sync(0xffffffffu, hit)) {
+                            n_passed++;
+                            const double d = (double)p->d, y64 = p->y64, c64 = p->c64;
+                            const double w = __dmul_rn(d, 0.0174533);  // kernel.rs:216
+                            // (every chain: a vote per chain to leave out the ones below
+                            // the test measured 6.71 against 6.30 ms at 1201^2)
+#pragma unroll
+                            for (int k = 0; k < K; k++) {
+                                const double hp64 = __dadd_rn((double)hp[k], o64);
+                                const double ang = __dsub_rn(
+                                    div_table64(__dsub_rn((double)hs[k], hp64), y64, d), c64);
+                                const bool v = ang > m[k];  // false for a NaN: m stays (f64::max)
+                                acc[k] = v ? __dadd_rn(acc[k], w) : acc[k];
+                                m[k] = v ? ang : m[k];
+                                const float m32 = __double2float_rn(m[k]);
+                                lo[k] = __fmaf_rn(fabsf(m32), -kRel, m32);
+                            }
+                        }
+                    };
+                    sweep_fast([&](int k, float bound) { return bound < lo[k]; }, step);
+                    for (; i < n; i++) {  // past the table division's domain: IEEE division
+                        const double4 *q = D.dtab + (uint64_t)(a.first_sector + (group >> 1)) * D.step_cap + i;
+                        const double c64 = __ldg(&q->y), w = __ldg(&q->z), d = __ldg(&q->w);
+                        float h[K];
+                        load(s_t[i].next, h);
+#pragma unroll
+                        for (int k = 0; k < K; k++) {
+                            const double hp64 = __dadd_rn((double)hp[k], o64);
+                            const double ang = __dsub_rn(__ddiv_rn(__dsub_rn((double)h[k], hp64), d), c64);
+                            if (ang > m[k]) acc[k] = __dadd_rn(acc[k], w);
+                            m[k] = fmax(ang, m[k]);
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < K; k++) out[k] = acc[k];
                 } else if constexpr (!kMix) {
                     // ---- exact f32, the running maximum held exactly ----------
                     // where the first test passes the reference's angle is computed
@@ -983,7 +1061,7 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                     if (!ok || !(active >> k & 1u)) continue;
                     const uint64_t p = point(k);
                     // in L2: another SM wrote the previous item's values
-                    if constexpr (kMix) {
+                    if constexpr (kWide) {
                         const double cum = __dadd_rn(__ldcg(D.cumulative64 + p), out[k]);
                         __stcg(D.cumulative64 + p, cum);
                         if (dir) {
@@ -1034,7 +1112,7 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                     const uint32_t col = tx + LX * (k % KX), row = ty + RS * (k / KX);
                     on[k] = col < D.tvs_width && row < D.row_end;
                     p[k] = on[k] ? (uint64_t)row * D.tvs_width + col : 0;
-                    if constexpr (kMix) cum[k] = on[k] ? __ldcg(D.cumulative64 + p[k]) : 0.0;
+                    if constexpr (kWide) cum[k] = on[k] ? __ldcg(D.cumulative64 + p[k]) : 0.0;
                     else cum[k] = on[k] ? __ldcg(D.cumulative + p[k]) : 0.0f;
                     total[k] = on[k] && D.total ? __ldcg(D.total + p[k]) : 0.0f;
                     c32[k] = 0.0f;
@@ -1060,7 +1138,7 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                         any = true;
 #pragma unroll
                         for (int k = 0; k < K; k++) {
-                            if constexpr (kMix) {
+                            if constexpr (kWide) {
                                 cum[k] = __dadd_rn(__dadd_rn(cum[k], f[q][k]), b[q][k]);
                                 c32[k] = __double2float_rn(cum[k]);
                             } else {
@@ -1074,7 +1152,7 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
 #pragma unroll
                 for (int k = 0; k < K; k++) {
                     if (!on[k] || !any) continue;
-                    if constexpr (kMix) __stcg(D.cumulative64 + p[k], cum[k]);
+                    if constexpr (kWide) __stcg(D.cumulative64 + p[k], cum[k]);
                     __stcg(D.cumulative + p[k], c32[k]);
                     if (D.total) __stcg(D.total + p[k], total[k]);
                 }
@@ -1108,7 +1186,7 @@ cudaError_t ring_slots(uint32_t step_cap, uint32_t *n_slots) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-    const size_t three = SplitSmem<kPrec>::total(step_cap, 3) * split_min_blocks<kRings>();
+    const size_t three = SplitSmem<kPrec>::total(step_cap, 3) * split_min_blocks<kPrec, kRings>();
     *n_slots = three <= (size_t)per_sm / 2 ? 3 : 2;
     return e;
 }
@@ -1121,7 +1199,7 @@ cudaError_t launch_split_t(const QueueArgs &a, cudaStream_t s) {
     const size_t smem = SplitSmem<kPrec>::total(a.max_step_cap, n_slots);
     return launch_persistent(
         reinterpret_cast<const void *>(&k_sweep_split<kPrec, kLayout, kRings>), a,
-        (uint64_t)a.chunks * a.n_sectors * 2, dim3(32 * split_warps<kRings>()), smem, s, n_slots);
+        (uint64_t)a.chunks * a.n_sectors * 2, dim3(32 * split_warps<kPrec, kRings>()), smem, s, n_slots);
 }
 
 template <int kPrec, bool kRings>
@@ -1213,6 +1291,7 @@ cudaError_t launch_persistent(const void *fn, const QueueArgs &a, uint64_t items
 
 size_t split_smem_bytes(int precision, uint32_t step_cap) {
     switch (precision) {
+    case TVS_PRECISION_FP64: return SplitSmem<TVS_PRECISION_FP64>::total(step_cap, 2);
     case TVS_PRECISION_EXACT32: return SplitSmem<TVS_PRECISION_EXACT32>::total(step_cap, 2);
     case TVS_PRECISION_MIXED64: return SplitSmem<TVS_PRECISION_MIXED64>::total(step_cap, 2);
     case TVS_PRECISION_FP32: return SplitSmem<TVS_PRECISION_FP32>::total(step_cap, 2);
@@ -1224,7 +1303,8 @@ size_t split_plane_bytes(int precision, const QueueConfig &c, uint32_t tiles_per
                          uint32_t n_sectors, uint32_t *sectors) {
     *sectors = 0;
     if (c.layout == 0 || tiles_per_sector == 0) return 0;
-    const size_t one = precision == TVS_PRECISION_MIXED64 ? sizeof(double) : sizeof(float);
+    const size_t one = precision == TVS_PRECISION_MIXED64 || precision == TVS_PRECISION_FP64
+                           ? sizeof(double) : sizeof(float);
     const size_t sector = (size_t)2 * tiles_per_sector * 32 * K * one;
     // launches of about even size
     const size_t fit = std::min<size_t>(n_sectors, std::max<size_t>(kPlaneBytes / sector, 1));
@@ -1248,6 +1328,11 @@ cudaError_t launch_sweep_split(const QueueArgs &a, int precision, int layout, cu
         if (a.max_step_cap > 0x10000u) return cudaErrorInvalidValue;
         return rings ? launch_split_layout<TVS_PRECISION_MIXED64, true>(a, layout, s)
                      : launch_split_layout<TVS_PRECISION_MIXED64, false>(a, layout, s);
+    case TVS_PRECISION_FP64:  // the quad layout's tiling only; ring records elsewhere
+        if (rings) return cudaErrorInvalidValue;
+        return layout == kQuadLayout     ? launch_split_t<TVS_PRECISION_FP64, kQuadLayout, false>(a, s)
+               : layout == kQuadFallback ? launch_split_t<TVS_PRECISION_FP64, kQuadFallback, false>(a, s)
+                                         : cudaErrorInvalidValue;
     case TVS_PRECISION_FP32:
         return rings ? launch_split_layout<TVS_PRECISION_FP32, true>(a, layout, s)
                      : launch_split_layout<TVS_PRECISION_FP32, false>(a, layout, s);

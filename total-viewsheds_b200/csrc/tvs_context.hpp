@@ -96,6 +96,7 @@ struct tvs_context {
 // Helpers capi.cu shares with the other host files of the library.
 void tvs_set_create_error(const std::string &msg);
 namespace tvs_host {
+tvs_sweep_config public_config(int precision, const tvs::QueueConfig &c);
 tvs::ShapeArgs shape_args_of(tvs_context *c, uint32_t first_slot);
 tvs::QueueDem queue_dem_of(const tvs_context *c);
 int header_status_of(tvs_context *c, uint32_t first, uint32_t count);
