@@ -21,6 +21,7 @@ thread_local std::string g_create_error;
 constexpr double kRadsPerDeg = 3.14159265358979323846 / 180.0;  // Rust f64::to_radians
 constexpr double kSqrt2 = 1.41421356237309504880;               // core::f64::consts::SQRT_2
 constexpr uint32_t kSpillCap = 1u << 22;
+constexpr size_t kSmallPlanes = (size_t)4 << 20;  // planes that a new context comes with
 
 int fail(tvs_context *ctx, int code, const std::string &msg) {
     if (ctx) ctx->err = msg; else g_create_error = msg;
@@ -778,6 +779,22 @@ int tvs_create(const tvs_params *params, const float *elevations, uint64_t n_ele
     for (auto &a : allocs) {
         if ((e = cudaMalloc(a.p, a.bytes)) != cudaSuccess) return bail(e, "cudaMalloc");
         c->device_bytes += a.bytes;
+    }
+    // a small grid's planes for one sector, so that the first call of a per-sector
+    // loop allocates nothing
+    if (params->sweep_kernel == TVS_SWEEP_ENGINE) {
+        tvs::QueueDem d{};
+        d.tvs_width = g.tvs_width;
+        d.row_begin = rb;
+        d.row_end = re;
+        uint32_t tiles = 0, done = 0, chunks = 0, per = 0;
+        tvs::queue_tile(&d, 1, c->qcfg, &tiles, &done, &chunks);
+        const size_t need = tvs::split_plane_bytes((int)params->precision, c->qcfg, tiles, 1, &per);
+        if (need != 0 && need <= kSmallPlanes) {
+            if ((e = cudaMalloc(&c->d_planes, need)) != cudaSuccess) return bail(e, "cudaMalloc");
+            c->planes_cap = need;
+            c->device_bytes += need;
+        }
     }
     c->d_done = c->d_queue + 1;
     if (params->precision == TVS_PRECISION_MIXED64 || params->precision == TVS_PRECISION_FP64) {

@@ -29,9 +29,13 @@ constexpr int kQueueThreads = kQueueTileX * kQueueTileY;
 // Warps per CTA of the split sweep and warp tiles per chunk of its queue.
 constexpr int kSplitWarps = 16;
 constexpr uint32_t kSplitChunk = kSplitWarps;
-// The split sweep's launches take as many sectors as have planes of surfaces
-// (one per sector and direction) of about this size.
-constexpr size_t kPlaneBytes = (size_t)256 << 20;
+// The split sweep's launches take as many sectors as have planes of surfaces (one
+// per sector and direction) of kPlaneBytes, and kPlaneSectors of a large DEM's up
+// to kPlaneBytesMost: the end of a launch leaves the GPU half idle for one tile's
+// time (12 tiles of up to 1601^2: 65.0, 57.5, 53.6 and 51.8 ms with 32, 64, 128 and
+// 256 MB).
+constexpr size_t kPlaneBytes = (size_t)256 << 20, kPlaneBytesMost = (size_t)1 << 30;
+constexpr uint32_t kPlaneSectors = 16;
 
 // Direction-split layouts 1-9: a warp holds LX columns x 32/LX rows of lanes;
 // each lane sweeps four points of view, LX columns apart (layouts 1-3: LX = 8,

@@ -1307,7 +1307,8 @@ size_t split_plane_bytes(int precision, const QueueConfig &c, uint32_t tiles_per
                            ? sizeof(double) : sizeof(float);
     const size_t sector = (size_t)2 * tiles_per_sector * 32 * K * one;
     // launches of about even size
-    const size_t fit = std::min<size_t>(n_sectors, std::max<size_t>(kPlaneBytes / sector, 1));
+    const size_t budget = std::min(kPlaneBytesMost, std::max(kPlaneBytes, kPlaneSectors * sector));
+    const size_t fit = std::min<size_t>(n_sectors, std::max<size_t>(budget / sector, 1));
     const uint32_t launches = (uint32_t)((n_sectors + fit - 1) / fit);
     *sectors = (n_sectors + launches - 1) / launches;
     return *sectors * sector;
