@@ -78,9 +78,8 @@ namespace tvs {
 namespace {
 
 constexpr int K = kSplitCols;     // chains per lane
-// Iterations of a wait for a chunk of the CTA's own ring (at least 64 ns each:
-// seconds, against a real wait of at most a few work items).
-constexpr uint32_t kRingSpinLimit = 1u << 26;
+// Iterations of a wait for a chunk of the CTA's own ring (of about 100 ns: seconds, against a real wait of at most a few work items).
+constexpr uint32_t kRingSpinLimit = 1u << 25;
 
 __device__ __forceinline__ float div_table32(float e, float y, float d) {
     const float q = __fmul_rn(e, y);
@@ -188,7 +187,8 @@ struct SplitSlot {
 };
 
 struct SplitCtl {
-    uint32_t ready;              // chunks brought in so far
+    uint32_t ready;              // slots brought in so far
+    uint32_t item, upto;         // chunks taken from the queue and not yet in a slot
     unsigned long long diag[4];  // counters, flushed at the end
 };
 
@@ -272,29 +272,29 @@ __device__ __forceinline__ void raise_exact(float ang, float &m, float &s, float
         : "+f"(m), "+f"(s), "+f"(lo)
         : "f"(ang), "f"(w), "f"(-kRelExact));
 }
-// MIXED64, where x = f - mid >= -hw: mid = f (kept negated; computed again, for a
-// predicated multiply-add goes to the FMA pipe and a predicated move to the busier
-// ALU), hw = 2^-20 |f| + band, the surface gains w, and j's half kHi becomes step.
+// MIXED64, where x = f - mid >= -hw: hw = 2^-20 |f| + band, the surface gains w, and
+// j's half kHi becomes step.  The surface takes w times 1.0 or 0.0 in one rounding
+// (the same sum; w is finite and the surface not negative): a predicated FP64 add
+// comes out as two selects, this as one.
 template <int kHi>
-__device__ __forceinline__ void raise_mix(float x, float f, float e, float y, float z, float band,
-                                          uint32_t step, double w, float &nmid, float &hw,
+__device__ __forceinline__ void raise_mix(float x, float f, float band, uint32_t step, double w, float &hw,
                                           uint32_t &j, double &acc) {
     asm("{\n\t"
         ".reg .pred p;\n\t"
         ".reg .f32 a, n;\n\t"
-        "neg.f32 n, %1;\n\t"
-        "setp.ge.f32 p, %4, n;\n\t"
-        "abs.f32 a, %5;\n\t"
-        "neg.f32 n, %6;\n\t"
-        "@p fma.rn.f32 %1, a, %12, %9;\n\t"
-        "neg.f32 a, %8;\n\t"
-        "@p fma.rn.f32 %0, n, %7, a;\n\t"
-        "@p add.rn.f64 %3, %3, %11;\n\t"
-        "@p prmt.b32 %2, %2, %10, %13;\n\t"
+        ".reg .b32 h;\n\t"
+        ".reg .f64 v;\n\t"
+        "neg.f32 n, %0;\n\t"
+        "setp.ge.f32 p, %3, n;\n\t"
+        "abs.f32 a, %4;\n\t"
+        "@p fma.rn.f32 %0, a, %8, %5;\n\t"
+        "selp.b32 h, 0x3ff00000, 0, p;\n\t"
+        "mov.b64 v, {0, h};\n\t"
+        "fma.rn.f64 %2, %7, v, %2;\n\t"
+        "@p prmt.b32 %1, %1, %6, %9;\n\t"
         "}"
-        : "+f"(nmid), "+f"(hw), "+r"(j), "+d"(acc)
-        : "f"(x), "f"(f), "f"(e), "f"(y), "f"(z), "f"(band), "r"(step), "d"(w), "f"(kRel),
-          "n"(kHi ? 0x5410 : 0x3254));
+        : "+f"(hw), "+r"(j), "+d"(acc)
+        : "f"(x), "f"(f), "f"(band), "r"(step), "d"(w), "f"(kRel), "n"(kHi ? 0x5410 : 0x3254));
 }
 
 // A value that every lane holds, in a uniform register: the branches and shared
@@ -341,7 +341,7 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
     const uint32_t warp = uni(threadIdx.x >> 5);
     const uint32_t n_items = a.chunks * a.n_sectors * 2;
     if (threadIdx.x < 4) ctl.diag[threadIdx.x] = 0;
-    if (threadIdx.x == 0) ctl.ready = 0;
+    if (threadIdx.x == 0) ctl.ready = ctl.item = ctl.upto = 0;
     __syncthreads();
 
     // Brings chunk c into its slot (one warp): the next item of the queue and
@@ -351,9 +351,18 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
         SplitSlot &sl = *reinterpret_cast<SplitSlot *>(base);
         Step<kPrec> *s_t = reinterpret_cast<Step<kPrec> *>(base + L::table());
         SegBound *s_seg = reinterpret_cast<SegBound *>(base + L::seg(cap));
-        uint32_t item = 0;
-        if (lane == 0) item = atomicAdd(a.queue, 1u);
-        item = uni(item);
+        // this CTA's chunks [item, upto); more from the queue when it has none left
+        uint32_t item = uni(ctl.item), upto = uni(ctl.upto);
+        __syncwarp();
+        if (item == upto) {
+            constexpr uint32_t kGrab = kSplitGrab * kWarps / kSplitWarps / (kF64 ? 2 : 1);
+            const uint32_t grab = item + 2 * kGrab * gridDim.x < n_items ? kGrab : 1u;
+            item = 0;
+            if (lane == 0) item = atomicAdd(a.queue, grab);
+            item = uni(item);
+            upto = min(item + grab, max(n_items, item));
+        }
+        uint32_t taken = 0;  // of them, in this slot
         if (item < n_items) {
             const uint32_t group = item / a.chunks, r = item - group * a.chunks;
             const uint32_t dir = group & 1u, slot = a.first_sector + (group >> 1);
@@ -457,11 +466,14 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                     }
                 }
             }
+            // the consecutive chunks of this DEM, sector and direction
+            const uint32_t tiles = uni(D.tiles_x * D.tiles_y), per = uni(D.chunk);
+            const uint32_t tile0 = (r - uni(D.chunk_base)) * per;
+            taken = min(upto - item, (tiles - tile0 + per - 1) / per);
             if (lane == 0) {
                 for (uint32_t q = 0; q < kAhead; q++) s_t[n + q].next = 0;  // the point of view itself
-                const uint32_t tiles = D.tiles_x * D.tiles_y;
-                sl.tile0 = (r - D.chunk_base) * D.chunk;
-                sl.n_tiles = min(D.chunk, tiles - sl.tile0);
+                sl.tile0 = tile0;
+                sl.n_tiles = min(taken * per, tiles - tile0);
                 sl.group = group;
                 sl.n = n;
                 sl.n_fast = nf;
@@ -471,6 +483,8 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
         }
         __syncwarp();
         if (lane == 0) {
+            ctl.item = item + taken;
+            ctl.upto = upto;
             sl.next = 0;
             sl.left = 0;
             sl.end = item >= n_items;
@@ -490,7 +504,7 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                 __syncwarp();
                 return false;
             }
-            __nanosleep(64);
+            __nanosleep(100);
         }
         return true;
     };
@@ -815,7 +829,7 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                                 const double ang = __dsub_rn(
                                     div_table64(__dsub_rn((double)hs[k], hp64), y64, d), c64);
                                 const bool v = ang > m[k];  // false for a NaN: m stays (f64::max)
-                                acc[k] = v ? __dadd_rn(acc[k], w) : acc[k];
+                                acc[k] = __fma_rn(w, __hiloint2double(v ? 0x3ff00000 : 0, 0), acc[k]);
                                 m[k] = v ? ang : m[k];
                                 const float m32 = __double2float_rn(m[k]);
                                 lo[k] = __fmaf_rn(fabsf(m32), -kRel, m32);
@@ -935,30 +949,40 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                             bool amb = false;  // inside the band
 #pragma unroll
                             for (int k = 0; k < K; k++) amb |= fabsf(x[k]) <= hw[k];
+                            [[maybe_unused]] uint32_t vis = 0;
                             if (__any_sync(0xffffffffu, amb)) {
                                 uint32_t n_amb = 0;
 #pragma unroll
                                 for (int k = 0; k < K; k++) {
-                                    if (!(fabsf(x[k]) <= hw[k])) continue;
-                                    n_amb++;
-                                    const int32_t j = getj(k);
-                                    if (!mix_visible(load1(s_t[st].next, k), load1(s_t[max(j, 0)].next, k),
-                                                     hp[k], D.observer_height, gdt, st, j))
-                                        x[k] = -INFINITY;
+                                    if (!(x[k] >= -hw[k])) continue;
+                                    if (fabsf(x[k]) <= hw[k]) {
+                                        n_amb++;
+                                        const int32_t j = getj(k);
+                                        if (!mix_visible(load1(s_t[st].next, k), load1(s_t[max(j, 0)].next, k),
+                                                         hp[k], D.observer_height, gdt, st, j))
+                                            continue;
+                                    }
+                                    nmid[k] = -f[k];
+                                    hw[k] = __fmaf_rn(fabsf(f[k]), kRel, band);
+                                    jpk[k / 2] = __byte_perm(jpk[k / 2], st, (k & 1) ? 0x5410 : 0x3254);
+                                    acc[k] = __dadd_rn(acc[k], w);
+                                    vis |= 1u << k;
                                 }
                                 if (n_amb) atomicAdd(&ctl.diag[3], (unsigned long long)n_amb);
                                 __syncwarp();
-                            }
-                            // now every chain at or above its band is visible
-                            [[maybe_unused]] uint32_t vis = 0;
-                            if constexpr (kRings) {
+                            } else {
+                                // outside the band the larger estimate is the maximum's
+                                if constexpr (kRings) {
 #pragma unroll
-                                for (int k = 0; k < K; k++) vis |= (uint32_t)(x[k] >= -hw[k]) << k;
+                                    for (int k = 0; k < K; k++) vis |= (uint32_t)(x[k] >= -hw[k]) << k;
+                                }
+                                raise_mix<0>(x[0], f[0], band, st, w, hw[0], jpk[0], acc[0]);
+                                raise_mix<1>(x[1], f[1], band, st, w, hw[1], jpk[0], acc[1]);
+                                raise_mix<0>(x[2], f[2], band, st, w, hw[2], jpk[1], acc[2]);
+                                raise_mix<1>(x[3], f[3], band, st, w, hw[3], jpk[1], acc[3]);
+#pragma unroll
+                                for (int k = 0; k < K; k++) nmid[k] = fminf(nmid[k], -f[k]);  // a NaN leaves it
                             }
-                            raise_mix<0>(x[0], f[0], e[0], y, z, band, st, w, nmid[0], hw[0], jpk[0], acc[0]);
-                            raise_mix<1>(x[1], f[1], e[1], y, z, band, st, w, nmid[1], hw[1], jpk[0], acc[1]);
-                            raise_mix<0>(x[2], f[2], e[2], y, z, band, st, w, nmid[2], hw[2], jpk[1], acc[2]);
-                            raise_mix<1>(x[3], f[3], e[3], y, z, band, st, w, nmid[3], hw[3], jpk[1], acc[3]);
                             if constexpr (kRings) events(vis, st);
                         }
                     };
