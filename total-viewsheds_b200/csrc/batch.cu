@@ -82,11 +82,14 @@ int upload_dems(tvs_batch *b) {
     const size_t need = tvs::split_plane_bytes((int)b->precision, b->cfg, b->tiles_per_sector,
                                                tvs::kSectorSteps, &per);
     if (need > b->planes_cap) {
-        if (b->d_planes) cudaFree(b->d_planes);
+        if (b->d_planes) {
+            cudaStreamSynchronize(b->stream);
+            tvs::plane_free(b->d_planes, b->stream);
+        }
         b->device_bytes -= b->planes_cap;
         b->d_planes = nullptr;
         b->planes_cap = 0;
-        if (cudaMalloc(&b->d_planes, need) == cudaSuccess) {
+        if (tvs::plane_alloc(&b->d_planes, need, b->stream) == cudaSuccess) {
             b->planes_cap = need;
             b->device_bytes += need;
         } else {
@@ -228,10 +231,10 @@ void tvs_batch_destroy(tvs_batch *b) {
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     drop_graph(b);
-    void *ptrs[] = {b->d_shape, b->d_dems, b->d_queue, b->d_error, b->d_rechecks,
-                    b->d_planes};
+    void *ptrs[] = {b->d_shape, b->d_dems, b->d_queue, b->d_error, b->d_rechecks};
     for (void *p : ptrs)
         if (p) cudaFree(p);
+    if (b->d_planes) tvs::plane_free(b->d_planes, b->stream);
     if (b->stream) cudaStreamDestroy(b->stream);
     for (tvs_context *c : b->dems) tvs_destroy(c);
     delete b;

@@ -148,9 +148,10 @@ void free_all(tvs_context *c) {
                     c->d_deltas, c->d_dists, c->d_rings, c->d_spill, c->d_counters, c->d_sf,
                     c->d_sb, c->d_tab_deltas, c->d_tab_dists, c->d_installed,
                     c->d_rc_blocks, c->d_rc_offsets, c->d_rc_ids, c->d_bmax, c->d_qdem_rings,
-                    c->d_diag, c->d_quad, c->d_planes};
+                    c->d_diag, c->d_quad};
     for (void *p : ptrs)
         if (p) cudaFree(p);
+    if (c->d_planes) tvs::plane_free(c->d_planes, c->stream);
     drop_tvs_graph(c);
     for (cudaEvent_t ev : {c->ev_begin, c->ev_shaped, c->ev_swept})
         if (ev) cudaEventDestroy(ev);
@@ -400,12 +401,15 @@ void *ensure_planes(tvs_context *c, const tvs::QueueConfig &q, uint32_t tiles, u
     const size_t need = tvs::split_plane_bytes((int)c->p.precision, q, tiles, n_sectors, sectors);
     if (need != 0 && c->held_tile == 0xFFFFFFFFu) {
         if (need <= c->planes_cap) return c->d_planes;
-        if (c->d_planes) cudaFree(c->d_planes);
+        if (c->d_planes) {
+            cudaStreamSynchronize(c->stream);
+            tvs::plane_free(c->d_planes, c->stream);
+        }
         c->device_bytes -= c->planes_cap;
         c->d_planes = nullptr;
         c->planes_cap = 0;
         drop_tvs_graph(c);  // a captured sweep holds the old planes
-        if (cudaMalloc(&c->d_planes, need) == cudaSuccess) {
+        if (tvs::plane_alloc(&c->d_planes, need, c->stream) == cudaSuccess) {
             c->planes_cap = need;
             c->device_bytes += need;
             return c->d_planes;
@@ -791,9 +795,13 @@ int tvs_create(const tvs_params *params, const float *elevations, uint64_t n_ele
         tvs::queue_tile(&d, 1, c->qcfg, &tiles, &done, &chunks);
         const size_t need = tvs::split_plane_bytes((int)params->precision, c->qcfg, tiles, 1, &per);
         if (need != 0 && need <= kSmallPlanes) {
-            if ((e = cudaMalloc(&c->d_planes, need)) != cudaSuccess) return bail(e, "cudaMalloc");
-            c->planes_cap = need;
-            c->device_bytes += need;
+            if (tvs::plane_alloc(&c->d_planes, need, c->stream) == cudaSuccess) {
+                c->planes_cap = need;
+                c->device_bytes += need;
+            } else {
+                cudaGetLastError();
+                c->d_planes = nullptr;
+            }
         }
     }
     c->d_done = c->d_queue + 1;

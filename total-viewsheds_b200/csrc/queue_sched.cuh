@@ -42,6 +42,7 @@ constexpr uint32_t kSplitChunk = kSplitWarps, kSplitGrab = 4;
 // 256 MB).
 constexpr size_t kPlaneBytes = (size_t)256 << 20, kPlaneBytesMost = (size_t)1 << 30;
 constexpr uint32_t kPlaneSectors = 16;
+constexpr uint64_t kPlanePoolBytes = (uint64_t)512 << 20;
 
 // Direction-split layouts 1-9: a warp holds LX columns x 32/LX rows of lanes;
 // each lane sweeps four points of view, LX columns apart (layouts 1-3: LX = 8,

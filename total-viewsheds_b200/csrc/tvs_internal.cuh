@@ -323,6 +323,13 @@ void queue_tile(QueueDem *dems, uint32_t n_dems, const QueueConfig &c, uint32_t 
                 uint32_t *done_total, uint32_t *chunks);
 // Bytes of the surface planes that a split sweep over that many tiles per sector
 // wants, and the sectors that one of its launches then takes (at most n_sectors).
+// The planes come from a pool per device, so that a program that opens one DEM
+// after another does not map and unmap them each time (a 301^2 context's 33 MB cost
+// its first run 1 ms): plane_alloc and plane_free order on the stream; while any
+// plane is held the pool keeps up to kPlanePoolBytes of freed ones, and gives all
+// back with the last.
+cudaError_t plane_alloc(void **p, size_t bytes, cudaStream_t s);
+void plane_free(void *p, cudaStream_t s);
 size_t split_plane_bytes(int precision, const QueueConfig &c, uint32_t tiles_per_sector,
                          uint32_t n_sectors, uint32_t *sectors);
 cudaError_t launch_shape_batch(const ShapeArgs *d_args, uint32_t n_dems, uint32_t n_sectors,
