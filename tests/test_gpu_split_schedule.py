@@ -117,3 +117,33 @@ def test_fp64_batch_equals_engines(tvs, synth):
             want = eng.run()[:2]
         for a, b in zip(g, want):
             assert np.array_equal(bits(a), bits(b))
+
+
+@pytest.mark.parametrize("precision", ["exact32", "mixed64", "fp32"])
+@pytest.mark.parametrize("los", [8, 54, 58, 112])
+def test_ring_records_where_segments_are_skipped(tvs, oracle, synth, precision, los):
+    """A ring open before a skipped segment or step closes at its first step: a ridge
+    in front of low ground, where whole segments lie below every horizon, and a
+    flat sea; several sectors per call and one."""
+    w = 3 * los + 5
+    z = synth.fbm(w, w, 0.7, los, 0.0, 30.0)
+    z[::max(los // 2, 3), :] += 900.0
+    z[:, ::max(los // 3, 3)] += 500.0
+    z[: w // 4] = 0.0
+    g = oracle.geometry(w, 30.0, los * 30)
+    mode = ORACLE_MODE[precision]
+    with tvs.Engine(z, w, 30.0, los * 30, observer_height=1.65, precision=precision) as eng:
+        cum = np.zeros(eng.count, np.float32)
+        offsets, ids, _ = eng.compute_sectors_rings(88, 4, cum)
+        per = eng.geometry.total_bands
+        for s in range(4):
+            d, x, _ = oracle.compile_band_data(g, float(88 + s))
+            c0, n0, ids0 = oracle.sweep_sector(g, z, 1.65, d, x, mode=mode, compact=True)
+            one = np.zeros(eng.count, np.float32)
+            o1, i1, _ = eng.compute_sector_rings(88 + s, one)
+            assert np.array_equal(bits(one), bits(c0.astype(np.float32)))
+            assert np.array_equal(np.diff(o1).astype(np.uint32), n0)
+            assert np.array_equal(i1, ids0)
+            span = offsets[s * per:(s + 1) * per + 1]
+            assert np.array_equal(np.diff(span).astype(np.uint32), n0)
+            assert np.array_equal(ids[span[0]:span[-1]], ids0)

@@ -147,7 +147,7 @@ void free_all(tvs_context *c) {
                     c->d_rechecks, c->d_qdem,
                     c->d_deltas, c->d_dists, c->d_rings, c->d_spill, c->d_counters, c->d_sf,
                     c->d_sb, c->d_tab_deltas, c->d_tab_dists, c->d_installed,
-                    c->d_rc_blocks, c->d_rc_offsets, c->d_rc_ids, c->d_bmax, c->d_qdem_rings,
+                    c->d_rc_blocks, c->d_rc_offsets, c->d_rc_lens, c->d_rc_ids, c->d_bmax, c->d_qdem_rings,
                     c->d_diag, c->d_quad};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -425,7 +425,9 @@ void *ensure_planes(tvs_context *c, const tvs::QueueConfig &q, uint32_t tiles, u
 // count is 1 and the sector's ring records go to d_rings with ring_slots u32
 // per band (the reference's reservation for its layout, compact_slots for the
 // compact stream).
-int enqueue_sweep(tvs_context *c, uint32_t first, uint32_t count, uint32_t ring_slots) {
+// lens (nullable, split sweep only): the records' counts go there in place of slot 0.
+int enqueue_sweep(tvs_context *c, uint32_t first, uint32_t count, uint32_t ring_slots,
+                  uint32_t *lens = nullptr) {
     const bool rings = ring_slots != 0;
     if (c->p.sweep_kernel == TVS_SWEEP_PLAIN) {
         int rc = ensure_plain_scratch(c);
@@ -493,6 +495,7 @@ int enqueue_sweep(tvs_context *c, uint32_t first, uint32_t count, uint32_t ring_
         q.rechecks = c->d_rechecks;
         q.diag = c->diag_on ? c->d_diag : nullptr;
         q.rings = c->d_rings;
+        q.ring_lens = lens;
         q.ring_reserved = ring_slots;
         q.ref_reserved = c->g.reserved_rings_per_band;
         q.half_bands = c->g.computable_points_count;
@@ -1032,16 +1035,20 @@ int tvs_compute_sectors_rings(tvs_context *ctx, uint32_t first_angle, uint32_t n
         if (ctx->d_rc_offsets) {
             cudaFree(ctx->d_rc_offsets);
             cudaFree(ctx->d_rc_blocks);
+            cudaFree(ctx->d_rc_lens);
             ctx->device_bytes -= (ctx->rc_records_cap + 1 + tvs::ring_scan_blocks(ctx->rc_records_cap) + 1) *
-                                 sizeof(uint64_t);
+                                     sizeof(uint64_t) +
+                                 ctx->rc_records_cap * sizeof(uint32_t);
             ctx->d_rc_offsets = nullptr;
             ctx->d_rc_blocks = nullptr;
+            ctx->d_rc_lens = nullptr;
             ctx->rc_records_cap = 0;
         }
         TVS_CUDA(ctx, cudaMalloc(&ctx->d_rc_offsets, (recs + 1) * sizeof(uint64_t)));
         TVS_CUDA(ctx, cudaMalloc(&ctx->d_rc_blocks, (nb + 1) * sizeof(uint64_t)));
+        TVS_CUDA(ctx, cudaMalloc(&ctx->d_rc_lens, std::max<uint64_t>(recs, 1) * sizeof(uint32_t)));
         ctx->rc_records_cap = recs;
-        ctx->device_bytes += (recs + 1 + nb + 1) * sizeof(uint64_t);
+        ctx->device_bytes += (recs + 1 + nb + 1) * sizeof(uint64_t) + recs * sizeof(uint32_t);
     }
     {
         int rc = ensure_shapes(ctx, first_angle, n_sectors);
@@ -1052,6 +1059,10 @@ int tvs_compute_sectors_rings(tvs_context *ctx, uint32_t first_angle, uint32_t n
     // per band double and the call runs again from the caller's surfaces (a
     // band has at most n_steps + 2 ids, so this ends).
     const uint32_t most = ctx->g.band_steps_filled + 4;
+    const bool split = ctx->p.sweep_kernel != TVS_SWEEP_PLAIN && ctx->p.precision != TVS_PRECISION_FP64 &&
+                       sweep_impl() == SweepImpl::Queue;
+    const uint32_t *lens = nullptr;
+    uint32_t stride = 0;
     uint32_t R = 0, cnt[4];
     uint64_t total = 0;
     int rc = TVS_OK;
@@ -1064,20 +1075,23 @@ int tvs_compute_sectors_rings(tvs_context *ctx, uint32_t first_angle, uint32_t n
                                           cudaMemcpyHostToDevice, ctx->stream));
         if (ctx->d_cum64 && count)
             TVS_CUDA(ctx, tvs::launch_widen(ctx->d_cum, ctx->d_cum64, count, ctx->stream));
-        // Every band the split sweep covers writes its count (slot 0) and its
-        // ids; the slots past a band's count are never read.  A row shard
-        // leaves the other bands unwritten (their counts must read 0), and the
-        // other sweeps write only where they have ids.
-        if (ctx->row_begin != 0 || ctx->row_end != ctx->g.tvs_height ||
-            ctx->p.sweep_kernel == TVS_SWEEP_PLAIN || ctx->p.precision == TVS_PRECISION_FP64 ||
-            sweep_impl() != SweepImpl::Queue)
+        // Every band the split sweep covers writes its count (to the dense
+        // lengths: 4 bytes a band to scan instead of a 32-byte sector) and its ids;
+        // the slots past a band's count are never read.  A row shard leaves the
+        // other bands unwritten (their counts must read 0), and the other sweeps
+        // count in slot 0 and write only where they have ids.
+        if (!split)
             TVS_CUDA(ctx, cudaMemsetAsync(ctx->d_rings, 0, recs * R * sizeof(uint32_t), ctx->stream));
+        else if (ctx->row_begin != 0 || ctx->row_end != ctx->g.tvs_height)
+            TVS_CUDA(ctx, cudaMemsetAsync(ctx->d_rc_lens, 0, recs * sizeof(uint32_t), ctx->stream));
         TVS_CUDA(ctx, cudaMemsetAsync(ctx->d_counters, 0, 4 * sizeof(uint32_t), ctx->stream));
-        rc = enqueue_sweep(ctx, first_angle, n_sectors, R);
+        rc = enqueue_sweep(ctx, first_angle, n_sectors, R, split ? ctx->d_rc_lens : nullptr);
         if (rc) return rc;
-        // the record lengths (slot 0 holds a band's whole count, spilled ids
-        // included) are scanned before the spill check: one wait for both
-        TVS_CUDA(ctx, tvs::launch_ring_count(ctx->d_rings, recs, R, ctx->d_rc_blocks, ctx->stream));
+        lens = split ? ctx->d_rc_lens : ctx->d_rings;
+        stride = split ? 1 : R;
+        // the record lengths (a band's whole count, spilled ids included) are
+        // scanned before the spill check: one wait for both
+        TVS_CUDA(ctx, tvs::launch_ring_count(lens, stride, recs, ctx->d_rc_blocks, ctx->stream));
         TVS_CUDA(ctx, cudaMemcpyAsync(cnt, ctx->d_counters, sizeof cnt, cudaMemcpyDeviceToHost,
                                       ctx->stream));
         TVS_CUDA(ctx, cudaMemcpyAsync(&total, ctx->d_rc_blocks + nb, sizeof total,
@@ -1115,7 +1129,7 @@ int tvs_compute_sectors_rings(tvs_context *ctx, uint32_t first_angle, uint32_t n
     }
     if (recs == 0)
         TVS_CUDA(ctx, cudaMemsetAsync(ctx->d_rc_offsets, 0, sizeof(uint64_t), ctx->stream));
-    TVS_CUDA(ctx, tvs::launch_ring_gather(ctx->d_rings, recs, R, ctx->d_rc_blocks, ctx->d_spill,
+    TVS_CUDA(ctx, tvs::launch_ring_gather(lens, stride, ctx->d_rings, recs, R, ctx->d_rc_blocks, ctx->d_spill,
                                           cnt[0], ctx->d_rc_offsets, ctx->d_rc_ids, ctx->stream));
     ctx->launches += 2;
     TVS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

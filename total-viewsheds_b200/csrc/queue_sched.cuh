@@ -27,13 +27,12 @@ constexpr int kQueueTileY = TVS_QUEUE_WARPS;
 constexpr int kQueueThreads = kQueueTileX * kQueueTileY;
 
 // Warps per CTA of the split sweep and warp tiles per chunk of its queue.  A CTA
-// takes kSplitGrab chunks at a time while many are left, and one at a time towards
-// the end of a launch and in a short one: with one tile per warp in a slot, a warp
-// whose tiles are skipped for the most part waited for the slowest to leave one
-// (3601^2 exact f32 86.2 against 82.9 ms), with four to the end the CTAs finish
-// unevenly (1201^2 3.71 against 3.88 ms).
+// takes kSplitGrab chunks at a time while many are left: with one tile per warp in
+// a slot, a warp whose tiles are skipped for the most part waits for the slowest to
+// leave one (3601^2 exact f32 86.2 against 82.9 ms); with 64 tiles to the end the
+// CTAs finish unevenly (1201^2 3.71 against 3.88 ms).
 constexpr int kSplitWarps = 16;
-constexpr uint32_t kSplitChunk = kSplitWarps, kSplitGrab = 4;
+constexpr uint32_t kSplitChunk = 8, kSplitGrab = 8;
 
 // The split sweep's launches take as many sectors as have planes of surfaces (one
 // per sector and direction) of kPlaneBytes, and kPlaneSectors of a large DEM's up

@@ -47,17 +47,17 @@ __device__ uint64_t block_exclusive(uint64_t v, uint64_t *cta_total) {
     return r;
 }
 
-__device__ __forceinline__ uint32_t record_length(const uint32_t *rings, uint64_t band, uint64_t bands,
-                                                  uint32_t reserved) {
-    return band < bands ? rings[band * reserved] : 0u;
+__device__ __forceinline__ uint32_t record_length(const uint32_t *lens, uint32_t stride, uint64_t band,
+                                                  uint64_t bands) {
+    return band < bands ? lens[band * stride] : 0u;
 }
 
 __global__ void __launch_bounds__(kRingThreads)
-k_ring_block_sums(const uint32_t *rings, uint64_t bands, uint32_t reserved, uint64_t *block_sums) {
+k_ring_block_sums(const uint32_t *lens, uint32_t stride, uint64_t bands, uint64_t *block_sums) {
     const uint64_t b0 = (uint64_t)blockIdx.x * kRingChunk + (uint64_t)threadIdx.x * kRingPer;
     uint64_t s = 0;
 #pragma unroll
-    for (int j = 0; j < kRingPer; j++) s += record_length(rings, b0 + j, bands, reserved);
+    for (int j = 0; j < kRingPer; j++) s += record_length(lens, stride, b0 + j, bands);
     __shared__ uint64_t total;
     block_exclusive(s, &total);
     if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
@@ -84,14 +84,14 @@ __global__ void __launch_bounds__(kRingThreads) k_ring_scan_blocks(uint64_t *blo
 // offsets[band] for every band (and offsets[bands] = total); the in-slot ids of
 // every band copied to ids[offsets[band] ..).
 __global__ void __launch_bounds__(kRingThreads)
-k_ring_gather(const uint32_t *rings, uint64_t bands, uint32_t reserved, const uint64_t *block_base,
-              uint64_t *offsets, uint32_t *ids) {
+k_ring_gather(const uint32_t *lens, uint32_t stride, const uint32_t *rings, uint64_t bands,
+              uint32_t reserved, const uint64_t *block_base, uint64_t *offsets, uint32_t *ids) {
     const uint64_t b0 = (uint64_t)blockIdx.x * kRingChunk + (uint64_t)threadIdx.x * kRingPer;
     uint32_t len[kRingPer];
     uint64_t s = 0;
 #pragma unroll
     for (int j = 0; j < kRingPer; j++) {
-        len[j] = record_length(rings, b0 + j, bands, reserved);
+        len[j] = record_length(lens, stride, b0 + j, bands);
         s += len[j];
     }
     __shared__ uint64_t total;
@@ -103,21 +103,28 @@ k_ring_gather(const uint32_t *rings, uint64_t bands, uint32_t reserved, const ui
         if (b0 + j < bands) offsets[b0 + j] = off;
         off += len[j];
     }
-    // The warp copies its 32 x kRingPer records one at a time, in band order:
-    // lane q moves id q of the record, so each record is one coalesced read of
-    // its slots and one contiguous write.
-    const uint32_t lane = threadIdx.x & 31u;
+    // The warp copies its 32 x kRingPer records in band order, four at a time: eight
+    // lanes move a record's ids (about nine of them on rough terrain), so the writes
+    // of a step are four runs that follow each other.  A whole warp per record kept
+    // one load in flight and 23 lanes idle: 1201^2, six sectors, 0.20 ms.
+    const uint32_t lane = threadIdx.x & 31u, sub = lane >> 3, q0 = lane & 7u;
     const uint64_t warp_b0 = (uint64_t)blockIdx.x * kRingChunk + (uint64_t)(threadIdx.x & ~31u) * kRingPer;
+    static_assert(kRingPer == 4, "a thread's records are one step of its warp");
+#pragma unroll 4
     for (uint32_t src = 0; src < 32; src++) {
+        // the four records of thread src, one per eight lanes
+        uint32_t n = 0;
+        uint64_t o = 0;
 #pragma unroll
         for (int j = 0; j < kRingPer; j++) {
-            const uint64_t band = warp_b0 + (uint64_t)src * kRingPer + j;
-            const uint32_t n = __shfl_sync(0xffffffffu, min(len[j], reserved - 1), src);
-            const uint64_t o = __shfl_sync(0xffffffffu, at[j], src);
-            if (band >= bands) continue;  // uniform over the warp
-            const uint32_t *rec = rings + band * reserved + 1;
-            for (uint32_t q = lane; q < n; q += 32) ids[o + q] = rec[q];
+            const uint32_t nj = __shfl_sync(0xffffffffu, min(len[j], reserved - 1), src);
+            const uint64_t oj = __shfl_sync(0xffffffffu, at[j], src);
+            if (sub == (uint32_t)j) n = nj, o = oj;
         }
+        const uint64_t band = warp_b0 + (uint64_t)src * kRingPer + sub;
+        if (band >= bands) n = 0;
+        const uint32_t *rec = rings + band * reserved + 1;
+        for (uint32_t q = q0; q < n; q += 8) ids[o + q] = __ldcs(rec + q);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) offsets[bands] = block_base[gridDim.x];
 }
@@ -137,21 +144,22 @@ __global__ void k_ring_scatter_spill(const uint4 *spill, uint32_t n, const uint6
 
 uint64_t ring_scan_blocks(uint64_t bands) { return (bands + kRingChunk - 1) / kRingChunk; }
 
-cudaError_t launch_ring_count(const uint32_t *rings, uint64_t bands, uint32_t reserved,
+cudaError_t launch_ring_count(const uint32_t *lens, uint32_t stride, uint64_t bands,
                               uint64_t *block_sums, cudaStream_t s) {
     const uint64_t nb = ring_scan_blocks(bands);
-    if (nb) k_ring_block_sums<<<(unsigned)nb, kRingThreads, 0, s>>>(rings, bands, reserved, block_sums);
+    if (nb) k_ring_block_sums<<<(unsigned)nb, kRingThreads, 0, s>>>(lens, stride, bands, block_sums);
     k_ring_scan_blocks<<<1, kRingThreads, 0, s>>>(block_sums, nb);
     return cudaGetLastError();
 }
 
-cudaError_t launch_ring_gather(const uint32_t *rings, uint64_t bands, uint32_t reserved,
+cudaError_t launch_ring_gather(const uint32_t *lens, uint32_t stride, const uint32_t *rings,
+                               uint64_t bands, uint32_t reserved,
                                const uint64_t *block_sums, const uint4 *spill, uint32_t n_spill,
                                uint64_t *offsets, uint32_t *ids, cudaStream_t s) {
     const uint64_t nb = ring_scan_blocks(bands);
     if (nb)
-        k_ring_gather<<<(unsigned)nb, kRingThreads, 0, s>>>(rings, bands, reserved, block_sums,
-                                                          offsets, ids);
+        k_ring_gather<<<(unsigned)nb, kRingThreads, 0, s>>>(lens, stride, rings, bands, reserved,
+                                                          block_sums, offsets, ids);
     if (n_spill)
         k_ring_scatter_spill<<<(n_spill + 255) / 256, 256, 0, s>>>(spill, n_spill, offsets, ids);
     return cudaGetLastError();

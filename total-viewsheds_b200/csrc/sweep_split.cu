@@ -61,8 +61,8 @@
 // Ring records (kRings): chains keep their previous visibility and record
 // count; an event (visibility changed) stores the sample's DEM id in the
 // band's next slot, slot 1 is the point of view, slot 0 the count at the end
-// (kernel.rs:141-145,220-243).  A chain that was visible at the previous step
-// is always evaluated, so its closing event is never skipped.
+// (kernel.rs:141-145,220-243).  Where a step or a segment is skipped, the chains
+// visible before it close their rings at it.
 #include <algorithm>
 #include <climits>
 #include <map>
@@ -140,19 +140,24 @@ __device__ __forceinline__ float window_exact(float c) { return __fmaf_rn(0x1p-2
 // i + kAhead, and entry i holds where step i's samples are (next: of the step
 // kAhead steps later; the point of view itself past the last step), in floats of
 // the DEM or bytes of the quad copies.  One 16-byte read so gives a step its
-// constants and the address of the loads that run two steps ahead.
-constexpr uint32_t kAhead = 2;
+// constants and the address of the loads that run ahead: two steps for the
+// surfaces, one for ring output, whose loop then has one copy of its long body
+// (with three, half of its issue slots waited for instructions).
+constexpr uint32_t kAheadMost = 2;
 template <int kPrec> struct Step;
 template <> struct __align__(16) Step<TVS_PRECISION_EXACT32> {
     float y, z, w;  // 1/d, -d/R + G, the surface addend
     int next;
     float d, c;     // the exact angle's d and d/R
-    float2 pad;
+    int orig;       // the sample's offset in the DEM (ring ids)
+    float pad;
 };
 template <> struct __align__(16) Step<TVS_PRECISION_MIXED64> {
     float y, z, band;  // 1/d, -(d/R + o/d), W
     int next;
-    double w, pad;  // RN64(d*0.0174533)
+    double w;  // RN64(d*0.0174533)
+    int orig;  // the sample's offset in the DEM (ring ids)
+    float pad;
 };
 template <> struct __align__(16) Step<TVS_PRECISION_FP64> {
     float y, z, d;  // 1/d, -(d/R + o/d) + G, d
@@ -200,7 +205,7 @@ template <int kPrec> struct SplitSmem {
     __host__ __device__ static size_t slots() { return align16(sizeof(SplitCtl)); }
     __host__ __device__ static size_t table() { return align16(sizeof(SplitSlot)); }
     __host__ __device__ static size_t seg(uint32_t cap) {
-        return table() + (size_t)(cap + kAhead) * sizeof(Step<kPrec>);
+        return table() + (size_t)(cap + kAheadMost) * sizeof(Step<kPrec>);
     }
     __host__ __device__ static size_t slot(uint32_t cap) {
         return seg(cap) + (size_t)seg_count(cap) * sizeof(SegBound);
@@ -242,6 +247,13 @@ __device__ __forceinline__ uint32_t add_release(uint32_t *p, uint32_t v) {
 __device__ __forceinline__ void red_release(uint32_t *p, uint32_t v) {
     asm volatile("red.release.cta.shared::cta.add.u32 [%0], %1;"
                  :: "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(v) : "memory");
+}
+
+// The largest of the lanes' values (a NaN is left out), as one reduction.
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
 }
 
 // A visible sample's state change, spelled with predicates: the compiler would
@@ -327,6 +339,7 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
     constexpr bool kMix = kPrec == TVS_PRECISION_MIXED64;
     constexpr bool kF64 = kPrec == TVS_PRECISION_FP64;
     constexpr bool kWide = kMix || kF64;  // surfaces in double
+    constexpr uint32_t kAhead = kRings ? 1 : kAheadMost;
     constexpr bool kQuad = kLayout == kQuadLayout;
     using L = SplitSmem<kPrec>;
     using S = Surface<kPrec>;
@@ -355,8 +368,15 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
         uint32_t item = uni(ctl.item), upto = uni(ctl.upto);
         __syncwarp();
         if (item == upto) {
-            constexpr uint32_t kGrab = kSplitGrab * kWarps / kSplitWarps / (kF64 ? 2 : 1);
-            const uint32_t grab = item + 2 * kGrab * gridDim.x < n_items ? kGrab : 1u;
+            // many at a time while many are left, towards the end two tiles per warp
+            // of a slot, in a short launch as few as spread it over the GPU
+            constexpr uint32_t kMost = kSplitGrab * kWarps / kSplitWarps / (kF64 ? 2 : 1);
+            constexpr uint32_t kLeast = kMost / 4 ? kMost / 4 : 1;
+            static_assert(kMost >= kLeast, "every grab takes a chunk");
+            const uint32_t left = n_items - min(item, n_items);
+            const uint32_t grab = left > 2 * kMost * gridDim.x          ? kMost
+                                  : n_items >= 4 * kLeast * gridDim.x ? kLeast
+                                                                       : 1u;
             item = 0;
             if (lane == 0) item = atomicAdd(a.queue, grab);
             item = uni(item);
@@ -434,6 +454,7 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                     Step<kPrec> &e = s_t[i + kAhead];
                     e.y = t.x;
                     e.z = z;
+                    if constexpr (kRings && !kFp32 && !kF64) e.orig = dir ? -go[i].x : go[i].x;
                     if constexpr (kMix) {
                         e.band = g;
                         e.w = gd[i].z;
@@ -625,12 +646,15 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                     if constexpr (quad) return __ldg(reinterpret_cast<const float *>(quad_at(off)) + k);
                     else return __ldg(at(off, k));
                 };
-                // ring records of chain k: kernel id and the DEM id of a sample;
-                // a call over several sectors keeps each sector's records apart: its
-                // sector s owns records s * total_bands ..
-                auto orig = [&](uint32_t st) -> long long {
-                    if constexpr (quad) {
-                        const long long o =
+                // ring records: the step's offset in the DEM, chain k's kernel id, and
+                // the DEM id of its sample (ids fit an int); a call over several
+                // sectors keeps each sector's records apart: its sector s owns records
+                // s * total_bands ..
+                auto orig = [&](uint32_t st) -> int {
+                    if constexpr (kPrec == TVS_PRECISION_EXACT32 || kMix) {
+                        return s_t[st + kAhead].orig;
+                    } else if constexpr (quad) {
+                        const int o =
                             __ldg(&D.offs[(uint64_t)(a.first_sector + (group >> 1)) * D.step_cap + st].x);
                         return dir ? -o : o;
                     } else {
@@ -642,15 +666,25 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                            (dir ? a.half_bands : 0) +
                            (uint64_t)(a.first_sector - a.first_record_sector + (group >> 1)) * 2 * a.half_bands;
                 };
-                auto dem_id = [&](int k, long long o) -> uint32_t {
-                    const long long pov = (long long)(ty + RS * (k / KX) + D.los) * D.width +
-                                          tx + LX * (k % KX) + D.los;
-                    return (uint32_t)(pov + o);
+                // the lane's first record, and chain k's from it (one 32-bit add and a
+                // wide multiply-add per id in place of two 64-bit products)
+                uint32_t *ring0 = nullptr;
+                uint32_t pov0 = 0, row_ids = 0, row_slots = 0, col_slots = 0;
+                if constexpr (kRings) {
+                    ring0 = a.rings + kid(0) * a.ring_reserved;
+                    pov0 = (ty + D.los) * D.width + tx + D.los;
+                    row_ids = RS * D.width;
+                    row_slots = RS * D.tvs_width * a.ring_reserved;
+                    col_slots = LX * a.ring_reserved;
+                }
+                auto dem_id = [&](int k, int o) -> uint32_t {
+                    return pov0 + (uint32_t)(k / KX) * row_ids + LX * (k % KX) + (uint32_t)o;
                 };
-                auto ring_put = [&](uint64_t band, uint32_t slot, uint32_t value) {
+                auto ring_put = [&](int k, uint32_t slot, uint32_t value) {
                     if (slot < a.ring_reserved) {
-                        a.rings[band * a.ring_reserved + slot] = value;
+                        ring0[(k / KX) * row_slots + (k % KX) * col_slots + slot] = value;
                     } else {
+                        const uint64_t band = kid(k);
                         const uint32_t at_ = atomicAdd(&a.ring_counters[0], 1u);
                         if (at_ < a.spill_cap)
                             a.spill[at_] = make_uint4((uint32_t)band, (uint32_t)(band >> 32), slot, value);
@@ -662,7 +696,7 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
 #pragma unroll
                     for (int k = 0; k < K; k++) {
                         nr[k] = 1;
-                        if (active >> k & 1u) ring_put(kid(k), 1, dem_id(k, 0));  // kernel.rs:145
+                        if (active >> k & 1u) ring_put(k, 1, dem_id(k, 0));  // kernel.rs:145
                     }
                 } else {
                     prev = 0;
@@ -670,12 +704,17 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                 auto events = [&](uint32_t vis, uint32_t st) {
                     const uint32_t ev = (vis ^ prev) & active;
                     if (__any_sync(0xffffffffu, ev != 0)) {
-                        const long long o = orig(st);
+                        const int o = orig(st);
 #pragma unroll
                         for (int k = 0; k < K; k++)
-                            if (ev >> k & 1u) ring_put(kid(k), ++nr[k], dem_id(k, o));
+                            if (ev >> k & 1u) ring_put(k, ++nr[k], dem_id(k, o));
+                        __syncwarp();
                     }
                     prev = vis;
+                };
+                // no chain is visible at step st
+                auto close = [&](uint32_t st) {
+                    if constexpr (kRings) events(0, st);
                 };
                 // The largest elevation any lane of this warp samples in a
                 // segment: the block maxima over the warp's patch of points of
@@ -695,20 +734,18 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                             if (y <= by1 && x <= bx1)
                                 m = fmaxf(m, __ldg(D.bmax + (uint32_t)y * D.bmax_w + x));
                         }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-                    return m;
+                    return warp_max(m);
                 };
                 // A segment can be skipped when no chain can change state at
                 // any of its steps: every sample h <= B, so e <= RN(B - h_pov)
                 // and the first test's value fma(e, y, z) is at most
                 // fma(RN(B - h_pov), y_max or y_min, z_max) (RN and fma are
-                // monotone).  A chain visible at the previous step must close
-                // its ring at the next one, so it is never skipped.
+                // monotone).  A chain visible at the previous step closes its ring
+                // at the segment's first one.
                 auto skippable = [&](uint32_t seg, auto &&below) -> bool {
                     const SegBound b = s_seg[seg];
                     const float B = segment_max(b);
-                    bool skip = prev == 0;
+                    bool skip = true;
 #pragma unroll
                     for (int k = 0; k < K; k++) {
                         const float E = __fsub_rn(B, hp[k]);
@@ -735,15 +772,24 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                     for (uint32_t seg = 0; i < n_fast; seg++) {
                         const uint32_t i1 = min(i + kSegSteps, n_fast);
                         if (skippable(seg, below)) {
+                            close(i);
                             i = i1;
                             continue;
                         }
                         n_swept += i1 - i;
-                        float h0[K], h1[K];
-                        load(s_t[i].next, h0);
-                        load(s_t[i + 1].next, h1);
                         const Step<kPrec> *p = s_t + i + kAhead;
-                        if constexpr (kFp32) {  // its short steps gain from four an iteration
+                        float h0[K];
+                        load(s_t[i].next, h0);
+                        if constexpr (kRings) {
+#pragma unroll 1
+                            for (; i < i1; i++, p++) step(i, p, h0);
+                            continue;
+                        }
+                        float h1[K];
+                        load(s_t[i + 1].next, h1);
+                        // four an iteration where the registers allow it (1201^2 exact f32
+                        // 3.66 -> 3.56 ms, 3601^2 FP32 64.1 -> 61.8; MIXED64 spills)
+                        if constexpr (!kWide) {
                             for (; i + 4 <= i1; i += 4, p += 4) {
                                 step(i, p, h0);
                                 step(i + 1, p + 1, h1);
@@ -872,7 +918,7 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                         bool hit = false;
 #pragma unroll
                         for (int k = 0; k < K; k++) hit |= f[k] >= lo[k];
-                        if (__any_sync(0xffffffffu, hit || prev != 0)) {
+                        if (__any_sync(0xffffffffu, hit)) {
                             n_passed++;
                             const float d = p->d, c = p->c;
                             [[maybe_unused]] uint32_t vis = 0;
@@ -883,6 +929,8 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                                 raise_exact(ang, m[k], sf[k], lo[k], w);
                             }
                             if constexpr (kRings) events(vis, st);
+                        } else {
+                            close(st);
                         }
                     };
                     sweep_fast([&](int k, float bound) { return bound < lo[k]; }, step);
@@ -943,7 +991,7 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                         bool hit = false;
 #pragma unroll
                         for (int k = 0; k < K; k++) hit |= x[k] >= -hw[k];
-                        if (__any_sync(0xffffffffu, hit || prev != 0)) {
+                        if (__any_sync(0xffffffffu, hit)) {
                             n_passed++;
                             const double w = p->w;
                             bool amb = false;  // inside the band
@@ -984,6 +1032,8 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                                 for (int k = 0; k < K; k++) nmid[k] = fminf(nmid[k], -f[k]);  // a NaN leaves it
                             }
                             if constexpr (kRings) events(vis, st);
+                        } else {
+                            close(st);
                         }
                     };
                     sweep_fast([&](int k, float bound) { return __fadd_rn(bound, nmid[k]) < -hw[k]; }, step);
@@ -1024,13 +1074,14 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                 if constexpr (kRings) {
                     // kernel.rs:237-243: close a ring cut off by the line of
                     // sight, then the count in slot 0
-                    const long long o_last = n ? orig(n - 1) : 0;
+                    const int o_last = n ? orig(n - 1) : 0;
                     uint32_t most = 0, over = 0;
 #pragma unroll
                     for (int k = 0; k < K; k++) {
                         if (!(active >> k & 1u)) continue;
-                        if (prev >> k & 1u) ring_put(kid(k), ++nr[k], dem_id(k, o_last));
-                        ring_put(kid(k), 0, nr[k]);
+                        if (prev >> k & 1u) ring_put(k, ++nr[k], dem_id(k, o_last));
+                        if (a.ring_lens) a.ring_lens[kid(k)] = nr[k];
+                        else ring_put(k, 0, nr[k]);
                         most = max(most, nr[k]);
                         over += nr[k] >= a.ref_reserved;
                     }

@@ -73,6 +73,7 @@ struct tvs_context {
     // compact ring records of the last tvs_compute_sector_rings (allocated on first use)
     uint64_t *d_rc_blocks = nullptr;   // scanned record-length block sums
     uint64_t *d_rc_offsets = nullptr;  // [total_bands + 1]
+    uint32_t *d_rc_lens = nullptr;     // record lengths (the split sweep's)
     uint32_t *d_rc_ids = nullptr;
     uint64_t rc_ids_cap = 0, rc_total = 0;
     uint64_t rc_records = 0;      // records of the last call (sectors x total_bands)

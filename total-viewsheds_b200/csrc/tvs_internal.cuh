@@ -223,6 +223,7 @@ struct QueueArgs {
     uint32_t *rings;
     uint32_t first_record_sector;      // the sector whose records are the first in `rings`
     uint32_t ring_reserved;            // slots per band in `rings`
+    uint32_t *ring_lens;               // nullable: the bands' counts, in place of slot 0
     uint32_t ref_reserved;             // the reference's slots per band (statistics)
     uint64_t half_bands;               // computable points of the whole grid
     uint4 *spill;
@@ -279,9 +280,11 @@ __host__ __device__ inline uint32_t f32_radix_key(float f) {
 // (ring_scan_blocks(bands) + 1 entries, exclusive-scanned, total last), then
 // the offsets and ids.
 uint64_t ring_scan_blocks(uint64_t bands);
-cudaError_t launch_ring_count(const uint32_t *rings, uint64_t bands, uint32_t reserved,
+// (lens[k * stride] is band k's count: a dense array, or slot 0 of the records)
+cudaError_t launch_ring_count(const uint32_t *lens, uint32_t stride, uint64_t bands,
                               uint64_t *block_sums, cudaStream_t s);
-cudaError_t launch_ring_gather(const uint32_t *rings, uint64_t bands, uint32_t reserved,
+cudaError_t launch_ring_gather(const uint32_t *lens, uint32_t stride, const uint32_t *rings,
+                               uint64_t bands, uint32_t reserved,
                                const uint64_t *block_sums, const uint4 *spill, uint32_t n_spill,
                                uint64_t *offsets, uint32_t *ids, cudaStream_t s);
 // bmax[(y / kBlockMax) * bmax_w + x / kBlockMax] = max elevation of the block
