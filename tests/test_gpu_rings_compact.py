@@ -190,3 +190,68 @@ def test_several_sectors_argument_errors(tvs, dem):
         assert L.tvs_compute_sectors_rings(eng.ctx, 0, 2, tvs._ptr(cum), ctypes.byref(total),
                                            None) == tvs.ERR_INVALID_ARGUMENT
         assert b"split sweep" in L.tvs_last_error(eng.ctx)
+
+
+@pytest.mark.parametrize("rpk", [5.0, 20.0, 200.0])
+@pytest.mark.parametrize("precision,rows", [("exact32", None), ("exact32", (20, 61)), ("mixed64", None)])
+def test_reserved_layout_laid_out_on_the_host(tvs, oracle, dem, rpk, precision, rows):
+    """The reference's slots from the compact records: with spilled ids (5/km), with
+    one thread's worth of slots, with several threads' (49 MB); dirty caller memory."""
+    g = oracle.geometry(W, SCALE, LOS, rpk)
+    f64 = precision == "mixed64"
+    with tvs.Engine(dem, W, SCALE, LOS, rings_per_km=rpk, observer_height=OBS, precision=precision,
+                    rows=rows) as eng:
+        R, bands = eng.geometry.reserved_rings_per_band, eng.geometry.total_bands
+        got = np.full(bands * R, 0xABCDABCD, np.uint32)
+        for angle in (0, 46):
+            d, x, _ = oracle.compile_band_data(g, float(angle))
+            want = np.zeros(oracle.ring_len(g), np.uint32)
+            surface = np.zeros(eng.count, np.float64 if f64 else np.float32)
+            oracle.compute_sector(g, dem, OBS, d, x, surface, want, f64=f64)
+            cum = np.zeros(eng.count, np.float32)
+            eng.compute_sector(angle, cum, got)
+            assert rpk > 5.0 or (want.reshape(-1, R)[:, 0] >= R).any()
+            if rows is None:
+                assert np.array_equal(got, want)
+                assert np.array_equal(bits(cum), bits(surface.astype(np.float32)))
+            else:
+                # an unspilled record of the shard is the oracle's, the others are empty
+                row = np.arange(bands) % (bands // 2) // eng.geometry.tvs_width
+                mine = (row >= rows[0]) & (row < rows[1])
+                a, b = got.reshape(-1, R), want.reshape(-1, R)
+                spilled = np.zeros(bands, bool)  # other bands' ids may be in it
+                for k in np.flatnonzero(b[:, 0] >= R):
+                    spilled[k + 1:k + 1 + b[k, 0] // R] = True
+                assert np.array_equal(a[mine & ~spilled], b[mine & ~spilled])
+                assert not a[~mine & ~spilled].any()
+
+
+def test_contexts_of_several_threads_share_the_host_buffers(tvs, dem):
+    """Calls that find the process's pinned buffers lent take their own way."""
+    import threading
+
+    def work(angle):
+        with tvs.Engine(dem, W, SCALE, LOS, rings_per_km=60.0, observer_height=OBS) as eng:
+            rings = np.zeros(eng.geometry.ring_slots_per_sector, np.uint32)
+            cum = np.zeros(eng.count, np.float32)
+            for _ in range(4):
+                cum[:] = 0
+                eng.compute_sector(angle, cum, rings)
+            run_cum, run_total, _ = eng.run()
+            return rings, cum, run_cum, run_total
+
+    angles = [3, 46, 91, 137]
+    want = [work(a) for a in angles]
+    got = [None] * len(angles)
+
+    def put(i):
+        got[i] = work(angles[i])
+
+    threads = [threading.Thread(target=put, args=(i,)) for i in range(len(angles))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for g, w in zip(got, want):
+        for x, y in zip(g, w):
+            assert np.array_equal(bits(x), bits(y))

@@ -12,6 +12,7 @@
 #include "tvs.h"
 #include "tvs_internal.cuh"
 
+#include "host_stage.hpp"
 #include "tvs_context.hpp"
 
 namespace {
@@ -147,7 +148,7 @@ void free_all(tvs_context *c) {
                     c->d_rechecks, c->d_qdem,
                     c->d_deltas, c->d_dists, c->d_rings, c->d_spill, c->d_counters, c->d_sf,
                     c->d_sb, c->d_tab_deltas, c->d_tab_dists, c->d_installed,
-                    c->d_rc_blocks, c->d_rc_offsets, c->d_rc_lens, c->d_rc_ids, c->d_bmax, c->d_qdem_rings,
+                    c->d_rc_blocks, c->d_rc_offsets, c->d_rc_lens, c->d_rc_ids, c->d_ref_scan, c->d_ref_ids, c->d_bmax, c->d_qdem_rings,
                     c->d_diag, c->d_quad};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -573,11 +574,8 @@ int enqueue_sweep(tvs_context *c, uint32_t first, uint32_t count, uint32_t ring_
     return TVS_OK;
 }
 
-int header_status(tvs_context *c, uint32_t first, uint32_t count) {
-    std::vector<tvs::ShapeHeader> h(count);
-    TVS_CUDA(c, cudaMemcpyAsync(h.data(), c->d_hdr + first, count * sizeof(tvs::ShapeHeader),
-                                cudaMemcpyDeviceToHost, c->stream));
-    TVS_CUDA(c, cudaStreamSynchronize(c->stream));
+// The first failure among the headers h of sectors first ..
+int check_headers(tvs_context *c, const tvs::ShapeHeader *h, uint32_t first, uint32_t count) {
     for (uint32_t i = 0; i < count; i++) {
         if (h[i].status == TVS_OK) continue;
         char b[256];
@@ -591,6 +589,44 @@ int header_status(tvs_context *c, uint32_t first, uint32_t count) {
         return fail(c, h[i].status, b);
     }
     return TVS_OK;
+}
+
+int header_status(tvs_context *c, uint32_t first, uint32_t count) {
+    std::vector<tvs::ShapeHeader> h(count);
+    TVS_CUDA(c, cudaMemcpyAsync(h.data(), c->d_hdr + first, count * sizeof(tvs::ShapeHeader),
+                                cudaMemcpyDeviceToHost, c->stream));
+    TVS_CUDA(c, cudaStreamSynchronize(c->stream));
+    return check_headers(c, h.data(), first, count);
+}
+
+// What tvs_device_finish reads back, and with it (small results) the surfaces.
+struct FinishBlock {
+    tvs::ShapeHeader hdr[tvs::kSectorSteps];
+    int32_t error;
+};
+
+// Enqueues the read-back of the headers and the error word.
+cudaError_t read_finish(tvs_context *c, FinishBlock *b) {
+    cudaError_t e = cudaMemcpyAsync(b->hdr, c->d_hdr, sizeof b->hdr, cudaMemcpyDeviceToHost, c->stream);
+    return e == cudaSuccess ? cudaMemcpyAsync(&b->error, c->d_error, sizeof b->error, cudaMemcpyDeviceToHost,
+                                              c->stream)
+                            : e;
+}
+
+// The first error of the sectors enqueued since the last call, from a block whose
+// read-back has been waited for.
+int judge_finish(tvs_context *c, const FinishBlock &b) {
+    int rc = TVS_OK;
+    for (uint32_t s = 0; s < tvs::kSectorSteps && rc == TVS_OK; s++)
+        if (c->pending[s]) rc = check_headers(c, b.hdr + s, s, 1);
+    for (bool &p : c->pending) p = false;
+    if (b.error != 0) {
+        TVS_CUDA(c, cudaMemset(c->d_error, 0, sizeof b.error));
+        if (rc == TVS_OK)
+            rc = fail(c, b.error, "sweep work queue: a tile's dependency wait gave up "
+                                  "(iteration limit); results of this run are incomplete");
+    }
+    return rc;
 }
 
 // The shape slots of sectors [first, first+count) for the per-sector calls:
@@ -618,16 +654,111 @@ int ensure_shapes(tvs_context *c, uint32_t first, uint32_t count) {
 }
 int ensure_shape(tvs_context *c, uint32_t angle) { return ensure_shapes(c, angle, 1); }
 
+// Ring records come from the split sweep, with their counts apart from the slots.
+bool split_rings(const tvs_context *c) {
+    return c->p.sweep_kernel != TVS_SWEEP_PLAIN && c->p.precision != TVS_PRECISION_FP64 &&
+           sweep_impl() == SweepImpl::Queue;
+}
+
+// One sector's sweep with ring records of the reference's reservation on the device
+// (ensure_rings has run).
+int sweep_reference_rings(tvs_context *c, uint32_t angle) {
+    const uint64_t bands = c->g.total_bands;
+    const uint32_t R = c->g.reserved_rings_per_band;
+    uint32_t *lens = nullptr;
+    if (split_rings(c)) {
+        if (!c->d_ref_lens) {  // without memory for it: counts in the slots, all of which cross
+            const uint64_t words = tvs::ring_scan_blocks(bands) + 1 + bands + 1;
+            const size_t bytes = words * sizeof(uint64_t) + std::max<uint64_t>(bands, 1) * sizeof(uint32_t);
+            if (cudaMalloc(&c->d_ref_scan, bytes) == cudaSuccess) {
+                c->d_ref_lens = reinterpret_cast<uint32_t *>(c->d_ref_scan + words);
+                c->device_bytes += bytes;
+            } else {
+                cudaGetLastError();
+                c->d_ref_scan = nullptr;
+            }
+        }
+        lens = c->d_ref_lens;
+    }
+    // (a row shard leaves the other bands' counts unwritten)
+    if (lens)
+        TVS_CUDA(c, cudaMemsetAsync(lens, 0, bands * sizeof(uint32_t), c->stream));
+    else
+        TVS_CUDA(c, cudaMemsetAsync(c->d_rings, 0, c->g.ring_slots_per_sector * sizeof(uint32_t), c->stream));
+    TVS_CUDA(c, cudaMemsetAsync(c->d_counters, 0, 4 * sizeof(uint32_t), c->stream));
+    return enqueue_sweep(c, angle, 1, R, lens);
+}
+
+// The sector's records to the reference's layout on the host.  Its slots are mostly
+// empty (39 MB for 2.4 MB of ids at 601^2, 2.0 ms through the driver's pageable
+// copy), so the records cross the bus compact and are laid out here.  The buffers
+// are apart from those that tvs_read_ring_records reads.
+int read_reference_rings(tvs_context *c, uint32_t *rings) {
+    const uint64_t bands = c->g.total_bands, nb = tvs::ring_scan_blocks(bands);
+    const uint32_t R = c->g.reserved_rings_per_band;
+    if (bands == 0) return TVS_OK;
+    uint64_t *blocks = c->d_ref_scan, *offsets = c->d_ref_scan + nb + 1;
+    TVS_CUDA(c, tvs::launch_ring_count(c->d_ref_lens, 1, bands, blocks, c->stream));
+    uint64_t total = 0;
+    TVS_CUDA(c, cudaMemcpyAsync(&total, blocks + nb, sizeof total, cudaMemcpyDeviceToHost, c->stream));
+    TVS_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (total > c->ref_ids_cap || !c->d_ref_ids) {
+        if (c->d_ref_ids) cudaFree(c->d_ref_ids);
+        c->device_bytes -= c->ref_ids_cap * sizeof(uint32_t);
+        c->d_ref_ids = nullptr;
+        c->ref_ids_cap = 0;
+        const uint64_t cap = std::max<uint64_t>(total + total / 2, 1);
+        if (cudaMalloc(&c->d_ref_ids, cap * sizeof(uint32_t)) == cudaSuccess) {
+            c->ref_ids_cap = cap;
+            c->device_bytes += cap * sizeof(uint32_t);
+        } else {  // no room to gather them: every slot crosses
+            cudaGetLastError();
+            c->d_ref_ids = nullptr;
+            std::vector<uint32_t> counts(bands);
+            TVS_CUDA(c, cudaMemcpyAsync(counts.data(), c->d_ref_lens, bands * sizeof(uint32_t),
+                                        cudaMemcpyDeviceToHost, c->stream));
+            TVS_CUDA(c, cudaMemcpyAsync(rings, c->d_rings, bands * R * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                                        c->stream));
+            TVS_CUDA(c, cudaStreamSynchronize(c->stream));
+            tvs_host::complete_records(rings, bands, R, counts.data());
+            return TVS_OK;
+        }
+    }
+    // (spilled ids have their places in the stream, which nothing reads here)
+    TVS_CUDA(c, tvs::launch_ring_gather(c->d_ref_lens, 1, c->d_rings, bands, R, blocks, nullptr, 0, offsets,
+                                        c->d_ref_ids, c->stream));
+    tvs_host::RecordBuffer buffer(c->stream);
+    unsigned char *host = buffer.get((bands + 1) * sizeof(uint64_t) + total * sizeof(uint32_t));
+    if (!host) return fail(c, TVS_ERR_OUT_OF_MEMORY, "ring records on the host");
+    uint64_t *h_offsets = reinterpret_cast<uint64_t *>(host);
+    uint32_t *h_ids = reinterpret_cast<uint32_t *>(h_offsets + bands + 1);
+    TVS_CUDA(c, cudaMemcpyAsync(h_offsets, offsets, (bands + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost,
+                                c->stream));
+    if (total)
+        TVS_CUDA(c, cudaMemcpyAsync(h_ids, c->d_ref_ids, total * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                                    c->stream));
+    TVS_CUDA(c, cudaStreamSynchronize(c->stream));
+    buffer.done();
+    tvs_host::expand_records(rings, bands, R, h_offsets, h_ids);
+    return TVS_OK;
+}
+
 // Copy one sector's ring records to the host and apply the spilled ids with
 // the reference's sequential semantics: band k writes slots k*R .. k*R+n_k
 // (kernel.rs:141-243), so an id past its own record lands in a later band's
 // record unless that band's own (later) writes cover the slot.
 int collect_rings(tvs_context *c, uint32_t *rings, uint64_t rings_len, tvs_sector_stats *st) {
+    const bool compact = split_rings(c) && c->d_ref_lens;
     uint32_t cnt[4];
     TVS_CUDA(c, cudaMemcpyAsync(cnt, c->d_counters, sizeof cnt, cudaMemcpyDeviceToHost,
                                 c->stream));
-    TVS_CUDA(c, cudaMemcpyAsync(rings, c->d_rings, c->g.ring_slots_per_sector * sizeof(uint32_t),
-                                cudaMemcpyDeviceToHost, c->stream));
+    if (compact) {
+        int rc = read_reference_rings(c, rings);
+        if (rc) return rc;
+    } else {
+        TVS_CUDA(c, cudaMemcpyAsync(rings, c->d_rings, c->g.ring_slots_per_sector * sizeof(uint32_t),
+                                    cudaMemcpyDeviceToHost, c->stream));
+    }
     TVS_CUDA(c, cudaStreamSynchronize(c->stream));
     if (st) {
         st->overflow_bands = cnt[1];
@@ -753,9 +884,11 @@ int tvs_create(const tvs_params *params, const float *elevations, uint64_t n_ele
         cudaGetLastError();
         free_all(c);
         delete c;
+        tvs_host::stage_unref();
         return fail(nullptr, code, m);
     };
     cudaError_t e = cudaSetDevice(params->device);
+    tvs_host::stage_ref(e == cudaSuccess);
     if (e != cudaSuccess) return bail(e, "cudaSetDevice");
     if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess)
         return bail(e, "cudaStreamCreate");
@@ -870,6 +1003,7 @@ void tvs_destroy(tvs_context *ctx) {
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     free_all(ctx);
     delete ctx;
+    tvs_host::stage_unref();
 }
 
 int tvs_get_geometry(const tvs_context *ctx, tvs_geometry *out) {
@@ -979,9 +1113,16 @@ int tvs_compute_sector(tvs_context *ctx, uint32_t angle, float *cumulative_surfa
         return fail(ctx, TVS_ERR_INVALID_ARGUMENT, "rings_len is smaller than one sector's slots");
     TVS_CUDA(ctx, cudaSetDevice(ctx->p.device));
     const uint64_t count = ctx->g.computable_points_count;
+    // small surfaces pass through pinned memory both ways
+    tvs_host::SmallStage stage(ctx->stream);
+    float *host = cumulative_surfaces;
+    if (stage.p && count * sizeof(float) <= tvs_host::kSmall) {
+        host = reinterpret_cast<float *>(stage.p);
+        std::memcpy(host, cumulative_surfaces, count * sizeof(float));
+    }
     if (count)
-        TVS_CUDA(ctx, cudaMemcpyAsync(ctx->d_cum, cumulative_surfaces, count * sizeof(float),
-                                      cudaMemcpyHostToDevice, ctx->stream));
+        TVS_CUDA(ctx, cudaMemcpyAsync(ctx->d_cum, host, count * sizeof(float), cudaMemcpyHostToDevice,
+                                      ctx->stream));
     // FP64/MIXED64 accumulate in double within the sector, from the caller's f32
     if (ctx->d_cum64 && count)
         TVS_CUDA(ctx, tvs::launch_widen(ctx->d_cum, ctx->d_cum64, count, ctx->stream));
@@ -989,27 +1130,26 @@ int tvs_compute_sector(tvs_context *ctx, uint32_t angle, float *cumulative_surfa
     if (rings) {
         int rc = ensure_rings(ctx, R);
         if (rc) return rc;
-        TVS_CUDA(ctx, cudaMemsetAsync(ctx->d_rings, 0,
-                                      ctx->g.ring_slots_per_sector * sizeof(uint32_t), ctx->stream));
-        TVS_CUDA(ctx, cudaMemsetAsync(ctx->d_counters, 0, 4 * sizeof(uint32_t), ctx->stream));
     }
     int rc = ensure_shape(ctx, angle);
     if (rc) return rc;
-    rc = enqueue_sweep(ctx, angle, 1, rings ? R : 0);
+    rc = rings ? sweep_reference_rings(ctx, angle) : enqueue_sweep(ctx, angle, 1, 0);
     if (rc) return rc;
     if (count)
-        TVS_CUDA(ctx, cudaMemcpyAsync(cumulative_surfaces, ctx->d_cum, count * sizeof(float),
-                                      cudaMemcpyDeviceToHost, ctx->stream));
+        TVS_CUDA(ctx, cudaMemcpyAsync(host, ctx->d_cum, count * sizeof(float), cudaMemcpyDeviceToHost,
+                                      ctx->stream));
     if (stats) {
         std::memset(stats, 0, sizeof *stats);
         stats->angle = angle;
         stats->band_steps_filled = ctx->g.band_steps_filled;
     }
-    if (rings) {
-        rc = collect_rings(ctx, rings, rings_len, stats);
-        if (rc) return rc;
-    }
-    TVS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (rings) rc = collect_rings(ctx, rings, rings_len, stats);
+    const cudaError_t waited = cudaStreamSynchronize(ctx->stream);
+    stage.done();
+    if (waited == cudaSuccess && host != cumulative_surfaces)
+        std::memcpy(cumulative_surfaces, host, count * sizeof(float));
+    if (rc) return rc;
+    TVS_CUDA(ctx, waited);
     return TVS_OK;
 }
 
@@ -1059,8 +1199,7 @@ int tvs_compute_sectors_rings(tvs_context *ctx, uint32_t first_angle, uint32_t n
     // per band double and the call runs again from the caller's surfaces (a
     // band has at most n_steps + 2 ids, so this ends).
     const uint32_t most = ctx->g.band_steps_filled + 4;
-    const bool split = ctx->p.sweep_kernel != TVS_SWEEP_PLAIN && ctx->p.precision != TVS_PRECISION_FP64 &&
-                       sweep_impl() == SweepImpl::Queue;
+    const bool split = split_rings(ctx);
     const uint32_t *lens = nullptr;
     uint32_t stride = 0;
     uint32_t R = 0, cnt[4];
@@ -1206,25 +1345,13 @@ int tvs_device_run_sectors(tvs_context *ctx, uint32_t first_angle, uint32_t coun
 int tvs_device_finish(tvs_context *ctx) {
     if (!ctx) return TVS_ERR_INVALID_ARGUMENT;
     TVS_CUDA(ctx, cudaSetDevice(ctx->p.device));
+    tvs_host::SmallStage stage(ctx->stream);
+    FinishBlock own;
+    FinishBlock *b = stage.p ? reinterpret_cast<FinishBlock *>(stage.p) : &own;
+    TVS_CUDA(ctx, read_finish(ctx, b));
     TVS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    int rc = TVS_OK;
-    for (uint32_t s = 0; s < tvs::kSectorSteps && rc == TVS_OK; s++) {
-        if (!ctx->pending[s]) continue;
-        uint32_t e = s;
-        while (e < tvs::kSectorSteps && ctx->pending[e]) e++;
-        rc = header_status(ctx, s, e - s);
-        s = e - 1;
-    }
-    for (bool &p : ctx->pending) p = false;
-    int32_t err = 0;
-    TVS_CUDA(ctx, cudaMemcpy(&err, ctx->d_error, sizeof err, cudaMemcpyDeviceToHost));
-    if (err != 0) {
-        TVS_CUDA(ctx, cudaMemset(ctx->d_error, 0, sizeof err));
-        if (rc == TVS_OK)
-            rc = fail(ctx, err, "sweep work queue: a tile's dependency wait gave up "
-                                "(iteration limit); results of this run are incomplete");
-    }
-    return rc;
+    stage.done();
+    return judge_finish(ctx, *b);
 }
 
 int tvs_read_surfaces(tvs_context *ctx, float *cumulative_out, float *total_out) {
@@ -1452,13 +1579,37 @@ uint64_t tvs_device_bytes(const tvs_context *ctx) { return ctx ? ctx->device_byt
 int tvs_run(tvs_context *ctx, float *cumulative_out, float *total_out, int want_rings,
             tvs_sector_callback callback, void *user) {
     if (!ctx) return TVS_ERR_INVALID_ARGUMENT;
-    int rc = tvs_device_reset(ctx);
-    if (rc) return rc;
+    int rc = TVS_OK;
     if (!want_rings) {
-        rc = tvs_device_run_tvs(ctx);
+        rc = tvs_device_run_tvs(ctx);  // (zeroes the surfaces)
         if (rc) return rc;
-        rc = tvs_device_finish(ctx);
-        if (rc) return rc;
+        // small surfaces come back with the statuses, in one wait
+        const size_t bytes = ctx->g.computable_points_count * sizeof(float);
+        const size_t head = (sizeof(FinishBlock) + 255) & ~(size_t)255;
+        bool there = false;
+        if (head + 2 * bytes <= tvs_host::kSmall) {
+            tvs_host::SmallStage stage(ctx->stream);
+            if (stage.p) {
+                FinishBlock *b = reinterpret_cast<FinishBlock *>(stage.p);
+                unsigned char *cum = stage.p + head, *tot = cum + bytes;
+                TVS_CUDA(ctx, read_finish(ctx, b));
+                if (cumulative_out && bytes)
+                    TVS_CUDA(ctx, cudaMemcpyAsync(cum, ctx->d_cum, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+                if (total_out && bytes)
+                    TVS_CUDA(ctx, cudaMemcpyAsync(tot, ctx->d_total, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+                TVS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+                stage.done();
+                rc = judge_finish(ctx, *b);
+                if (rc) return rc;
+                if (cumulative_out && bytes) std::memcpy(cumulative_out, cum, bytes);
+                if (total_out && bytes) std::memcpy(total_out, tot, bytes);
+                there = true;
+            }
+        }
+        if (!there) {
+            rc = tvs_device_finish(ctx);
+            if (rc) return rc;
+        }
         if (callback)
             for (uint32_t s = 0; s < tvs::kSectorSteps; s++) {
                 tvs_sector_stats st{};
@@ -1466,8 +1617,10 @@ int tvs_run(tvs_context *ctx, float *cumulative_out, float *total_out, int want_
                 st.band_steps_filled = ctx->g.band_steps_filled;
                 if (callback(user, s, nullptr, 0, &st)) break;
             }
-        return tvs_read_surfaces(ctx, cumulative_out, total_out);
+        return there ? TVS_OK : tvs_read_surfaces(ctx, cumulative_out, total_out);
     }
+    rc = tvs_device_reset(ctx);
+    if (rc) return rc;
     if ((ctx->p.precision == TVS_PRECISION_MIXED64 || ctx->p.precision == TVS_PRECISION_FP64) &&
         !ctx->d_cum64)
         return fail(ctx, TVS_ERR_INVALID_ARGUMENT, "FP64 context without FP64 accumulator");
@@ -1475,14 +1628,11 @@ int tvs_run(tvs_context *ctx, float *cumulative_out, float *total_out, int want_
     if (rc) return rc;
     std::vector<uint32_t> host_rings(ctx->g.ring_slots_per_sector);
     for (uint32_t s = 0; s < tvs::kSectorSteps; s++) {
-        TVS_CUDA(ctx, cudaMemsetAsync(ctx->d_rings, 0,
-                                      ctx->g.ring_slots_per_sector * sizeof(uint32_t), ctx->stream));
-        TVS_CUDA(ctx, cudaMemsetAsync(ctx->d_counters, 0, 4 * sizeof(uint32_t), ctx->stream));
         rc = enqueue_shape(ctx, s, 1);
         if (rc) return rc;
         rc = header_status(ctx, s, 1);
         if (rc) return rc;
-        rc = enqueue_sweep(ctx, s, 1, ctx->g.reserved_rings_per_band);
+        rc = sweep_reference_rings(ctx, s);
         if (rc) return rc;
         tvs_sector_stats st{};
         st.angle = s;

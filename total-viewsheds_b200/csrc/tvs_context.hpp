@@ -58,6 +58,13 @@ struct tvs_context {
     tvs::QueueDem *d_qdem_rings = nullptr;     // this context tiled for the ring sweep
     uint32_t ring_layout = 0;                  // the ring sweep's split layout
     uint32_t q_ring_tiles = 0, q_ring_chunks = 0;
+    // the reference's ring layout on its way to the host: record lengths, scanned
+    // block sums and offsets, ids (allocated on first use; apart from the compact
+    // stream's, which tvs_read_ring_records reads)
+    uint32_t *d_ref_lens = nullptr;    // (the scan's allocation)
+    uint64_t *d_ref_scan = nullptr;
+    uint32_t *d_ref_ids = nullptr;
+    uint64_t ref_ids_cap = 0;
     // plain-kernel scratch (allocated on first use)
     float *d_sf = nullptr, *d_sb = nullptr;
     // band shapes installed as tables (the reference's shape cache), in place of
