@@ -264,13 +264,16 @@ const float *tvs_device_cumulative(const tvs_context *ctx);
 void *tvs_stream(const tvs_context *ctx);
 /* Number of kernels the last tvs_device_run_sectors call enqueued. */
 uint64_t tvs_last_launch_count(const tvs_context *ctx);
-/* Bytes of device memory the context holds (its peak: buffers are only ever
- * added, the ring buffers on the first run that asks for ring records). */
+/* Bytes of device memory the context holds: the buffers of tvs_create, the
+ * surface planes from the first sweep on, the ring buffers from the first run
+ * that asks for ring records.  (The planes come from a pool per device that may
+ * keep up to 512 MB of freed ones until the process's last context there ends.) */
 uint64_t tvs_device_bytes(const tvs_context *ctx);
 
 /* Failure detection of the persistent sweep (no counterpart in the reference,
- * which has no device waits).  A work item waits for its tile's previous
- * sector before adding its surfaces; the wait sleeps in steps of ~256 ns and
+ * which has no device waits).  Where surfaces are added in turn (the row layouts;
+ * the split layouts without memory for surface planes, or with a held tile) a work
+ * item waits for its tile's previous one before adding its own; the wait sleeps in steps of ~256 ns and
  * gives up after spin_limit steps (0 = the default, about 2 s): the item's
  * writes are skipped, later waits give up at once, and tvs_device_finish
  * returns TVS_ERR_TIMEOUT.  held_tile (0xFFFFFFFF = none) is a test hook:
@@ -303,8 +306,9 @@ int tvs_read_sweep_counters(tvs_context *ctx, uint64_t *counters);
  * L = 9 is L = 8's tiling read from four row-interleaved copies of the DEM
  * (one 16-byte load per lane and step; the context holds the copies, 4x the
  * DEM, when the DEM fits 32-bit offsets into them, else L = 9 runs as L = 8).
- * Defaults: the fastest split layout per precision on one B200; rows 2x1 for
- * FP64 (the only layout it runs).  Results do not depend on any of them. */
+ * Defaults: the fastest split layout per precision on one B200; FP64
+ * reports rows 2x1 and runs a split form of its own until a configuration is set,
+ * then the row layout that was set.  Results do not depend on any of them. */
 typedef struct tvs_sweep_config {
     int32_t points_x;
     int32_t points_y;

@@ -147,3 +147,41 @@ def test_ring_records_where_segments_are_skipped(tvs, oracle, synth, precision, 
             span = offsets[s * per:(s + 1) * per + 1]
             assert np.array_equal(np.diff(span).astype(np.uint32), n0)
             assert np.array_equal(ids[span[0]:span[-1]], ids0)
+
+
+@pytest.mark.parametrize("precision", ["exact32", "mixed64", "fp64"])
+@pytest.mark.parametrize("planes_before", [0, 1, 20])
+def test_sweeps_in_a_callers_capture(tvs, synth, precision, planes_before):
+    """A caller's graph of a sweep computes the sweep whatever planes there were when it
+    was captured (none, one sector's, all), and after the context's planes have grown."""
+    import torch
+
+    z = synth.fbm(301, 301, 0.8, 5, 0.0, 1500.0)
+    with tvs.Engine(z, 301, 30.0, 3000, observer_height=1.65, precision=precision) as eng, \
+            tvs.Engine(z, 301, 30.0, 3000, observer_height=1.65, precision=precision) as other:
+        other.device_reset()
+        other.device_run_sectors(40, 20)
+        other.device_finish()
+        want, _ = other.read_surfaces()
+        if planes_before:
+            eng.device_run_sectors(40, planes_before)
+        else:  # (uploads what a first sweep uploads; a held tile takes no planes)
+            eng.set_queue_wait(0, 1 << 30)
+            eng.device_run_sectors(40, 1)
+            eng.set_queue_wait()
+        eng.device_finish()
+        graph = torch.cuda.CUDAGraph()
+        stream = torch.cuda.ExternalStream(eng.stream())
+        with torch.cuda.stream(stream):
+            graph.capture_begin(capture_error_mode="thread_local")
+            eng.device_reset()
+            eng.device_run_sectors(40, 20)
+            graph.capture_end()
+        for _ in range(2):
+            with torch.cuda.stream(stream):
+                graph.replay()
+            eng.device_finish()
+            got, _ = eng.read_surfaces()
+            assert np.array_equal(bits(got), bits(want))
+            eng.run()  # 180 sectors: more planes
+        del graph

@@ -22,7 +22,6 @@ thread_local std::string g_create_error;
 constexpr double kRadsPerDeg = 3.14159265358979323846 / 180.0;  // Rust f64::to_radians
 constexpr double kSqrt2 = 1.41421356237309504880;               // core::f64::consts::SQRT_2
 constexpr uint32_t kSpillCap = 1u << 22;
-constexpr size_t kSmallPlanes = (size_t)4 << 20;  // planes that a new context comes with
 
 int fail(tvs_context *ctx, int code, const std::string &msg) {
     if (ctx) ctx->err = msg; else g_create_error = msg;
@@ -153,6 +152,7 @@ void free_all(tvs_context *c) {
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (c->d_planes) tvs::plane_free(c->d_planes, c->stream);
+    for (void *p : c->old_planes) tvs::plane_free(p, c->stream);
     drop_tvs_graph(c);
     for (cudaEvent_t ev : {c->ev_begin, c->ev_shaped, c->ev_swept})
         if (ev) cudaEventDestroy(ev);
@@ -396,17 +396,32 @@ int ring_queue_dem(tvs_context *c, const tvs::QueueDem **dem, uint32_t *tiles, u
 
 // The split sweep's surface planes for a sweep of n_sectors and the sectors that
 // each of its launches takes; null (and every sector) where it adds the surfaces
-// in turn: a held tile of the failure test, or no memory for the planes.
+// in turn: a held tile of the failure test, or no memory for the planes.  A caller's
+// capture of the context's stream takes the planes that there are, and those then
+// stay where they are until the context's end.
 void *ensure_planes(tvs_context *c, const tvs::QueueConfig &q, uint32_t tiles, uint32_t n_sectors,
                     uint32_t *sectors) {
     const size_t need = tvs::split_plane_bytes((int)c->p.precision, q, tiles, n_sectors, sectors);
     if (need != 0 && c->held_tile == 0xFFFFFFFFu) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        cudaStreamIsCapturing(c->stream, &capture);
+        if (capture != cudaStreamCaptureStatusNone && !c->capturing_tvs) c->planes_captured = true;
         if (need <= c->planes_cap) return c->d_planes;
+        if (capture != cudaStreamCaptureStatusNone) {
+            const size_t one = need / *sectors;
+            *sectors = c->planes_cap >= one ? (uint32_t)(c->planes_cap / one) : n_sectors;
+            return c->planes_cap >= one ? c->d_planes : nullptr;
+        }
         if (c->d_planes) {
             cudaStreamSynchronize(c->stream);
-            tvs::plane_free(c->d_planes, c->stream);
+            if (c->planes_captured) {
+                c->old_planes.push_back(c->d_planes);
+            } else {
+                tvs::plane_free(c->d_planes, c->stream);
+                c->device_bytes -= c->planes_cap;
+            }
+            c->planes_captured = false;
         }
-        c->device_bytes -= c->planes_cap;
         c->d_planes = nullptr;
         c->planes_cap = 0;
         drop_tvs_graph(c);  // a captured sweep holds the old planes
@@ -919,26 +934,6 @@ int tvs_create(const tvs_params *params, const float *elevations, uint64_t n_ele
     for (auto &a : allocs) {
         if ((e = cudaMalloc(a.p, a.bytes)) != cudaSuccess) return bail(e, "cudaMalloc");
         c->device_bytes += a.bytes;
-    }
-    // a small grid's planes for one sector, so that the first call of a per-sector
-    // loop allocates nothing
-    if (params->sweep_kernel == TVS_SWEEP_ENGINE) {
-        tvs::QueueDem d{};
-        d.tvs_width = g.tvs_width;
-        d.row_begin = rb;
-        d.row_end = re;
-        uint32_t tiles = 0, done = 0, chunks = 0, per = 0;
-        tvs::queue_tile(&d, 1, c->qcfg, &tiles, &done, &chunks);
-        const size_t need = tvs::split_plane_bytes((int)params->precision, c->qcfg, tiles, 1, &per);
-        if (need != 0 && need <= kSmallPlanes) {
-            if (tvs::plane_alloc(&c->d_planes, need, c->stream) == cudaSuccess) {
-                c->planes_cap = need;
-                c->device_bytes += need;
-            } else {
-                cudaGetLastError();
-                c->d_planes = nullptr;
-            }
-        }
     }
     c->d_done = c->d_queue + 1;
     if (params->precision == TVS_PRECISION_MIXED64 || params->precision == TVS_PRECISION_FP64) {
@@ -1508,7 +1503,9 @@ int tvs_device_run_tvs(tvs_context *ctx) {
         if (rc) return rc;
         const uint64_t plain = ctx->launches;
         TVS_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+        ctx->capturing_tvs = true;
         rc = enqueue_tvs(true);
+        ctx->capturing_tvs = false;
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
         if (rc != TVS_OK) {

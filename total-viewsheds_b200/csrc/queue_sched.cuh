@@ -1,5 +1,6 @@
-// queue_sched.cuh -- the work queue shared by the persistent sweeps
-// (sweep_queue.cu: row layouts; sweep_split.cu: direction-split layouts).
+// queue_sched.cuh -- the tile shapes of the persistent sweeps (sweep_queue.cu: row
+// layouts; sweep_split.cu: direction-split layouts) and the row layouts' queue (the
+// split sweep's is described and kept in its file).
 //
 // The grid is the resident capacity of the GPU.  Each CTA takes the next
 // (sector, tile) item from a global counter in sector-major order, re-stages

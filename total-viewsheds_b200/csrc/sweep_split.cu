@@ -1364,16 +1364,6 @@ cudaError_t launch_persistent(const void *fn, const QueueArgs &a, uint64_t items
     return cudaGetLastError();
 }
 
-size_t split_smem_bytes(int precision, uint32_t step_cap) {
-    switch (precision) {
-    case TVS_PRECISION_FP64: return SplitSmem<TVS_PRECISION_FP64>::total(step_cap, 2);
-    case TVS_PRECISION_EXACT32: return SplitSmem<TVS_PRECISION_EXACT32>::total(step_cap, 2);
-    case TVS_PRECISION_MIXED64: return SplitSmem<TVS_PRECISION_MIXED64>::total(step_cap, 2);
-    case TVS_PRECISION_FP32: return SplitSmem<TVS_PRECISION_FP32>::total(step_cap, 2);
-    default: return 0;
-    }
-}
-
 namespace {
 struct PlanePool {
     cudaMemPool_t pool = nullptr;

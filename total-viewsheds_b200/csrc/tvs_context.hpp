@@ -3,6 +3,7 @@
 
 #include <cstdint>
 #include <string>
+#include <vector>
 
 #include "tvs.h"
 #include "tvs_internal.cuh"
@@ -44,6 +45,9 @@ struct tvs_context {
     uint32_t q_tiles_per_sector = 0, q_chunks = 0;
     void *d_planes = nullptr;                  // split_plane_bytes (grown on use)
     size_t planes_cap = 0;
+    bool capturing_tvs = false;                // tvs_device_run_tvs captures its own graph
+    bool planes_captured = false;              // a caller's graph may hold d_planes
+    std::vector<void *> old_planes;            // ... or these
     uint32_t spin_limit = tvs::kDefaultSpinLimit;  // dependency-wait iteration limit
     uint32_t held_tile = 0xFFFFFFFFu;               // failure-detection test hook
     int32_t *d_deltas = nullptr;

@@ -311,10 +311,9 @@ cudaError_t launch_sweep_const(const SweepArgs &a, int precision, uint32_t n_ste
 cudaError_t launch_sweep_plain(const PlainArgs &a, cudaStream_t s);
 cudaError_t launch_sweep_queue(const QueueArgs &a, int precision, const QueueConfig &c,
                                cudaStream_t s);
-// The direction-split layouts 1-6 (sweep_split.cu): EXACT32, MIXED64 and
-// FP32; ring records when a.rings is set (one sector).
+// The direction-split layouts 1-9 (sweep_split.cu): every precision; ring records
+// (not FP64's) when a.rings is set.
 cudaError_t launch_sweep_split(const QueueArgs &a, int precision, int layout, cudaStream_t s);
-size_t split_smem_bytes(int precision, uint32_t step_cap);
 uint32_t queue_tiles_bound(uint32_t tvs_width, uint32_t rows);
 bool queue_config_valid(const QueueConfig &c);
 QueueConfig default_queue_config(int precision);
