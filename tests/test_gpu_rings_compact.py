@@ -255,3 +255,20 @@ def test_contexts_of_several_threads_share_the_host_buffers(tvs, dem):
     for g, w in zip(got, want):
         for x, y in zip(g, w):
             assert np.array_equal(bits(x), bits(y))
+
+
+@pytest.mark.parametrize("rpk", [5.0, 60.0])
+def test_gather_of_long_and_short_records(tvs, oracle, rpk):
+    """Noise on a bowl: records of 2 to 44 ids, past what a lane reads ahead; 5/km clips them at 15 slots."""
+    rng = np.random.default_rng(3)
+    y, x = np.mgrid[:W, :W].astype(np.float64) - W / 2
+    z = (30.0 * 1e-4 * 30.0 * (x * x + y * y) + rng.uniform(0, 12.0, (W, W))).astype(np.float32)
+    z[: W // 2, : W // 2] = 0.0
+    angles = [0, 45]
+    want = oracle_records(oracle, z, angles, rpk=60.0)
+    assert max(int(np.diff(o.astype(np.int64)).max()) for o, _ in want) > 30
+    with tvs.Engine(z, W, SCALE, LOS, rings_per_km=rpk, observer_height=OBS) as eng:
+        cum = np.zeros(eng.count, np.float32)
+        for a, (wo, wi) in zip(angles, want):
+            off, ids, _ = eng.compute_sector_rings(a, cum)
+            assert np.array_equal(off, wo) and np.array_equal(ids, wi), a

@@ -83,48 +83,65 @@ __global__ void __launch_bounds__(kRingThreads) k_ring_scan_blocks(uint64_t *blo
 
 // offsets[band] for every band (and offsets[bands] = total); the in-slot ids of
 // every band copied to ids[offsets[band] ..).
+//
+// Bound by the latency of its scattered reads, so by the reads in flight: eight lanes
+// move a record's ids (9 to 15 of them on rough terrain), a warp has sixteen records
+// under way and a lane up to kRingAhead ids of each of its four before the first is
+// stored; their places come from shared memory.  With one read per lane under way and
+// the places from eight shuffles per four records, the first six groups of six sectors
+// at 3601^2 (1 GB of ids each) took 1.65 ms, now 0.80; with the ids past the first 24
+// of a record one by one, 1.05.
+constexpr int kRingAhead = 3;
 __global__ void __launch_bounds__(kRingThreads)
 k_ring_gather(const uint32_t *lens, uint32_t stride, const uint32_t *rings, uint64_t bands,
               uint32_t reserved, const uint64_t *block_base, uint64_t *offsets, uint32_t *ids) {
-    const uint64_t b0 = (uint64_t)blockIdx.x * kRingChunk + (uint64_t)threadIdx.x * kRingPer;
+    __shared__ uint32_t s_at[kRingChunk + 1];  // within the CTA's ids
+    const uint64_t cta_b0 = (uint64_t)blockIdx.x * kRingChunk, base = block_base[blockIdx.x];
+    const uint32_t t0 = threadIdx.x * kRingPer;
     uint32_t len[kRingPer];
     uint64_t s = 0;
 #pragma unroll
     for (int j = 0; j < kRingPer; j++) {
-        len[j] = record_length(lens, stride, b0 + j, bands);
+        len[j] = record_length(lens, stride, cta_b0 + t0 + j, bands);
         s += len[j];
     }
     __shared__ uint64_t total;
-    uint64_t off = block_base[blockIdx.x] + block_exclusive(s, &total);
-    uint64_t at[kRingPer];
+    uint64_t off = block_exclusive(s, &total);
 #pragma unroll
     for (int j = 0; j < kRingPer; j++) {
-        at[j] = off;
-        if (b0 + j < bands) offsets[b0 + j] = off;
+        s_at[t0 + j] = (uint32_t)off;
+        if (cta_b0 + t0 + j < bands) offsets[cta_b0 + t0 + j] = base + off;
         off += len[j];
     }
-    // The warp copies its 32 x kRingPer records in band order, four at a time: eight
-    // lanes move a record's ids (about nine of them on rough terrain), so the writes
-    // of a step are four runs that follow each other.  A whole warp per record kept
-    // one load in flight and 23 lanes idle: 1201^2, six sectors, 0.20 ms.
+    if (threadIdx.x == kRingThreads - 1) s_at[kRingChunk] = (uint32_t)off;
+    __syncthreads();
     const uint32_t lane = threadIdx.x & 31u, sub = lane >> 3, q0 = lane & 7u;
-    const uint64_t warp_b0 = (uint64_t)blockIdx.x * kRingChunk + (uint64_t)(threadIdx.x & ~31u) * kRingPer;
-    static_assert(kRingPer == 4, "a thread's records are one step of its warp");
-#pragma unroll 4
-    for (uint32_t src = 0; src < 32; src++) {
-        // the four records of thread src, one per eight lanes
-        uint32_t n = 0;
-        uint64_t o = 0;
+    const uint32_t warp_r0 = (threadIdx.x & ~31u) * kRingPer;
+    uint32_t *out = ids + base;
+    for (uint32_t r0 = warp_r0; r0 < warp_r0 + 32 * kRingPer; r0 += 16) {
+        uint32_t at[4], n[4], most = 0;
+        const uint32_t *rec[4];
 #pragma unroll
-        for (int j = 0; j < kRingPer; j++) {
-            const uint32_t nj = __shfl_sync(0xffffffffu, min(len[j], reserved - 1), src);
-            const uint64_t oj = __shfl_sync(0xffffffffu, at[j], src);
-            if (sub == (uint32_t)j) n = nj, o = oj;
+        for (int i = 0; i < 4; i++) {
+            const uint32_t r = r0 + 4 * i + sub;
+            at[i] = s_at[r];
+            n[i] = min(s_at[r + 1] - at[i], reserved - 1);  // (0 past the last band)
+            most = max(most, n[i]);
+            rec[i] = rings + (cta_b0 + r) * reserved + 1;
         }
-        const uint64_t band = warp_b0 + (uint64_t)src * kRingPer + sub;
-        if (band >= bands) n = 0;
-        const uint32_t *rec = rings + band * reserved + 1;
-        for (uint32_t q = q0; q < n; q += 8) ids[o + q] = __ldcs(rec + q);
+        for (uint32_t q = q0; q < most; q += 8 * kRingAhead) {
+            uint32_t v[4][kRingAhead];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int t = 0; t < kRingAhead; t++)
+                    if (q + 8 * t < n[i]) v[i][t] = __ldcs(rec[i] + q + 8 * t);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int t = 0; t < kRingAhead; t++)
+                    if (q + 8 * t < n[i]) out[at[i] + q + 8 * t] = v[i][t];
+        }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) offsets[bands] = block_base[gridDim.x];
 }
