@@ -267,7 +267,7 @@ uint64_t tvs_last_launch_count(const tvs_context *ctx);
 /* Bytes of device memory the context holds: the buffers of tvs_create, the
  * surface planes from the first sweep on, the ring buffers from the first run
  * that asks for ring records.  (The planes come from a pool per device that may
- * keep up to 512 MB of freed ones until the process's last context there ends.) */
+ * keep up to 1 GB of freed ones until the process's last context there ends.) */
 uint64_t tvs_device_bytes(const tvs_context *ctx);
 
 /* Failure detection of the persistent sweep (no counterpart in the reference,

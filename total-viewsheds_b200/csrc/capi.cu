@@ -147,8 +147,8 @@ void free_all(tvs_context *c) {
                     c->d_rechecks, c->d_qdem,
                     c->d_deltas, c->d_dists, c->d_rings, c->d_spill, c->d_counters, c->d_sf,
                     c->d_sb, c->d_tab_deltas, c->d_tab_dists, c->d_installed,
-                    c->d_rc_blocks, c->d_rc_offsets, c->d_rc_lens, c->d_rc_ids, c->d_ref_scan, c->d_ref_ids, c->d_bmax, c->d_qdem_rings,
-                    c->d_diag, c->d_quad};
+                    c->d_rc_blocks, c->d_rc_offsets, c->d_rc_lens, c->d_rc_ids, c->d_ref_scan,
+                    c->d_ref_ids, c->d_bmax, c->d_qdem_rings, c->d_diag, c->d_quad};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (c->d_planes) tvs::plane_free(c->d_planes, c->stream);
@@ -941,8 +941,9 @@ int tvs_create(const tvs_params *params, const float *elevations, uint64_t n_ele
             return bail(e, "cudaMalloc");
         c->device_bytes += count * sizeof(double);
     }
-    // the quad layout's copies (4x the DEM); without them (the plain kernel, a DEM past the 32-bit offsets, or no memory for them) the quad
-    // layout's tiling runs from the plain DEM
+    // the quad layout's copies (4x the DEM); without them (the plain kernel, a DEM past
+    // the 32-bit offsets, or no memory for them) the quad layout's tiling runs from the
+    // plain DEM
     if (params->sweep_kernel == TVS_SWEEP_ENGINE && tvs::quad_fits(g.width, g.height)) {
         const size_t qb = 4 * tvs::quad_copy_elems(g.width, g.height) * sizeof(float4);
         if (cudaMalloc(&c->d_quad, qb) == cudaSuccess) {

@@ -39,10 +39,12 @@ constexpr uint32_t kSplitChunk = 8, kSplitGrab = 8;
 // per sector and direction) of kPlaneBytes, and kPlaneSectors of a large DEM's up
 // to kPlaneBytesMost: the end of a launch leaves the GPU half idle for one tile's
 // time (12 tiles of up to 1601^2: 65.0, 57.5, 53.6 and 51.8 ms with 32, 64, 128 and
-// 256 MB).
+// 256 MB; 3601^2 MIXED64, 23 MB a sector: 103.5, 100.6 and 98.9 ms with 16, 32 and 64
+// sectors, exact f32 83.5, 82.4 and 81.3; 7201^2 MIXED64 with 1, 2 and 4 GB: 785, 779
+// and 774 ms, and as much as that longer to map them).
 constexpr size_t kPlaneBytes = (size_t)256 << 20, kPlaneBytesMost = (size_t)1 << 30;
-constexpr uint32_t kPlaneSectors = 16;
-constexpr uint64_t kPlanePoolBytes = (uint64_t)512 << 20;
+constexpr uint32_t kPlaneSectors = 32;
+constexpr uint64_t kPlanePoolBytes = kPlaneBytesMost;
 
 // Direction-split layouts 1-9: a warp holds LX columns x 32/LX rows of lanes;
 // each lane sweeps four points of view, LX columns apart (layouts 1-3: LX = 8,

@@ -78,7 +78,8 @@ namespace tvs {
 namespace {
 
 constexpr int K = kSplitCols;     // chains per lane
-// Iterations of a wait for a chunk of the CTA's own ring (of about 100 ns: seconds, against a real wait of at most a few work items).
+// Iterations of a wait for a chunk of the CTA's own ring (of about 100 ns: seconds,
+// against a real wait of at most a few work items).
 constexpr uint32_t kRingSpinLimit = 1u << 25;
 
 __device__ __forceinline__ float div_table32(float e, float y, float d) {
