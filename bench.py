@@ -283,7 +283,7 @@ def run_batching(args, rank, world, local, torch):
                 "autotuned_sweep": repr(cfg), "autotune_s": tune_s,
                 "los_samples_per_step": ref_samples, "evaluated_samples_per_step": eval_samples,
                 "hbm_bytes_batch": b.device_bytes(),
-                "launches_per_step": "1 graph replay: surface resets, 1 shape launch, 1 sweep",
+                "launches_per_step": "1 graph replay: surface resets, 1 shape launch, the sweep",
                 "l2": "flushed between steps (256 MiB write)",
             },
             "clocks": clocks.summary(),
@@ -597,7 +597,8 @@ def main():
             "peak": fp32_peak / 1e12, "unit": "Tinstr/s", "frac": achieved / fp32_peak,
             "traffic": (traffic_from_profiles(f"k_sweep_split<{args.precision}>")
                         if args.kernel == "engine" else None),
-            "kernel": f"k_sweep_split<{args.precision}> (one persistent launch: 180 sectors)"
+            "kernel": f"k_sweep_split<{args.precision}> (persistent launches of as many sectors "
+                      "as have surface planes)"
                       if args.kernel == "engine" else "k_sweep_plain (one launch per sector)",
             "algorithmic_work": "5 FP32 instructions per evaluated sample (sub, fma, setp, max, "
                                 "predicated add); the 2 zero-distance tail steps are the last "
