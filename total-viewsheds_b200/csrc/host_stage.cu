@@ -12,7 +12,7 @@ namespace tvs_host {
 namespace {
 
 struct Stage {
-    std::mutex refs;  // users, and the block's existence
+    std::mutex refs;  // users
     int users = 0;
     std::mutex lent;  // held by the call that uses the block
     unsigned char *block = nullptr;
@@ -34,10 +34,14 @@ void stage_ref(bool device_set) {
     st.users++;
     std::lock_guard<std::mutex> lent(st.lent);
     if (st.block || !device_set) return;
-    if (cudaHostAlloc((void **)&st.block, kSmall, cudaHostAllocPortable) != cudaSuccess) {
+    void *p = nullptr;
+    if (posix_memalign(&p, 4096, kSmall) != 0) return;
+    if (cudaHostRegister(p, kSmall, cudaHostRegisterPortable) != cudaSuccess) {
         cudaGetLastError();
-        st.block = nullptr;
+        std::free(p);
+        return;
     }
+    st.block = (unsigned char *)p;
 }
 
 void stage_unref() {
@@ -45,8 +49,6 @@ void stage_unref() {
     std::lock_guard<std::mutex> lock(st.refs);
     if (--st.users > 0) return;
     std::lock_guard<std::mutex> lent(st.lent);
-    if (st.block) cudaFreeHost(st.block);
-    st.block = nullptr;
     std::lock_guard<std::mutex> records(st.records_lent);
     if (st.records) cudaFreeHost(st.records);
     st.records = nullptr;

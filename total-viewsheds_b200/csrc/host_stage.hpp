@@ -10,9 +10,10 @@ namespace tvs_host {
 
 // A copy to pageable memory waits by itself and goes through the driver's own pinned
 // buffer.  The small results of a call share a pinned block instead, so that one
-// wait serves all.  The block belongs to the process, from the first context to the
-// last, and is lent to one call at a time; a call that finds it lent (another
-// thread's) takes the driver's path.
+// wait serves all.  The block is ordinary memory of the process, pinned with its first
+// context and left so (pinning and unpinning it with every only context of a program
+// took 2.6 ms of a 301^2 context's 3.5), and is lent to one call at a time; a call that
+// finds it lent (another thread's) takes the driver's path.
 constexpr size_t kSmall = 256 << 10;
 
 void stage_ref(bool device_set);  // a context exists, its device current
@@ -35,8 +36,8 @@ private:
 };
 
 // Host memory for the compact records of one call, for as long as this lives: the
-// process's pinned buffer (grown up to kPinnedMost, lent and given back as the block
-// above is, done() included), or memory of its own where that is lent or too small.
+// process's pinned buffer (grown up to kPinnedMost, lent as the block above is, done()
+// included, and freed with the last context), or memory of its own where that is lent or too small.
 class RecordBuffer {
 public:
     explicit RecordBuffer(cudaStream_t stream);
