@@ -404,7 +404,7 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
             const uint32_t nf = uni(h->n_fast);
             // surfaces stop at the last step that adds to them
             const uint32_t n = uni(kRings ? h->n_steps : max(nf, min(h->n_surf, h->n_steps)));
-            const bool plain = !kQuad || uni(h->wide) != 0;
+            const bool wide = uni(h->wide) != 0, plain = !kQuad || wide;
             const float4 *gs = D.steps + (uint64_t)slot * D.step_cap;
             const int2 *go = D.offs + (uint64_t)slot * D.step_cap;
             const int2 *gq = D.quads + (uint64_t)slot * D.step_cap;
@@ -481,6 +481,9 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                         ymin = fminf(ymin, __shfl_xor_sync(0xffffffffu, ymin, o));
                         zmax = fmaxf(zmax, __shfl_xor_sync(0xffffffffu, zmax, o));
                     }
+                    // (no segment of a wide sector is skipped: its linear sample ids wrap into
+                    // neighbouring rows, where the moved patch does not bound them)
+                    if (wide) zmax = INFINITY;
                     if (lane == 0) {
                         const int4 q = gseg[b];
                         s_seg[b] = dir ? SegBound{-q.y, -q.x, -q.w, -q.z, ymax, ymin, zmax, 0.0f}
@@ -738,7 +741,7 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                     return warp_max(m);
                 };
                 // A segment can be skipped when no chain can change state at
-                // any of its steps: every sample h <= B, so e <= RN(B - h_pov)
+                // any of its steps (in a wide sector never): every sample h <= B, so e <= RN(B - h_pov)
                 // and the first test's value fma(e, y, z) is at most
                 // fma(RN(B - h_pov), y_max or y_min, z_max) (RN and fma are
                 // monotone).  A chain visible at the previous step closes its ring
