@@ -64,6 +64,7 @@
 // (kernel.rs:141-145,220-243).  Where a step or a segment is skipped, the chains
 // visible before it close their rings at it.
 #include <algorithm>
+#include <cfloat>
 #include <climits>
 #include <map>
 #include <mutex>
@@ -850,9 +851,12 @@ k_sweep_split(QueueArgs a, uint32_t n_slots) {
                     float lo[K];
 #pragma unroll
                     for (int k = 0; k < K; k++) {
-                        const bool on = active >> k & 1u;  // off the grid: never visible
-                        m[k] = on ? (double)kMaxAngle : (double)INFINITY;
-                        lo[k] = on ? __fmaf_rn(2000.0f, -kRel, kMaxAngle) : INFINITY;
+                        // off the grid: above every angle, and finite (an infinite m makes lo
+                        // a NaN at the warp's first passing step, below which no bound
+                        // lies: the tile then skipped no segment any more)
+                        const float first = active >> k & 1u ? kMaxAngle : FLT_MAX;
+                        m[k] = (double)first;
+                        lo[k] = __fmaf_rn(fabsf(first), -kRel, first);
                         acc[k] = 0.0;
                     }
                     const double o64 = (double)D.observer_height;
