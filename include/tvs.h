@@ -306,9 +306,10 @@ int tvs_read_sweep_counters(tvs_context *ctx, uint64_t *counters);
  * L = 9 is L = 8's tiling read from four row-interleaved copies of the DEM
  * (one 16-byte load per lane and step; the context holds the copies, 4x the
  * DEM, when the DEM fits 32-bit offsets into them, else L = 9 runs as L = 8).
- * Defaults: the fastest split layout per precision on one B200; FP64
- * reports rows 2x1 and runs a split form of its own until a configuration is set,
- * then the row layout that was set.  Results do not depend on any of them. */
+ * Defaults: the fastest split layout per precision on one B200; FP64's is rows 2x1
+ * (no prefetch, not packed), which names a split form of its own, the other row
+ * configurations its row kernel.  A configuration that was read (or chosen by the
+ * autotuner) can be set again.  Results do not depend on any of them. */
 typedef struct tvs_sweep_config {
     int32_t points_x;
     int32_t points_y;

@@ -46,3 +46,72 @@ def test_step_loop_remainders(tvs, oracle, synth, los):
             cum = np.zeros(eng.count, np.float32)
             eng.compute_sector(angle, cum)
             assert np.array_equal(bits(cum), bits(want.astype(np.float32))), angle
+
+
+def swept(eng):
+    """Whether the split form ran: it counts its steps, the row kernel does not."""
+    eng.sweep_counters(True)
+    out = eng.run()[:2]
+    steps = eng.sweep_counters()[2]
+    eng.sweep_counters(False)
+    return steps > 0, out
+
+
+def set_again(eng, c):
+    eng.set_sweep_config(c.points_x, c.points_y, bool(c.packed), bool(c.prefetch), c.layout)
+
+
+def fields(c):
+    return c.points_x, c.points_y, c.packed, c.prefetch, c.layout
+
+
+def test_configuration_read_and_set_back(tvs, synth):
+    """What is read, or chosen by the autotuner, names what runs: setting it changes
+    nothing.  The row kernel stays within reach and agrees bit for bit."""
+    z = np.round(synth.fbm(301, 301, 0.7, 9, 0.0, 1500.0))
+    with tvs.Engine(z, 301, 30.0, 3000, observer_height=1.65, precision="fp64") as eng:
+        split, want = swept(eng)
+        assert split
+        before = eng.sweep_config()
+        set_again(eng, before)
+        assert fields(eng.sweep_config()) == fields(before) and swept(eng)[0]
+        for px, py, prefetch in ((1, 1, False), (4, 1, False), (2, 2, False), (2, 1, True)):
+            eng.set_sweep_config(px, py, prefetch=prefetch)
+            split, got = swept(eng)
+            assert not split
+            for a, b in zip(got, want):
+                assert np.array_equal(bits(a), bits(b))
+        chosen = eng.autotune(4)
+        tuned = swept(eng)[0]
+        set_again(eng, chosen)
+        assert fields(eng.sweep_config()) == fields(chosen) and swept(eng)[0] == tuned
+        set_again(eng, before)
+        assert swept(eng)[0]
+        with pytest.raises(tvs.TvsError):
+            eng.set_sweep_config(4, 1, layout=9)
+
+
+def test_batch_configuration_read_and_set_back(tvs, synth):
+    import ctypes
+
+    z = np.round(synth.fbm(257, 261, 0.7, 5, 0.0, 900.0))
+    with tvs.Batch([(z, 30.0, 2550)], observer_height=1.65, precision="fp64") as b:
+        def config():
+            c = tvs.SweepConfig()
+            assert tvs.lib().tvs_batch_get_sweep_config(b.b, ctypes.byref(c)) == tvs.OK
+            return c
+
+        def run():
+            b.run()
+            b.finish()
+            return b.read(0)
+
+        want, held = run(), b.device_bytes()  # (the split form's surface planes are in it)
+        before = config()
+        set_again(b, before)
+        assert fields(config()) == fields(before) and b.device_bytes() == held
+        for c in (b.autotune(4), before):
+            set_again(b, c)
+            assert fields(config()) == fields(c)
+            for x, y in zip(run(), want):
+                assert np.array_equal(bits(x), bits(y))

@@ -270,7 +270,7 @@ int tvs_batch_set_sweep_config(tvs_batch *b, const tvs_sweep_config *cfg) {
         return bfail(b, TVS_ERR_INVALID_ARGUMENT, "sweep layouts 1-9 are not available for FP64");
     if (c.layout == 0 && b->precision == TVS_PRECISION_FP32)
         return bfail(b, TVS_ERR_INVALID_ARGUMENT, "the FP32 form runs on sweep layouts 1-9 only");
-    return set_config(b, c);
+    return set_config(b, tvs::run_config((int)b->precision, c));
 }
 
 int tvs_batch_get_sweep_config(const tvs_batch *b, tvs_sweep_config *cfg) {
@@ -301,11 +301,8 @@ int tvs_batch_autotune(tvs_batch *b, uint32_t sample_sectors, tvs_sweep_config *
     tvs::QueueConfig best_cfg = b->cfg;
     int rc = TVS_OK;
     for (const tvs::QueueConfig &c : cands) {
-        // (FP64's split form is tiled as layout 9 and not selected by name)
-        if ((c.packed && !exact) || (c.layout != 0 && c.layout != tvs::kQuadLayout && f64) ||
-            (c.layout == 0 && fp32))
-            continue;
-        if ((rc = set_config(b, c))) break;
+        if ((c.packed && !exact) || (c.layout != 0 && f64) || (c.layout == 0 && fp32)) continue;
+        if ((rc = set_config(b, tvs::run_config((int)b->precision, c)))) break;
         float ms = 0.0f;
         for (int rep = 0; rep < 2 && rc == TVS_OK; rep++) {  // the first run warms up
             cudaEventRecord(t0, b->stream);
@@ -318,7 +315,7 @@ int tvs_batch_autotune(tvs_batch *b, uint32_t sample_sectors, tvs_sweep_config *
         if (rc) break;
         if (ms < best) {
             best = ms;
-            best_cfg = c;
+            best_cfg = b->cfg;
         }
     }
     cudaEventDestroy(t0);

@@ -815,7 +815,7 @@ int collect_rings(tvs_context *c, uint32_t *rings, uint64_t rings_len, tvs_secto
 void tvs_set_create_error(const std::string &msg) { g_create_error = msg; }
 
 namespace tvs_host {
-// A sweep configuration as callers see it: FP64's split form is its rows 2x1.
+// A sweep configuration as callers see it (tvs::run_config's inverse).
 tvs_sweep_config public_config(int precision, const tvs::QueueConfig &c) {
     if (precision == TVS_PRECISION_FP64 && c.layout != 0) return tvs_sweep_config{2, 1, 0, 0, 0};
     return tvs_sweep_config{c.px, c.py, c.packed, c.prefetch, c.layout};
@@ -1375,6 +1375,7 @@ int tvs_set_sweep_config(tvs_context *ctx, const tvs_sweep_config *cfg) {
         return fail(ctx, TVS_ERR_INVALID_ARGUMENT, "sweep layouts 1-9 are not available for FP64");
     if (c.layout == 0 && ctx->p.precision == TVS_PRECISION_FP32)
         return fail(ctx, TVS_ERR_INVALID_ARGUMENT, "the FP32 form runs on sweep layouts 1-9 only");
+    c = tvs::run_config((int)ctx->p.precision, c);
     if (c.px != ctx->qcfg.px || c.py != ctx->qcfg.py || c.packed != ctx->qcfg.packed ||
         c.prefetch != ctx->qcfg.prefetch || c.layout != ctx->qcfg.layout)
         drop_tvs_graph(ctx);
@@ -1411,11 +1412,8 @@ int tvs_autotune(tvs_context *ctx, uint32_t sample_sectors, tvs_sweep_config *ch
     int rc = enqueue_shape(ctx, 0, sample_sectors);
     for (const tvs::QueueConfig &c : cands) {
         if (rc) break;
-        // (FP64's split form is tiled as layout 9 and not selected by name)
-        if ((c.packed && !exact) || (c.layout != 0 && c.layout != tvs::kQuadLayout && f64) ||
-            (c.layout == 0 && fp32))
-            continue;
-        ctx->qcfg = c;
+        if ((c.packed && !exact) || (c.layout != 0 && f64) || (c.layout == 0 && fp32)) continue;
+        ctx->qcfg = tvs::run_config((int)ctx->p.precision, c);
         float ms = 0.0f;
         for (int rep = 0; rep < 2 && rc == TVS_OK; rep++) {  // the first run warms up
             cudaEventRecord(t0, ctx->stream);
@@ -1427,7 +1425,7 @@ int tvs_autotune(tvs_context *ctx, uint32_t sample_sectors, tvs_sweep_config *ch
         }
         if (rc == TVS_OK && ms < best) {
             best = ms;
-            best_cfg = c;
+            best_cfg = ctx->qcfg;
         }
     }
     cudaEventDestroy(t0);

@@ -603,9 +603,7 @@ bool queue_config_valid(const QueueConfig &c) {
 }
 
 QueueConfig default_queue_config(int precision) {
-    static bool rows = false;  // the environment asks for a row layout
     static QueueConfig v = [] {
-        rows = getenv("TVS_SWEEP_SHAPE") || getenv("TVS_SWEEP_PACKED") || getenv("TVS_SWEEP_PREFETCH");
         QueueConfig d{2, 1, 0, 0, 0};
         const char *e = getenv("TVS_SWEEP_SHAPE");
         int x = 0, y = 0;
@@ -619,12 +617,18 @@ QueueConfig default_queue_config(int precision) {
         if (f) d.prefetch = atoi(f) != 0;
         return d;
     }();
-    // FP64's split form takes the quad layout's tiling and no other; callers see it
-    // as rows 2x1, the one configuration that FP64 always had by default, and get
-    // the row kernel, which evaluates every step in double, by setting one (1201^2,
-    // 180 sectors: rows 13.5 ms).
-    if (precision == TVS_PRECISION_FP64) return rows ? v : QueueConfig{kSplitCols, 1, 0, 0, kQuadLayout};
-    return default_split_config(precision);
+    return precision == TVS_PRECISION_FP64 ? run_config(precision, v) : default_split_config(precision);
+}
+
+// FP64's split form takes the quad layout's tiling and no other.  Callers know it as
+// rows 2x1, the one configuration that FP64 always had by default; every other row
+// configuration is the row kernel's, which evaluates every step in double (1201^2, 180
+// sectors: rows 13.5 ms, the split form 6.1).  One name per form: what is read back
+// from a context can be set again.
+QueueConfig run_config(int precision, const QueueConfig &named) {
+    const bool split = precision == TVS_PRECISION_FP64 && named.px == 2 && named.py == 1 &&
+                       !named.packed && !named.prefetch && named.layout == 0;
+    return split ? QueueConfig{kSplitCols, 1, 0, 0, kQuadLayout} : named;
 }
 
 QueueConfig default_split_config(int precision) {

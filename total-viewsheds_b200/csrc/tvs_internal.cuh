@@ -317,6 +317,8 @@ cudaError_t launch_sweep_split(const QueueArgs &a, int precision, int layout, cu
 uint32_t queue_tiles_bound(uint32_t tvs_width, uint32_t rows);
 bool queue_config_valid(const QueueConfig &c);
 QueueConfig default_queue_config(int precision);
+// The configuration that a public one names (they differ for FP64 only).
+QueueConfig run_config(int precision, const QueueConfig &named);
 // The precision's default direction-split layout (for the ring sweep when the
 // context's own configuration is a row layout).
 QueueConfig default_split_config(int precision);
