@@ -1110,9 +1110,9 @@ int tvs_compute_sector(tvs_context *ctx, uint32_t angle, float *cumulative_surfa
     TVS_CUDA(ctx, cudaSetDevice(ctx->p.device));
     const uint64_t count = ctx->g.computable_points_count;
     // small surfaces pass through pinned memory both ways
-    tvs_host::SmallStage stage(ctx->stream);
+    tvs_host::SmallStage stage(ctx->stream, count * sizeof(float));
     float *host = cumulative_surfaces;
-    if (stage.p && count * sizeof(float) <= tvs_host::kSmall) {
+    if (stage.p) {
         host = reinterpret_cast<float *>(stage.p);
         std::memcpy(host, cumulative_surfaces, count * sizeof(float));
     }
@@ -1341,7 +1341,7 @@ int tvs_device_run_sectors(tvs_context *ctx, uint32_t first_angle, uint32_t coun
 int tvs_device_finish(tvs_context *ctx) {
     if (!ctx) return TVS_ERR_INVALID_ARGUMENT;
     TVS_CUDA(ctx, cudaSetDevice(ctx->p.device));
-    tvs_host::SmallStage stage(ctx->stream);
+    tvs_host::SmallStage stage(ctx->stream, sizeof(FinishBlock));
     FinishBlock own;
     FinishBlock *b = stage.p ? reinterpret_cast<FinishBlock *>(stage.p) : &own;
     TVS_CUDA(ctx, read_finish(ctx, b));
@@ -1583,8 +1583,8 @@ int tvs_run(tvs_context *ctx, float *cumulative_out, float *total_out, int want_
         const size_t bytes = ctx->g.computable_points_count * sizeof(float);
         const size_t head = (sizeof(FinishBlock) + 255) & ~(size_t)255;
         bool there = false;
-        if (head + 2 * bytes <= tvs_host::kSmall) {
-            tvs_host::SmallStage stage(ctx->stream);
+        {
+            tvs_host::SmallStage stage(ctx->stream, head + 2 * bytes);
             if (stage.p) {
                 FinishBlock *b = reinterpret_cast<FinishBlock *>(stage.p);
                 unsigned char *cum = stage.p + head, *tot = cum + bytes;

@@ -2,6 +2,7 @@
 #include "host_stage.hpp"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -12,10 +13,10 @@ namespace tvs_host {
 namespace {
 
 struct Stage {
-    std::mutex refs;  // users
+    std::mutex refs;  // users, and who makes the block
     int users = 0;
-    std::mutex lent;  // held by the call that uses the block
-    unsigned char *block = nullptr;
+    std::mutex lent;  // held by the call that uses the block, for as long as it waits for the GPU
+    std::atomic<unsigned char *> block{nullptr};  // made once, never freed
     std::mutex records_lent;  // the same for the record buffer
     unsigned char *records = nullptr;
     size_t records_cap = 0;
@@ -32,7 +33,6 @@ void stage_ref(bool device_set) {
     Stage &st = stage();
     std::lock_guard<std::mutex> lock(st.refs);
     st.users++;
-    std::lock_guard<std::mutex> lent(st.lent);
     if (st.block || !device_set) return;
     void *p = nullptr;
     if (posix_memalign(&p, 4096, kSmall) != 0) return;
@@ -41,23 +41,22 @@ void stage_ref(bool device_set) {
         std::free(p);
         return;
     }
-    st.block = (unsigned char *)p;
+    st.block = (unsigned char *)p;  // (a call that looked before takes the driver's path)
 }
 
 void stage_unref() {
     Stage &st = stage();
     std::lock_guard<std::mutex> lock(st.refs);
     if (--st.users > 0) return;
-    std::lock_guard<std::mutex> lent(st.lent);
     std::lock_guard<std::mutex> records(st.records_lent);
     if (st.records) cudaFreeHost(st.records);
     st.records = nullptr;
     st.records_cap = 0;
 }
 
-SmallStage::SmallStage(cudaStream_t stream) : stream_(stream) {
+SmallStage::SmallStage(cudaStream_t stream, size_t bytes) : stream_(stream) {
     Stage &st = stage();
-    if (!st.lent.try_lock()) return;
+    if (bytes > kSmall || !st.lent.try_lock()) return;
     p = st.block;
     if (!p) st.lent.unlock();
 }

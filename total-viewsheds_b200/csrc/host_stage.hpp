@@ -19,12 +19,13 @@ constexpr size_t kSmall = 256 << 10;
 void stage_ref(bool device_set);  // a context exists, its device current
 void stage_unref();
 
-// The block, for as long as this lives; p is null when it is lent or missing.  The
+// The block, for as long as this lives; p is null when it is lent, missing or smaller
+// than bytes.  No call waits for a lent block, nor does a context's creation or end.  The
 // copies between it and the device run on stream; unless done() has said that they
 // were waited for, the end of this waits for them (error paths).
 class SmallStage {
 public:
-    explicit SmallStage(cudaStream_t stream);
+    explicit SmallStage(cudaStream_t stream, size_t bytes = 0);
     void done() { stream_ = nullptr; }
     ~SmallStage();
     SmallStage(const SmallStage &) = delete;
