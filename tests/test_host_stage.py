@@ -66,3 +66,43 @@ int main() {
     return 0;
 }
 """) == 0
+
+
+def test_slots_without_memory_for_threads(tmp_path):
+    """The slots are laid out whatever memory there is for threads: none, or for the first
+    few alone.  (A single-core machine starts none.)"""
+    assert run(tmp_path, r"""
+#include <new>
+#include <vector>
+long left = -1;  // allocations until the first that fails (-1: none fails)
+void *operator new(size_t n) {
+    if (left == 0) throw std::bad_alloc();
+    if (left > 0) left--;
+    void *p = std::malloc(n);
+    if (!p) throw std::bad_alloc();
+    return p;
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, size_t) noexcept { std::free(p); }
+int main() {
+    const uint32_t bands = 40000, reserved = 200;  // 32 MB
+    std::vector<uint64_t> offsets(bands + 1);
+    for (uint32_t k = 0; k < bands; k++) offsets[k + 1] = offsets[k] + 1 + k % 7 + (k == 11) * 300;
+    std::vector<uint32_t> ids(offsets[bands]), rings((size_t)bands * reserved);
+    for (size_t i = 0; i < ids.size(); i++) ids[i] = (uint32_t)i + 1;
+    for (long memory : {0l, 2l, -1l}) {
+        rings.assign(rings.size(), 0xABCDABCDu);
+        left = memory;
+        tvs_host::expand_records(rings.data(), bands, reserved, offsets.data(), ids.data());
+        left = -1;
+        for (uint32_t k = 0; k < bands; k++) {
+            const uint32_t *row = &rings[(size_t)k * reserved];
+            const uint64_t n = offsets[k + 1] - offsets[k];
+            if (row[0] != n) return 1;
+            for (uint32_t i = 1; i < reserved; i++)
+                if (row[i] != (i <= n ? (uint32_t)(offsets[k] + i) : 0)) return 2;
+        }
+    }
+    return 0;
+}
+""") == 0

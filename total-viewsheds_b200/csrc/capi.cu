@@ -5,7 +5,9 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -407,15 +409,20 @@ void *ensure_planes(tvs_context *c, const tvs::QueueConfig &q, uint32_t tiles, u
         cudaStreamIsCapturing(c->stream, &capture);
         if (capture != cudaStreamCaptureStatusNone && !c->capturing_tvs) c->planes_captured = true;
         if (need <= c->planes_cap) return c->d_planes;
-        if (capture != cudaStreamCaptureStatusNone) {
+        auto as_they_are = [&]() -> void * {
             const size_t one = need / *sectors;
             *sectors = c->planes_cap >= one ? (uint32_t)(c->planes_cap / one) : n_sectors;
             return c->planes_cap >= one ? c->d_planes : nullptr;
-        }
+        };
+        if (capture != cudaStreamCaptureStatusNone) return as_they_are();
         if (c->d_planes) {
             cudaStreamSynchronize(c->stream);
             if (c->planes_captured) {
-                c->old_planes.push_back(c->d_planes);
+                try {
+                    c->old_planes.push_back(c->d_planes);
+                } catch (const std::bad_alloc &) {
+                    return as_they_are();
+                }
             } else {
                 tvs::plane_free(c->d_planes, c->stream);
                 c->device_bytes -= c->planes_cap;
@@ -729,13 +736,15 @@ int read_reference_rings(tvs_context *c, uint32_t *rings) {
         } else {  // no room to gather them: every slot crosses
             cudaGetLastError();
             c->d_ref_ids = nullptr;
-            std::vector<uint32_t> counts(bands);
-            TVS_CUDA(c, cudaMemcpyAsync(counts.data(), c->d_ref_lens, bands * sizeof(uint32_t),
+            const std::unique_ptr<uint32_t, void (*)(void *)> counts(
+                static_cast<uint32_t *>(std::malloc(bands * sizeof(uint32_t))), std::free);
+            if (!counts) return fail(c, TVS_ERR_OUT_OF_MEMORY, "ring record counts on the host");
+            TVS_CUDA(c, cudaMemcpyAsync(counts.get(), c->d_ref_lens, bands * sizeof(uint32_t),
                                         cudaMemcpyDeviceToHost, c->stream));
             TVS_CUDA(c, cudaMemcpyAsync(rings, c->d_rings, bands * R * sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                         c->stream));
             TVS_CUDA(c, cudaStreamSynchronize(c->stream));
-            tvs_host::complete_records(rings, bands, R, counts.data());
+            tvs_host::complete_records(rings, bands, R, counts.get());
             return TVS_OK;
         }
     }

@@ -5,8 +5,8 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <mutex>
-#include <system_error>
 #include <thread>
 
 namespace tvs_host {
@@ -124,7 +124,7 @@ void expand_records(uint32_t *rings, uint64_t bands, uint32_t reserved, const ui
             helpers[started] = std::thread(rows, at, to);
             at = to;
         }
-    } catch (const std::system_error &) {  // no more threads: the rest is done here
+    } catch (const std::exception &) {  // no more threads, or no memory for one: the rest is done here
     }
     rows(at, bands);
     for (int t = 0; t < started; t++) helpers[t].join();

@@ -68,6 +68,7 @@
 #include <climits>
 #include <map>
 #include <mutex>
+#include <new>
 #include <type_traits>
 #include <utility>
 
@@ -1387,6 +1388,13 @@ cudaError_t plane_alloc(void **p, size_t bytes, cudaStream_t s) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     std::lock_guard<std::mutex> lock(plane_mutex);
+    if (!plane_pools.count(dev)) {
+        try {
+            plane_pools[dev] = PlanePool{};
+        } catch (const std::bad_alloc &) {
+            return cudaErrorMemoryAllocation;
+        }
+    }
     PlanePool &q = plane_pools[dev];
     if (!q.pool) {
         cudaMemPoolProps props{};
