@@ -48,7 +48,8 @@ def _stale(target, deps):
 
 
 def build(force=False, verbose=False, ptxas_info=False):
-    deps = [CSRC / s for s in SOURCES] + list(CSRC.glob("*.cuh")) + [ROOT / "include" / "tvs.h"]
+    deps = ([CSRC / s for s in SOURCES] + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.hpp")) +
+            [ROOT / "include" / "tvs.h"])
     if force or ptxas_info or _stale(LIB, deps):
         cmd = [nvcc()] + flags() + (["-Xptxas", "-v"] if ptxas_info else []) + [
             "-shared", "-o", str(LIB)] + [str(CSRC / s) for s in SOURCES]
