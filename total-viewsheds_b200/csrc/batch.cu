@@ -138,8 +138,11 @@ int enqueue_run(tvs_batch *b, uint32_t count) {
             if (!c->d_quad) cfg.layout = tvs::kQuadFallback;
     uint32_t per = count;  // sectors per launch
     tvs::QueueArgs q = queue_args(b, 0, count);
+    // (a shorter run than the 180 sectors that the planes are sized for may want more a
+    // launch than those are evened out to: it takes the planes that there are)
     const size_t planes = tvs::split_plane_bytes((int)b->precision, b->cfg, b->tiles_per_sector, count, &per);
-    if (planes != 0 && planes <= b->planes_cap) q.planes = b->d_planes;
+    per = tvs::plane_sectors(b->planes_cap, planes, per, count);
+    if (per != 0) q.planes = b->d_planes;
     else per = count;
     for (uint32_t s = 0; s < count; s += per) {
         q.first_sector = s;

@@ -410,9 +410,9 @@ void *ensure_planes(tvs_context *c, const tvs::QueueConfig &q, uint32_t tiles, u
         if (capture != cudaStreamCaptureStatusNone && !c->capturing_tvs) c->planes_captured = true;
         if (need <= c->planes_cap) return c->d_planes;
         auto as_they_are = [&]() -> void * {
-            const size_t one = need / *sectors;
-            *sectors = c->planes_cap >= one ? (uint32_t)(c->planes_cap / one) : n_sectors;
-            return c->planes_cap >= one ? c->d_planes : nullptr;
+            const uint32_t per = tvs::plane_sectors(c->planes_cap, need, *sectors, n_sectors);
+            *sectors = per ? per : n_sectors;
+            return per ? c->d_planes : nullptr;
         };
         if (capture != cudaStreamCaptureStatusNone) return as_they_are();
         if (c->d_planes) {

@@ -336,6 +336,16 @@ cudaError_t plane_alloc(void **p, size_t bytes, cudaStream_t s);
 void plane_free(void *p, cudaStream_t s);
 size_t split_plane_bytes(int precision, const QueueConfig &c, uint32_t tiles_per_sector,
                          uint32_t n_sectors, uint32_t *sectors);
+// Sectors per launch of a sweep over n_sectors, which wants planes of `want` bytes for
+// `sectors` a launch, with planes of `held` bytes: launches of about even size of what
+// they hold; 0 where not one sector's fit (its surfaces are added in turn).
+inline uint32_t plane_sectors(size_t held, size_t want, uint32_t sectors, uint32_t n_sectors) {
+    if (want == 0 || want <= held) return want == 0 ? 0 : sectors;
+    const uint32_t fit = (uint32_t)(held / (want / sectors));
+    if (fit == 0) return 0;
+    const uint32_t launches = (n_sectors + fit - 1) / fit;
+    return (n_sectors + launches - 1) / launches;
+}
 cudaError_t launch_shape_batch(const ShapeArgs *d_args, uint32_t n_dems, uint32_t n_sectors,
                                cudaStream_t s);
 cudaError_t launch_combine(float *cum, float *total, const float *sf, const float *sb,
