@@ -1,0 +1,80 @@
+"""Surface planes are only speed: with little device memory left, calls that need some
+take the planes', and the sweeps that then find no room for planes give the same bits."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+W, LOS = 1201, 400  # 245 MB of planes for EXACT32's 180 sectors
+MB = 1 << 20
+
+
+def bits(a):
+    return np.ascontiguousarray(a).view(np.uint32)
+
+
+def engine(tvs, z, precision="exact32"):
+    return tvs.Engine(z, W, 30.0, LOS * 30, observer_height=1.65, precision=precision)
+
+
+def leave(free):
+    """Holds the device's memory but for `free` bytes (to within an allocation's 2 MB)."""
+    import torch
+
+    torch.empty(1, device="cuda")
+    torch.cuda.empty_cache()
+    torch.cuda.synchronize()
+    return torch.empty(torch.cuda.mem_get_info()[0] - free, dtype=torch.uint8, device="cuda")
+
+
+@pytest.fixture(scope="module")
+def terrain(synth):
+    return synth.fbm(W, W, 0.75, 3, 0.0, 1500.0)
+
+
+def test_ring_records_take_the_planes_memory(tvs, terrain):
+    """One sector's ring records need 82 MB of slots and a 64 MB list: neither is left
+    beside the planes of a whole run (100 MB), both are without them (345 MB)."""
+    import torch
+
+    with engine(tvs, terrain) as eng:
+        cum = np.zeros(eng.count, np.float32)
+        want = eng.compute_sector_rings(46, cum)
+    with engine(tvs, terrain) as eng:
+        run = eng.run()[:2]
+        before = eng.device_bytes()
+        held = leave(100 * MB)
+        try:
+            got = np.zeros(eng.count, np.float32)
+            offsets, ids, _ = eng.compute_sector_rings(46, got)
+            assert np.array_equal(bits(got), bits(cum))
+            assert np.array_equal(offsets, want[0]) and np.array_equal(ids, want[1])
+            after = eng.device_bytes()
+            again = eng.run()[:2]
+        finally:
+            del held
+            torch.cuda.empty_cache()
+        assert after < before + 200 * MB  # the planes' 245 MB are not counted any more
+        for a, b in zip(again, run):
+            assert np.array_equal(bits(a), bits(b))
+
+
+def test_a_context_takes_the_memory_of_freed_planes(tvs, terrain):
+    """The pool keeps freed planes while any context lives; a new context's own buffers (the
+    DEM's 5.8 MB, its copies' 23 MB and more, beside 6 MB left) come first."""
+    import torch
+
+    with engine(tvs, terrain) as first:
+        want = first.run()[:2]
+        with engine(tvs, terrain) as second:
+            second.run()
+        held = leave(6 * MB)
+        try:
+            with engine(tvs, terrain) as third:
+                got = third.run()[:2]
+        finally:
+            del held
+            torch.cuda.empty_cache()
+    for a, b in zip(got, want):
+        assert np.array_equal(bits(a), bits(b))

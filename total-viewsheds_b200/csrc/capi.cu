@@ -143,6 +143,27 @@ void drop_tvs_graph(tvs_context *c) {
     c->tvs_graph = nullptr;
 }
 
+// A buffer that a call cannot do without.  The surface planes are only speed: where
+// memory runs out the context's own go first (the driver takes freed ones back from
+// their pool by itself), and the next sweep takes what planes it then finds room for.
+template <typename T> cudaError_t needed_malloc(tvs_context *c, T **p, size_t bytes) {
+    const cudaError_t e = cudaMalloc(p, bytes);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (e != cudaErrorMemoryAllocation || !c->d_planes || c->planes_captured ||
+        cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess ||
+        capture != cudaStreamCaptureStatusNone)
+        return e;
+    cudaGetLastError();
+    cudaStreamSynchronize(c->stream);
+    drop_tvs_graph(c);  // a captured sweep holds them
+    tvs::plane_free(c->d_planes, c->stream);
+    cudaStreamSynchronize(c->stream);
+    c->device_bytes -= c->planes_cap;
+    c->d_planes = nullptr;
+    c->planes_cap = 0;
+    return cudaMalloc(p, bytes);
+}
+
 void free_all(tvs_context *c) {
     void *ptrs[] = {c->d_elev, c->d_cum, c->d_total, c->d_cum64, c->d_trig, c->d_hdr,
                     c->d_steps, c->d_offs, c->d_dtab, c->d_quads, c->d_segs, c->d_queue, c->d_error, c->d_hmax,
@@ -272,7 +293,7 @@ int ensure_rings(tvs_context *c, uint32_t slots) {
             c->d_rings = nullptr;
             c->ring_capacity = 0;
         }
-        e = cudaMalloc(&c->d_rings, std::max<uint64_t>(need, 1) * sizeof(uint32_t));
+        e = needed_malloc(c, &c->d_rings, std::max<uint64_t>(need, 1) * sizeof(uint32_t));
         if (e == cudaSuccess) {
             c->ring_capacity = std::max<uint64_t>(need, 1);
             c->device_bytes += c->ring_capacity * sizeof(uint32_t);
@@ -280,8 +301,8 @@ int ensure_rings(tvs_context *c, uint32_t slots) {
     }
     if (e == cudaSuccess && !c->d_spill) {
         c->spill_cap = kSpillCap;
-        e = cudaMalloc(&c->d_spill, (size_t)c->spill_cap * sizeof(uint4));
-        if (e == cudaSuccess) e = cudaMalloc(&c->d_counters, 4 * sizeof(uint32_t));
+        e = needed_malloc(c, &c->d_spill, (size_t)c->spill_cap * sizeof(uint4));
+        if (e == cudaSuccess) e = needed_malloc(c, &c->d_counters, 4 * sizeof(uint32_t));
         if (e == cudaSuccess) c->device_bytes += (size_t)c->spill_cap * sizeof(uint4) + 4 * sizeof(uint32_t);
     }
     if (e != cudaSuccess) {
@@ -295,8 +316,8 @@ int ensure_rings(tvs_context *c, uint32_t slots) {
 int ensure_plain_scratch(tvs_context *c) {
     if (c->d_sf) return TVS_OK;
     const uint64_t n = (uint64_t)(c->row_end - c->row_begin) * c->g.tvs_width;
-    TVS_CUDA(c, cudaMalloc(&c->d_sf, std::max<uint64_t>(n, 1) * sizeof(float)));
-    TVS_CUDA(c, cudaMalloc(&c->d_sb, std::max<uint64_t>(n, 1) * sizeof(float)));
+    TVS_CUDA(c, needed_malloc(c, &c->d_sf, std::max<uint64_t>(n, 1) * sizeof(float)));
+    TVS_CUDA(c, needed_malloc(c, &c->d_sb, std::max<uint64_t>(n, 1) * sizeof(float)));
     c->device_bytes += 2 * std::max<uint64_t>(n, 1) * sizeof(float);
     return TVS_OK;
 }
@@ -381,7 +402,7 @@ int ring_queue_dem(tvs_context *c, const tvs::QueueDem **dem, uint32_t *tiles, u
     }
     const tvs::QueueConfig q = tvs::default_split_config((int)c->p.precision);
     if (!c->d_qdem_rings) {
-        TVS_CUDA(c, cudaMalloc(&c->d_qdem_rings, sizeof(tvs::QueueDem)));
+        TVS_CUDA(c, needed_malloc(c, &c->d_qdem_rings, sizeof(tvs::QueueDem)));
         c->device_bytes += sizeof(tvs::QueueDem);
         tvs::QueueDem d = queue_dem(c);
         uint32_t done_total = 0;
@@ -839,6 +860,7 @@ int enqueue_shape_of(tvs_context *c, uint32_t first, uint32_t count) {
     return enqueue_shape(c, first, count);
 }
 void drop_tvs_graph_of(tvs_context *c) { drop_tvs_graph(c); }
+cudaError_t needed_malloc_of(tvs_context *c, void **p, size_t bytes) { return needed_malloc(c, p, bytes); }
 }  // namespace tvs_host
 
 extern "C" {
@@ -1047,7 +1069,7 @@ int tvs_axes(tvs_context *ctx, uint32_t angle, uint64_t first_rank, uint64_t cou
         if (count > tvs::kCandidateCap)
             return fail(ctx, TVS_ERR_CAPACITY, "tvs_axes rank range exceeds the candidate capacity");
         uint32_t *d_ids = nullptr;
-        TVS_CUDA(ctx, cudaMalloc(&d_ids, count * sizeof(uint32_t)));
+        TVS_CUDA(ctx, needed_malloc(ctx, &d_ids, count * sizeof(uint32_t)));
         const uint32_t slot = tvs::kSectorSteps;  // scratch slot
         tvs::SectorTrig t;
         TVS_CUDA(ctx, cudaMemcpyAsync(&t, ctx->d_trig + angle, sizeof t, cudaMemcpyDeviceToHost,
@@ -1074,7 +1096,7 @@ int tvs_axes(tvs_context *ctx, uint32_t angle, uint64_t first_rank, uint64_t cou
         TVS_CUDA(ctx, cudaMemcpy(&t, ctx->d_trig + angle, sizeof t, cudaMemcpyDeviceToHost));
         // The same device projection the shape stage uses (axes.rs:154-189).
         float *d_out = nullptr;
-        TVS_CUDA(ctx, cudaMalloc(&d_out, ctx->g.size * sizeof(float)));
+        TVS_CUDA(ctx, needed_malloc(ctx, &d_out, ctx->g.size * sizeof(float)));
         cudaError_t e = tvs::launch_sight_distances(t, ctx->g.width, ctx->g.height, d_out,
                                                     ctx->stream);
         if (e == cudaSuccess)
@@ -1189,9 +1211,9 @@ int tvs_compute_sectors_rings(tvs_context *ctx, uint32_t first_angle, uint32_t n
             ctx->d_rc_lens = nullptr;
             ctx->rc_records_cap = 0;
         }
-        TVS_CUDA(ctx, cudaMalloc(&ctx->d_rc_offsets, (recs + 1) * sizeof(uint64_t)));
-        TVS_CUDA(ctx, cudaMalloc(&ctx->d_rc_blocks, (nb + 1) * sizeof(uint64_t)));
-        TVS_CUDA(ctx, cudaMalloc(&ctx->d_rc_lens, std::max<uint64_t>(recs, 1) * sizeof(uint32_t)));
+        TVS_CUDA(ctx, needed_malloc(ctx, &ctx->d_rc_offsets, (recs + 1) * sizeof(uint64_t)));
+        TVS_CUDA(ctx, needed_malloc(ctx, &ctx->d_rc_blocks, (nb + 1) * sizeof(uint64_t)));
+        TVS_CUDA(ctx, needed_malloc(ctx, &ctx->d_rc_lens, std::max<uint64_t>(recs, 1) * sizeof(uint32_t)));
         ctx->rc_records_cap = recs;
         ctx->device_bytes += (recs + 1 + nb + 1) * sizeof(uint64_t) + recs * sizeof(uint32_t);
     }
@@ -1267,7 +1289,7 @@ int tvs_compute_sectors_rings(tvs_context *ctx, uint32_t first_angle, uint32_t n
         // twice the need: sectors' record counts vary, and a reallocation
         // (free + malloc of gigabytes) costs more than the spare memory
         const uint64_t cap = 2 * total;
-        TVS_CUDA(ctx, cudaMalloc(&ctx->d_rc_ids, std::max<uint64_t>(cap, 1) * sizeof(uint32_t)));
+        TVS_CUDA(ctx, needed_malloc(ctx, &ctx->d_rc_ids, std::max<uint64_t>(cap, 1) * sizeof(uint32_t)));
         ctx->rc_ids_cap = std::max<uint64_t>(cap, 1);
         ctx->device_bytes += ctx->rc_ids_cap * sizeof(uint32_t);
     }

@@ -100,9 +100,9 @@ int ensure_tables(tvs_context *c) {
     if (c->d_installed) return TVS_OK;
     const uint64_t bds = std::max<uint32_t>(c->g.band_deltas_size, 1);
     const uint64_t n = (uint64_t)tvs::kSectorSteps * bds;
-    TVS_CCUDA(c, cudaMalloc(&c->d_tab_deltas, n * sizeof(int32_t)));
-    TVS_CCUDA(c, cudaMalloc(&c->d_tab_dists, n * sizeof(float)));
-    TVS_CCUDA(c, cudaMalloc(&c->d_installed, tvs::kSectorSteps));
+    TVS_CCUDA(c, tvs_host::needed_malloc_of(c, (void **)&c->d_tab_deltas, n * sizeof(int32_t)));
+    TVS_CCUDA(c, tvs_host::needed_malloc_of(c, (void **)&c->d_tab_dists, n * sizeof(float)));
+    TVS_CCUDA(c, tvs_host::needed_malloc_of(c, (void **)&c->d_installed, tvs::kSectorSteps));
     TVS_CCUDA(c, cudaMemsetAsync(c->d_installed, 0, tvs::kSectorSteps, c->stream));
     c->device_bytes += n * (sizeof(int32_t) + sizeof(float)) + tvs::kSectorSteps;
     return TVS_OK;

@@ -115,4 +115,5 @@ int header_status_of(tvs_context *c, uint32_t first, uint32_t count);
 int fail_of(tvs_context *c, int code, const std::string &msg);
 int enqueue_shape_of(tvs_context *c, uint32_t first, uint32_t count);
 void drop_tvs_graph_of(tvs_context *c);
+cudaError_t needed_malloc_of(tvs_context *c, void **p, size_t bytes);
 }  // namespace tvs_host
