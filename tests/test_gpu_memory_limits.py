@@ -1,6 +1,8 @@
 """Surface planes are only speed: with little device memory left, calls that need some
 take the planes', and the sweeps that then find no room for planes give the same bits."""
 
+import contextlib
+
 import numpy as np
 import pytest
 
@@ -18,6 +20,7 @@ def engine(tvs, z, precision="exact32"):
     return tvs.Engine(z, W, 30.0, LOS * 30, observer_height=1.65, precision=precision)
 
 
+@contextlib.contextmanager
 def leave(free):
     """Holds the device's memory but for `free` bytes (to within an allocation's 2 MB)."""
     import torch
@@ -25,7 +28,12 @@ def leave(free):
     torch.empty(1, device="cuda")
     torch.cuda.empty_cache()
     torch.cuda.synchronize()
-    return torch.empty(torch.cuda.mem_get_info()[0] - free, dtype=torch.uint8, device="cuda")
+    held = torch.empty(torch.cuda.mem_get_info()[0] - free, dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        held.untyped_storage().resize_(0)
+        torch.cuda.empty_cache()
 
 
 @pytest.fixture(scope="module")
@@ -36,25 +44,19 @@ def terrain(synth):
 def test_ring_records_take_the_planes_memory(tvs, terrain):
     """One sector's ring records need 82 MB of slots and a 64 MB list: neither is left
     beside the planes of a whole run (100 MB), both are without them (345 MB)."""
-    import torch
-
     with engine(tvs, terrain) as eng:
         cum = np.zeros(eng.count, np.float32)
         want = eng.compute_sector_rings(46, cum)
     with engine(tvs, terrain) as eng:
         run = eng.run()[:2]
         before = eng.device_bytes()
-        held = leave(100 * MB)
-        try:
+        with leave(100 * MB):
             got = np.zeros(eng.count, np.float32)
             offsets, ids, _ = eng.compute_sector_rings(46, got)
             assert np.array_equal(bits(got), bits(cum))
             assert np.array_equal(offsets, want[0]) and np.array_equal(ids, want[1])
             after = eng.device_bytes()
             again = eng.run()[:2]
-        finally:
-            del held
-            torch.cuda.empty_cache()
         assert after < before + 200 * MB  # the planes' 245 MB are not counted any more
         for a, b in zip(again, run):
             assert np.array_equal(bits(a), bits(b))
@@ -63,18 +65,36 @@ def test_ring_records_take_the_planes_memory(tvs, terrain):
 def test_a_context_takes_the_memory_of_freed_planes(tvs, terrain):
     """The pool keeps freed planes while any context lives; a new context's own buffers (the
     DEM's 5.8 MB, its copies' 23 MB and more, beside 6 MB left) come first."""
-    import torch
-
     with engine(tvs, terrain) as first:
         want = first.run()[:2]
         with engine(tvs, terrain) as second:
             second.run()
-        held = leave(6 * MB)
-        try:
-            with engine(tvs, terrain) as third:
-                got = third.run()[:2]
-        finally:
-            del held
-            torch.cuda.empty_cache()
+        with leave(6 * MB), engine(tvs, terrain) as third:
+            got = third.run()[:2]
     for a, b in zip(got, want):
         assert np.array_equal(bits(a), bits(b))
+
+
+def test_plain_kernel_scratch_in_part(tvs, synth):
+    """The plain kernel's two scratch buffers (2.6 MB each): where only one fits the call
+    fails, also when it is made again, and the context computes once there is room."""
+    z = synth.fbm(2401, 2401, 0.75, 3, 0.0, 1500.0)
+    with tvs.Engine(z, 2401, 30.0, 800 * 30, observer_height=1.65, sweep_kernel="plain") as eng:
+        failed = 0
+        for free in (2, 3, 4, 5, 6):
+            with leave(free * MB):
+                for _ in range(2):
+                    try:
+                        eng.device_run_sectors(46, 1)
+                        eng.device_finish()
+                        break
+                    except tvs.TvsError as e:
+                        assert "out of memory" in str(e)
+                        failed += 1
+        assert failed >= 2
+        cum = np.zeros(eng.count, np.float32)
+        eng.compute_sector(46, cum)
+    with tvs.Engine(z, 2401, 30.0, 800 * 30, observer_height=1.65) as eng:
+        want = np.zeros(eng.count, np.float32)
+        eng.compute_sector(46, want)
+    assert np.array_equal(bits(cum), bits(want))

@@ -314,11 +314,13 @@ int ensure_rings(tvs_context *c, uint32_t slots) {
 }
 
 int ensure_plain_scratch(tvs_context *c) {
-    if (c->d_sf) return TVS_OK;
     const uint64_t n = (uint64_t)(c->row_end - c->row_begin) * c->g.tvs_width;
-    TVS_CUDA(c, needed_malloc(c, &c->d_sf, std::max<uint64_t>(n, 1) * sizeof(float)));
-    TVS_CUDA(c, needed_malloc(c, &c->d_sb, std::max<uint64_t>(n, 1) * sizeof(float)));
-    c->device_bytes += 2 * std::max<uint64_t>(n, 1) * sizeof(float);
+    const size_t bytes = std::max<uint64_t>(n, 1) * sizeof(float);
+    for (float **p : {&c->d_sf, &c->d_sb}) {  // (an earlier call may have got the first only)
+        if (*p) continue;
+        TVS_CUDA(c, needed_malloc(c, p, bytes));
+        c->device_bytes += bytes;
+    }
     return TVS_OK;
 }
 
