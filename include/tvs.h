@@ -266,8 +266,9 @@ void *tvs_stream(const tvs_context *ctx);
 uint64_t tvs_last_launch_count(const tvs_context *ctx);
 /* Bytes of device memory the context holds: the buffers of tvs_create, the
  * surface planes from the first sweep on, the ring buffers from the first run
- * that asks for ring records.  (The planes come from a pool per device that may
- * keep up to 1 GB of freed ones until the process's last context there ends.) */
+ * that asks for ring records.  (The library keeps up to 256 MB of the planes of
+ * contexts that ended, per device, until the last context with planes there ends or
+ * one of its own allocations finds no other memory.) */
 uint64_t tvs_device_bytes(const tvs_context *ctx);
 
 /* Failure detection of the persistent sweep (no counterpart in the reference,

@@ -84,14 +84,15 @@ int upload_dems(tvs_batch *b) {
     if (need > b->planes_cap) {
         if (b->d_planes) {
             cudaStreamSynchronize(b->stream);
-            tvs::plane_free(b->d_planes, b->stream);
+            tvs::plane_free(b->d_planes, b->planes_cap);
         }
         b->device_bytes -= b->planes_cap;
         b->d_planes = nullptr;
         b->planes_cap = 0;
-        if (tvs::plane_alloc(&b->d_planes, need, b->stream) == cudaSuccess) {
-            b->planes_cap = need;
-            b->device_bytes += need;
+        size_t bytes = need;
+        if (tvs::plane_alloc(&b->d_planes, &bytes) == cudaSuccess) {
+            b->planes_cap = bytes;
+            b->device_bytes += bytes;
         } else {
             cudaGetLastError();
             b->d_planes = nullptr;
@@ -202,7 +203,7 @@ int tvs_batch_create(const tvs_params *params, const float *const *elevations, u
         {(void **)&b->d_rechecks, sizeof(unsigned long long)},
     };
     for (auto &a : allocs) {
-        if (e == cudaSuccess) e = cudaMalloc(a.p, a.bytes);
+        if (e == cudaSuccess) e = tvs::device_malloc(a.p, a.bytes);
         if (e == cudaSuccess) b->device_bytes += a.bytes;
     }
     b->d_done = b->d_queue + 1;
@@ -237,7 +238,7 @@ void tvs_batch_destroy(tvs_batch *b) {
     void *ptrs[] = {b->d_shape, b->d_dems, b->d_queue, b->d_error, b->d_rechecks};
     for (void *p : ptrs)
         if (p) cudaFree(p);
-    if (b->d_planes) tvs::plane_free(b->d_planes, b->stream);
+    if (b->d_planes) tvs::plane_free(b->d_planes, b->planes_cap);
     if (b->stream) cudaStreamDestroy(b->stream);
     for (tvs_context *c : b->dems) tvs_destroy(c);
     delete b;

@@ -144,10 +144,10 @@ void drop_tvs_graph(tvs_context *c) {
 }
 
 // A buffer that a call cannot do without.  The surface planes are only speed: where
-// memory runs out the context's own go first (the driver takes freed ones back from
-// their pool by itself), and the next sweep takes what planes it then finds room for.
+// memory runs out the kept ones of other contexts go first, then the context's own, and
+// the next sweep takes what planes it then finds room for.
 template <typename T> cudaError_t needed_malloc(tvs_context *c, T **p, size_t bytes) {
-    const cudaError_t e = cudaMalloc(p, bytes);
+    const cudaError_t e = tvs::device_malloc(p, bytes);
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (e != cudaErrorMemoryAllocation || !c->d_planes || c->planes_captured ||
         cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess ||
@@ -156,12 +156,11 @@ template <typename T> cudaError_t needed_malloc(tvs_context *c, T **p, size_t by
     cudaGetLastError();
     cudaStreamSynchronize(c->stream);
     drop_tvs_graph(c);  // a captured sweep holds them
-    tvs::plane_free(c->d_planes, c->stream);
-    cudaStreamSynchronize(c->stream);
+    tvs::plane_free(c->d_planes, c->planes_cap);
     c->device_bytes -= c->planes_cap;
     c->d_planes = nullptr;
     c->planes_cap = 0;
-    return cudaMalloc(p, bytes);
+    return tvs::device_malloc(p, bytes);
 }
 
 void free_all(tvs_context *c) {
@@ -174,8 +173,8 @@ void free_all(tvs_context *c) {
                     c->d_ref_ids, c->d_bmax, c->d_qdem_rings, c->d_diag, c->d_quad};
     for (void *p : ptrs)
         if (p) cudaFree(p);
-    if (c->d_planes) tvs::plane_free(c->d_planes, c->stream);
-    for (void *p : c->old_planes) tvs::plane_free(p, c->stream);
+    if (c->d_planes) tvs::plane_free(c->d_planes, c->planes_cap);
+    for (const auto &p : c->old_planes) tvs::plane_free(p.first, p.second);
     drop_tvs_graph(c);
     for (cudaEvent_t ev : {c->ev_begin, c->ev_shaped, c->ev_swept})
         if (ev) cudaEventDestroy(ev);
@@ -442,12 +441,12 @@ void *ensure_planes(tvs_context *c, const tvs::QueueConfig &q, uint32_t tiles, u
             cudaStreamSynchronize(c->stream);
             if (c->planes_captured) {
                 try {
-                    c->old_planes.push_back(c->d_planes);
+                    c->old_planes.emplace_back(c->d_planes, c->planes_cap);
                 } catch (const std::bad_alloc &) {
                     return as_they_are();
                 }
             } else {
-                tvs::plane_free(c->d_planes, c->stream);
+                tvs::plane_free(c->d_planes, c->planes_cap);
                 c->device_bytes -= c->planes_cap;
             }
             c->planes_captured = false;
@@ -455,9 +454,10 @@ void *ensure_planes(tvs_context *c, const tvs::QueueConfig &q, uint32_t tiles, u
         c->d_planes = nullptr;
         c->planes_cap = 0;
         drop_tvs_graph(c);  // a captured sweep holds the old planes
-        if (tvs::plane_alloc(&c->d_planes, need, c->stream) == cudaSuccess) {
-            c->planes_cap = need;
-            c->device_bytes += need;
+        size_t bytes = need;
+        if (tvs::plane_alloc(&c->d_planes, &bytes) == cudaSuccess) {
+            c->planes_cap = bytes;
+            c->device_bytes += bytes;
             return c->d_planes;
         }
         cudaGetLastError();
@@ -715,7 +715,7 @@ int sweep_reference_rings(tvs_context *c, uint32_t angle) {
         if (!c->d_ref_lens) {  // without memory for it: counts in the slots, all of which cross
             const uint64_t words = tvs::ring_scan_blocks(bands) + 1 + bands + 1;
             const size_t bytes = words * sizeof(uint64_t) + std::max<uint64_t>(bands, 1) * sizeof(uint32_t);
-            if (cudaMalloc(&c->d_ref_scan, bytes) == cudaSuccess) {
+            if (tvs::device_malloc(&c->d_ref_scan, bytes) == cudaSuccess) {
                 c->d_ref_lens = reinterpret_cast<uint32_t *>(c->d_ref_scan + words);
                 c->device_bytes += bytes;
             } else {
@@ -753,7 +753,7 @@ int read_reference_rings(tvs_context *c, uint32_t *rings) {
         c->d_ref_ids = nullptr;
         c->ref_ids_cap = 0;
         const uint64_t cap = std::max<uint64_t>(total + total / 2, 1);
-        if (cudaMalloc(&c->d_ref_ids, cap * sizeof(uint32_t)) == cudaSuccess) {
+        if (tvs::device_malloc(&c->d_ref_ids, cap * sizeof(uint32_t)) == cudaSuccess) {
             c->ref_ids_cap = cap;
             c->device_bytes += cap * sizeof(uint32_t);
         } else {  // no room to gather them: every slot crosses
@@ -965,12 +965,12 @@ int tvs_create(const tvs_params *params, const float *elevations, uint64_t n_ele
         {(void **)&c->d_dists, (size_t)slots * bds * sizeof(float)},
     };
     for (auto &a : allocs) {
-        if ((e = cudaMalloc(a.p, a.bytes)) != cudaSuccess) return bail(e, "cudaMalloc");
+        if ((e = tvs::device_malloc(a.p, a.bytes)) != cudaSuccess) return bail(e, "cudaMalloc");
         c->device_bytes += a.bytes;
     }
     c->d_done = c->d_queue + 1;
     if (params->precision == TVS_PRECISION_MIXED64 || params->precision == TVS_PRECISION_FP64) {
-        if ((e = cudaMalloc(&c->d_cum64, count * sizeof(double))) != cudaSuccess)
+        if ((e = tvs::device_malloc(&c->d_cum64, count * sizeof(double))) != cudaSuccess)
             return bail(e, "cudaMalloc");
         c->device_bytes += count * sizeof(double);
     }
@@ -979,7 +979,7 @@ int tvs_create(const tvs_params *params, const float *elevations, uint64_t n_ele
     // plain DEM
     if (params->sweep_kernel == TVS_SWEEP_ENGINE && tvs::quad_fits(g.width, g.height)) {
         const size_t qb = 4 * tvs::quad_copy_elems(g.width, g.height) * sizeof(float4);
-        if (cudaMalloc(&c->d_quad, qb) == cudaSuccess) {
+        if (tvs::device_malloc(&c->d_quad, qb) == cudaSuccess) {
             c->device_bytes += qb;
         } else {
             cudaGetLastError();

@@ -44,7 +44,6 @@ constexpr uint32_t kSplitChunk = 8, kSplitGrab = 8;
 // and 774 ms, and as much as that longer to map them).
 constexpr size_t kPlaneBytes = (size_t)256 << 20, kPlaneBytesMost = (size_t)1 << 30;
 constexpr uint32_t kPlaneSectors = 32;
-constexpr uint64_t kPlanePoolBytes = kPlaneBytesMost;
 
 // Direction-split layouts 1-9: a warp holds LX columns x 32/LX rows of lanes;
 // each lane sweeps four points of view, LX columns apart (layouts 1-3: LX = 8,

@@ -68,7 +68,6 @@
 #include <climits>
 #include <map>
 #include <mutex>
-#include <new>
 #include <type_traits>
 #include <utility>
 
@@ -1371,61 +1370,6 @@ cudaError_t launch_persistent(const void *fn, const QueueArgs &a, uint64_t items
     e = cudaLaunchKernel(fn, dim3(grid), block, params, smem, s);
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
-}
-
-namespace {
-struct PlanePool {
-    cudaMemPool_t pool = nullptr;
-    uint64_t held = 0;  // planes not yet freed
-};
-std::mutex plane_mutex;
-std::map<int, PlanePool> plane_pools;  // by device
-}  // namespace
-
-cudaError_t plane_alloc(void **p, size_t bytes, cudaStream_t s) {
-    *p = nullptr;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> lock(plane_mutex);
-    if (!plane_pools.count(dev)) {
-        try {
-            plane_pools[dev] = PlanePool{};
-        } catch (const std::bad_alloc &) {
-            return cudaErrorMemoryAllocation;
-        }
-    }
-    PlanePool &q = plane_pools[dev];
-    if (!q.pool) {
-        cudaMemPoolProps props{};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.handleTypes = cudaMemHandleTypeNone;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        e = cudaMemPoolCreate(&q.pool, &props);
-        uint64_t keep = kPlanePoolBytes;
-        if (e == cudaSuccess)
-            e = cudaMemPoolSetAttribute(q.pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        if (e != cudaSuccess) return e;
-    }
-    e = cudaMallocFromPoolAsync(p, bytes, q.pool, s);
-    if (e == cudaSuccess) q.held++;
-    return e;
-}
-
-// The device is the one that the planes came from; the caller has waited for the
-// stream's work.
-void plane_free(void *p, cudaStream_t s) {
-    if (!p) return;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return;
-    std::lock_guard<std::mutex> lock(plane_mutex);
-    cudaFreeAsync(p, s);
-    PlanePool &q = plane_pools[dev];
-    if (--q.held == 0) {
-        cudaStreamSynchronize(s);
-        cudaMemPoolTrimTo(q.pool, 0);
-    }
 }
 
 size_t split_plane_bytes(int precision, const QueueConfig &c, uint32_t tiles_per_sector,

@@ -3,6 +3,7 @@
 
 #include <cstdint>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "tvs.h"
@@ -47,7 +48,7 @@ struct tvs_context {
     size_t planes_cap = 0;
     bool capturing_tvs = false;                // tvs_device_run_tvs captures its own graph
     bool planes_captured = false;              // a caller's graph may hold d_planes
-    std::vector<void *> old_planes;            // ... or these
+    std::vector<std::pair<void *, size_t>> old_planes;  // ... or these
     uint32_t spin_limit = tvs::kDefaultSpinLimit;  // dependency-wait iteration limit
     uint32_t held_tile = 0xFFFFFFFFu;               // failure-detection test hook
     int32_t *d_deltas = nullptr;

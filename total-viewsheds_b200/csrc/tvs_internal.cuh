@@ -327,15 +327,26 @@ void queue_tile(QueueDem *dems, uint32_t n_dems, const QueueConfig &c, uint32_t 
                 uint32_t *done_total, uint32_t *chunks);
 // Bytes of the surface planes that a split sweep over that many tiles per sector
 // wants, and the sectors that one of its launches then takes (at most n_sectors).
-// The planes come from a pool per device, so that a program that opens one DEM
-// after another does not map and unmap them each time (a 301^2 context's 33 MB cost
-// its first run 1 ms): plane_alloc and plane_free order on the stream; while any
-// plane is held the pool keeps up to kPlanePoolBytes of freed ones, and gives all
-// back with the last.
-cudaError_t plane_alloc(void **p, size_t bytes, cudaStream_t s);
-void plane_free(void *p, cudaStream_t s);
 size_t split_plane_bytes(int precision, const QueueConfig &c, uint32_t tiles_per_sector,
                          uint32_t n_sectors, uint32_t *sectors);
+// Their memory (planes.cu, of the current device): plane_alloc gives at least *bytes and
+// sets what it gave; plane_free takes planes that no work uses any more.  While any are
+// held up to kPlanesKept of freed ones are kept, so that a program that opens one DEM
+// after another allocates none; the last one's end and plane_trim give the kept ones
+// back.  They are ordinary allocations, mapped and unmapped in one piece: a driver's
+// memory pool does it in pieces of 33 MB, which for 245 MB took 1.65 and 1.55 ms against
+// 0.38 and 0.40, for 690 MB 4.6 and 4.4 against 0.63 and 0.73, paid by a program with
+// one context (1201^2 exact f32, create, run, destroy: 10.4 ms with the pool, 8.8 before
+// there were planes).
+constexpr size_t kPlanesKept = (size_t)256 << 20;
+cudaError_t plane_alloc(void **p, size_t *bytes);
+void plane_free(void *p, size_t bytes);
+void plane_trim();
+// cudaMalloc; where memory runs out the kept planes go first.
+cudaError_t device_malloc(void **p, size_t bytes);
+template <typename T> cudaError_t device_malloc(T **p, size_t bytes) {
+    return device_malloc(reinterpret_cast<void **>(p), bytes);
+}
 // Sectors per launch of a sweep over n_sectors, which wants planes of `want` bytes for
 // `sectors` a launch, with planes of `held` bytes: launches of about even size of what
 // they hold; 0 where not one sector's fit (its surfaces are added in turn).
