@@ -98,3 +98,17 @@ def test_plain_kernel_scratch_in_part(tvs, synth):
         want = np.zeros(eng.count, np.float32)
         eng.compute_sector(46, want)
     assert np.array_equal(bits(cum), bits(want))
+
+
+@pytest.mark.parametrize("precision", ["exact32", "fp64"])
+def test_a_context_without_memory_for_the_copies(tvs, terrain, precision):
+    """The DEM's row-interleaved copies (23 MB, with the DEM in one allocation) are only
+    speed too: where they do not fit beside a context's other buffers (15 MB), it runs
+    from the plain DEM, and adds the surfaces in turn."""
+    with engine(tvs, terrain, precision) as eng:
+        want = eng.run()[:2]
+    with leave(22 * MB), engine(tvs, terrain, precision) as eng:
+        assert eng.device_bytes() < 22 * MB
+        got = eng.run()[:2]
+    for a, b in zip(got, want):
+        assert np.array_equal(bits(a), bits(b))

@@ -170,7 +170,7 @@ void free_all(tvs_context *c) {
                     c->d_deltas, c->d_dists, c->d_rings, c->d_spill, c->d_counters, c->d_sf,
                     c->d_sb, c->d_tab_deltas, c->d_tab_dists, c->d_installed,
                     c->d_rc_blocks, c->d_rc_offsets, c->d_rc_lens, c->d_rc_ids, c->d_ref_scan,
-                    c->d_ref_ids, c->d_bmax, c->d_qdem_rings, c->d_diag, c->d_quad};
+                    c->d_ref_ids, c->d_bmax, c->d_qdem_rings, c->d_diag};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (c->d_planes) tvs::plane_free(c->d_planes, c->planes_cap);
@@ -944,7 +944,6 @@ int tvs_create(const tvs_params *params, const float *elevations, uint64_t n_ele
     const uint32_t slots = tvs::kSectorSteps + 1;
     const uint64_t bds = std::max<uint32_t>(g.band_deltas_size, 1);
     struct { void **p; size_t bytes; } allocs[] = {
-        {(void **)&c->d_elev, (g.size + tvs::kElevationPad) * sizeof(float)},
         {(void **)&c->d_cum, count * sizeof(float)},
         {(void **)&c->d_total, count * sizeof(float)},
         {(void **)&c->d_trig, slots * sizeof(tvs::SectorTrig)},
@@ -974,18 +973,22 @@ int tvs_create(const tvs_params *params, const float *elevations, uint64_t n_ele
             return bail(e, "cudaMalloc");
         c->device_bytes += count * sizeof(double);
     }
-    // the quad layout's copies (4x the DEM); without them (the plain kernel, a DEM past
-    // the 32-bit offsets, or no memory for them) the quad layout's tiling runs from the
-    // plain DEM
-    if (params->sweep_kernel == TVS_SWEEP_ENGINE && tvs::quad_fits(g.width, g.height)) {
-        const size_t qb = 4 * tvs::quad_copy_elems(g.width, g.height) * sizeof(float4);
-        if (tvs::device_malloc(&c->d_quad, qb) == cudaSuccess) {
-            c->device_bytes += qb;
-        } else {
-            cudaGetLastError();
-            c->d_quad = nullptr;
-        }
+    // The elevations, and behind them in one allocation (each costs 0.3 ms) the quad
+    // layout's copies (4x the DEM); without those (the plain kernel, a DEM past the 32-bit
+    // offsets, or no memory left for them) the quad layout's tiling runs from the plain DEM.
+    const size_t elev_bytes = ((g.size + tvs::kElevationPad) * sizeof(float) + 255) & ~(size_t)255;
+    size_t quad_bytes = params->sweep_kernel == TVS_SWEEP_ENGINE && tvs::quad_fits(g.width, g.height)
+                            ? 4 * tvs::quad_copy_elems(g.width, g.height) * sizeof(float4) : 0;
+    e = tvs::device_malloc(&c->d_elev, elev_bytes + quad_bytes);
+    if (e == cudaErrorMemoryAllocation && quad_bytes) {
+        cudaGetLastError();
+        quad_bytes = 0;
+        e = tvs::device_malloc(&c->d_elev, elev_bytes);
     }
+    if (e != cudaSuccess) return bail(e, "cudaMalloc");
+    if (quad_bytes)
+        c->d_quad = reinterpret_cast<float4 *>(reinterpret_cast<unsigned char *>(c->d_elev) + elev_bytes);
+    c->device_bytes += elev_bytes + quad_bytes;
     // Per-sector trigonometry on the host (glibc, as Rust std on linux-gnu):
     // axes.rs:95 shifts the angle in f32, axes.rs:127 adds 90 in f32.
     std::vector<tvs::SectorTrig> trig(slots);
