@@ -262,7 +262,8 @@ struct DeviceConstLock {
 // Sweep implementation for surface-only runs: the persistent work-queue
 // kernel (default), per-sector constant-table launches, or the one-launch
 // shared-memory kernel.  TVS_SWEEP_IMPL=queue|const|smem selects one for
-// comparisons; ring output always uses the shared-memory kernel.
+// comparisons; ring output uses the split sweep, but for FP64, TVS_SWEEP_IMPL and
+// the plain kernel (shared-memory kernel).
 enum class SweepImpl { Queue, Const, Smem };
 
 SweepImpl sweep_impl() {
@@ -346,7 +347,6 @@ tvs::QueueDem queue_dem(const tvs_context *c) {
     tvs::QueueDem d{};
     d.elev = c->d_elev;
     d.quad = c->d_quad;
-    d.quad_copy = tvs::quad_copy_elems(c->g.width, c->g.height);
     d.width = c->g.width;
     d.tvs_width = c->g.tvs_width;
     d.los = c->g.max_los_as_points;

@@ -175,7 +175,6 @@ struct SweepArgs {
 struct QueueDem {
     const float *elev;
     const float4 *quad;                // the row-interleaved copies (nullable)
-    uint64_t quad_copy;                // float4 per copy
     uint32_t width, tvs_width, los;
     uint32_t row_begin, row_end;
     float observer_height;
