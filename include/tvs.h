@@ -236,11 +236,12 @@ int tvs_device_reset(tvs_context *ctx);
  * (no host synchronisation, no rings).  Errors surface at tvs_device_finish. */
 int tvs_device_run_sectors(tvs_context *ctx, uint32_t first_angle, uint32_t count);
 /* The two stages of tvs_device_run_sectors, for callers that time them apart:
- * the shape stage (one CTA per sector) and the sweep (one launch). */
+ * the shape stage (one CTA per sector) and the sweep (a launch for as many sectors
+ * as its surface planes hold: 30 of MIXED64's at 3601^2, 11 at 7201^2). */
 int tvs_device_shape_sectors(tvs_context *ctx, uint32_t first_angle, uint32_t count);
 int tvs_device_sweep_sectors(tvs_context *ctx, uint32_t first_angle, uint32_t count);
 /* One whole total viewshed on the context's stream: zero the surfaces, the
- * shape stage of all 180 sectors and one persistent sweep over them.  The
+ * shape stage of all 180 sectors and the persistent sweep over them.  The
  * first call runs these as plain launches and captures them in a CUDA graph;
  * later calls replay the graph (one launch).  A new sweep configuration,
  * installed shapes, wait settings or counters drop the graph.  No counterpart
@@ -330,8 +331,8 @@ int tvs_autotune(tvs_context *ctx, uint32_t sample_sectors, tvs_sweep_config *ch
 
 /* No counterpart in the reference (which runs one DEM per process).  Many DEM
  * tiles of uneven, possibly rectangular size: every run computes all 180
- * sectors of every tile with one shape launch and one persistent sweep,
- * captured in a CUDA graph on the first run and replayed afterwards.
+ * sectors of every tile with one shape launch and the persistent sweep (whose
+ * launches take sectors of all tiles), captured in a CUDA graph on the first run and replayed afterwards.
  * params[i] and elevations[i] describe tile i (same device and precision for
  * every tile). */
 typedef struct tvs_batch tvs_batch;

@@ -296,7 +296,7 @@ class Engine:
         return offsets, ids[:total.value], st
 
     def compute_sectors_rings(self, first_angle, n_sectors, cumulative):
-        """Sectors first_angle .. first_angle + n_sectors - 1 in one launch, in
+        """Sectors first_angle .. first_angle + n_sectors - 1 together, in
         place on cumulative: (band_offsets u64 [n_sectors * total_bands + 1], ids
         u32, SectorStats); band k of sector first_angle + s is record
         s * total_bands + k."""
@@ -449,7 +449,7 @@ class Engine:
 
 class Batch:
     """Many DEM tiles (uneven, possibly rectangular), all 180 sectors each, one
-    shape launch and one persistent sweep per run (a replayed CUDA graph)."""
+    shape launch and the persistent sweep per run (a replayed CUDA graph)."""
 
     def __init__(self, dems, **kw):
         """dems: list of (heights [H, W] f32, scale, max_line_of_sight)."""

@@ -4,9 +4,10 @@
 // surfaces) and replays one captured graph per run:
 //   * the surfaces of every DEM are zeroed,
 //   * one shape launch computes every (DEM, sector) table (one CTA each),
-//   * one persistent sweep takes (sector, DEM, tile) items from a single
+//   * the persistent sweep takes (sector, DEM, tile) items from a single
 //     queue, so uneven and rectangular DEMs share the GPU without a tail per
-//     DEM (sweep_queue.cu).
+//     DEM, in launches of as many sectors as the surface planes hold
+//     (sweep_split.cu; the row layouts of sweep_queue.cu take all in one).
 // The sweep configuration (points of view per thread, tile shape, packed
 // arithmetic) comes from tvs_batch_autotune, which times the candidates on a
 // few sectors of the batch itself.

@@ -41,7 +41,7 @@ constexpr uint32_t kSplitChunk = 8, kSplitGrab = 8;
 // time (12 tiles of up to 1601^2: 65.0, 57.5, 53.6 and 51.8 ms with 32, 64, 128 and
 // 256 MB; 3601^2 MIXED64, 23 MB a sector: 103.5, 100.6 and 98.9 ms with 16, 32 and 64
 // sectors, exact f32 83.5, 82.4 and 81.3; 7201^2 MIXED64 with 1, 2 and 4 GB: 785, 779
-// and 774 ms, and as much as that longer to map them).
+// and 774 ms).
 constexpr size_t kPlaneBytes = (size_t)256 << 20, kPlaneBytesMost = (size_t)1 << 30;
 constexpr uint32_t kPlaneSectors = 32;
 

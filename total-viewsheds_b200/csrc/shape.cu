@@ -46,8 +46,8 @@ __device__ __forceinline__ uint32_t key_at(uint32_t x, double right, double s) {
     return f32_radix_key(projection32(x, right, s));
 }
 
-// The largest float below which no key < K lies, as the place where a projection
-// crosses from keys < K to keys >= K: halfway between the floats of K - 1 and K.
+// Where a projection crosses from keys < K to keys >= K: halfway between the floats of
+// the keys K - 1 and K.
 __device__ __forceinline__ double key_threshold(uint64_t K) {
     auto value = [](uint32_t k) -> double {
         return (double)__uint_as_float((k & 0x80000000u) ? k ^ 0x80000000u : ~k);
