@@ -437,6 +437,7 @@ void *ensure_planes(tvs_context *c, const tvs::QueueConfig &q, uint32_t tiles, u
             return per ? c->d_planes : nullptr;
         };
         if (capture != cudaStreamCaptureStatusNone) return as_they_are();
+        const tvs::AnyCapture any;
         if (c->d_planes) {
             cudaStreamSynchronize(c->stream);
             if (c->planes_captured) {

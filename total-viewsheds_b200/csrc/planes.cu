@@ -34,13 +34,6 @@ FreedPlanes *freed_of_current_device() {
     return cudaGetDevice(&dev) == cudaSuccess && dev < kDevices ? &freed[dev] : nullptr;
 }
 
-// A thread that captures another stream than the planes' may allocate and free them.
-struct AnyCapture {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    AnyCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    ~AnyCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-};
-
 // Frees (outside the lock: cudaFree waits for the device) what f keeps, and p.
 void give_back(FreedPlanes *f, std::unique_lock<std::mutex> lock, void *p = nullptr) {
     void *ps[FreedPlanes::kMost + 1] = {p};

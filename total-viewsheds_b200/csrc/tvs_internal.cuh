@@ -338,6 +338,13 @@ size_t split_plane_bytes(int precision, const QueueConfig &c, uint32_t tiles_per
 // one context (1201^2 exact f32, create, run, destroy: 10.4 ms with the pool, 8.8 before
 // there were planes).
 constexpr size_t kPlanesKept = (size_t)256 << 20;
+// While this lives, a thread that captures a stream of its own may allocate, free and
+// wait for other work, as a sweep that takes planes does.
+struct AnyCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    AnyCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~AnyCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
 cudaError_t plane_alloc(void **p, size_t *bytes);
 void plane_free(void *p, size_t bytes);
 void plane_trim();
