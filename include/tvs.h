@@ -274,7 +274,8 @@ uint64_t tvs_device_bytes(const tvs_context *ctx);
 
 /* Failure detection of the persistent sweep (no counterpart in the reference,
  * which has no device waits).  Where surfaces are added in turn (the row layouts;
- * the split layouts without memory for surface planes, or with a held tile) a work
+ * the split layouts without memory for one sector's surface planes, or with a held
+ * tile) a work
  * item waits for its tile's previous one before adding its own; the wait sleeps in steps of ~256 ns and
  * gives up after spin_limit steps (0 = the default, about 2 s): the item's
  * writes are skipped, later waits give up at once, and tvs_device_finish

@@ -112,3 +112,61 @@ def test_a_context_without_memory_for_the_copies(tvs, terrain, precision):
         got = eng.run()[:2]
     for a, b in zip(got, want):
         assert np.array_equal(bits(a), bits(b))
+
+
+@pytest.mark.parametrize("precision", ["exact32", "mixed64", "fp64"])
+def test_planes_of_fewer_sectors_where_memory_is_short(tvs, terrain, precision):
+    """70 MB hold a quarter or an eighth of the 180 sectors' planes (245, 489 MB): the sweep
+    takes launches of those, and neither asks again nor adds the surfaces in turn."""
+    with engine(tvs, terrain, precision) as eng:
+        want = eng.run()[:2]
+    with engine(tvs, terrain, precision) as eng:
+        before = eng.device_bytes()
+        with leave(70 * MB):
+            eng.device_reset()
+            eng.device_run_sectors(0, 180)
+            eng.device_finish()
+            held = eng.device_bytes()
+            assert 30 * MB <= held - before <= 70 * MB
+            assert 1 + 4 <= eng.last_launch_count() <= 1 + 9
+            got = eng.read_surfaces()
+            again = eng.run()[:2]
+        once_more = eng.run()[:2]  # (with memory to spare)
+        assert eng.device_bytes() == held
+    for r in (got, again, once_more):
+        for a, b in zip(r, want):
+            assert np.array_equal(bits(a), bits(b))
+
+
+@pytest.mark.parametrize("sectors_before", [0, 1])
+def test_a_callers_capture_allocates_planes(tvs, synth, sectors_before):
+    """A sweep that is captured takes planes for all its sectors, whatever there were."""
+    import torch
+
+    z = synth.fbm(601, 601, 0.8, 5, 0.0, 1500.0)
+    with tvs.Engine(z, 601, 30.0, 6000, observer_height=1.65) as eng:
+        want = eng.run()[:2]
+    with tvs.Engine(z, 601, 30.0, 6000, observer_height=1.65) as eng:
+        eng.set_queue_wait(0, 1 << 30)  # (uploads what a first sweep uploads, without planes)
+        eng.device_run_sectors(0, 1)
+        eng.set_queue_wait()
+        if sectors_before:
+            eng.device_run_sectors(0, sectors_before)
+        eng.device_finish()
+        before = eng.device_bytes()
+        graph, stream = torch.cuda.CUDAGraph(), torch.cuda.ExternalStream(eng.stream())
+        with torch.cuda.stream(stream):
+            graph.capture_begin(capture_error_mode="thread_local")
+            eng.device_reset()
+            eng.device_run_sectors(0, 180)
+            graph.capture_end()
+        assert eng.last_launch_count() == 2  # 338 tiles: 62 MB of planes
+        assert eng.device_bytes() - before >= 180 * 2 * 338 * 128 * 4
+        for _ in range(2):
+            with torch.cuda.stream(stream):
+                graph.replay()
+            eng.device_finish()
+            for a, b in zip(eng.read_surfaces(), want):
+                assert np.array_equal(bits(a), bits(b))
+        del graph
+        eng.run()

@@ -54,10 +54,10 @@ cudaError_t cudaFree(void *p) {
 #define CHECK(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); return 1; } } while (0)
 const size_t MB = 1 << 20;
 
-static void *take(size_t want, size_t *got = nullptr) {
+static void *take(size_t want, size_t *got = nullptr, size_t one = 0) {
     void *p;
     size_t n = want;
-    if (tvs::plane_alloc(&p, &n) != cudaSuccess) return nullptr;
+    if (tvs::plane_alloc(&p, &n, one) != cudaSuccess) return nullptr;
     if (got) *got = n;
     return p;
 }
@@ -110,6 +110,14 @@ int main() {
     CHECK(tvs::device_malloc(&buffer, 20 * MB) == cudaSuccess && used(0) == 30 * MB);
     CHECK(take(1000 * MB) == nullptr && used(0) == 30 * MB);
     cudaFree(buffer);
+    // where memory is short, the planes of fewer sectors: 180 of 1 MB, 90, 45, 22
+    room = used(0) + 40 * MB;
+    a = take(180 * MB, &got, MB);
+    CHECK(a && got == 22 * MB);
+    tvs::plane_free(a, got);
+    tvs::plane_trim();
+    room = used(0) + MB / 2;
+    CHECK(take(180 * MB, nullptr, MB) == nullptr);
     // the last one's end gives everything back
     room = (size_t)-1;
     a = take(100 * MB);

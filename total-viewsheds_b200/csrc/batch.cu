@@ -78,7 +78,7 @@ int upload_dems(tvs_batch *b) {
     TVS_BCUDA(b, cudaMemcpy(b->d_dems, d.data(), d.size() * sizeof(tvs::QueueDem),
                             cudaMemcpyHostToDevice));
     b->dems_uploaded = true;
-    // the split sweep's surface planes (without memory for them it adds in turn)
+    // the split sweep's surface planes (where memory is short, of fewer sectors)
     uint32_t per = 0;
     const size_t need = tvs::split_plane_bytes((int)b->precision, b->cfg, b->tiles_per_sector,
                                                tvs::kSectorSteps, &per);
@@ -91,7 +91,7 @@ int upload_dems(tvs_batch *b) {
         b->d_planes = nullptr;
         b->planes_cap = 0;
         size_t bytes = need;
-        if (tvs::plane_alloc(&b->d_planes, &bytes) == cudaSuccess) {
+        if (tvs::plane_alloc(&b->d_planes, &bytes, need / per) == cudaSuccess) {
             b->planes_cap = bytes;
             b->device_bytes += bytes;
         } else {

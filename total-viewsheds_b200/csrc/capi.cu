@@ -420,52 +420,73 @@ int ring_queue_dem(tvs_context *c, const tvs::QueueDem **dem, uint32_t *tiles, u
 
 // The split sweep's surface planes for a sweep of n_sectors and the sectors that
 // each of its launches takes; null (and every sector) where it adds the surfaces
-// in turn: a held tile of the failure test, or no memory for the planes.  A caller's
-// capture of the context's stream takes the planes that there are, and those then
-// stay where they are until the context's end.
+// in turn: a held tile of the failure test, or no memory for one sector's planes.  Planes
+// that a caller's capture of the context's stream may have taken stay where they are
+// until the context's end.
 void *ensure_planes(tvs_context *c, const tvs::QueueConfig &q, uint32_t tiles, uint32_t n_sectors,
                     uint32_t *sectors) {
     const size_t need = tvs::split_plane_bytes((int)c->p.precision, q, tiles, n_sectors, sectors);
-    if (need != 0 && c->held_tile == 0xFFFFFFFFu) {
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        cudaStreamIsCapturing(c->stream, &capture);
-        if (capture != cudaStreamCaptureStatusNone && !c->capturing_tvs) c->planes_captured = true;
-        if (need <= c->planes_cap) return c->d_planes;
-        auto as_they_are = [&]() -> void * {
-            const uint32_t per = tvs::plane_sectors(c->planes_cap, need, *sectors, n_sectors);
-            *sectors = per ? per : n_sectors;
-            return per ? c->d_planes : nullptr;
-        };
-        if (capture != cudaStreamCaptureStatusNone) return as_they_are();
-        const tvs::AnyCapture any;
-        if (c->d_planes) {
-            cudaStreamSynchronize(c->stream);
-            if (c->planes_captured) {
-                try {
-                    c->old_planes.emplace_back(c->d_planes, c->planes_cap);
-                } catch (const std::bad_alloc &) {
-                    return as_they_are();
-                }
-            } else {
-                tvs::plane_free(c->d_planes, c->planes_cap);
-                c->device_bytes -= c->planes_cap;
-            }
-            c->planes_captured = false;
+    if (need == 0 || c->held_tile != 0xFFFFFFFFu) {
+        *sectors = n_sectors;
+        return nullptr;
+    }
+    const size_t one = need / *sectors;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(c->stream, &status);
+    const bool capture = status != cudaStreamCaptureStatusNone;
+    if (capture && !c->capturing_tvs) c->planes_captured = true;
+    auto as_they_are = [&]() -> void * {
+        const uint32_t per = tvs::plane_sectors(c->planes_cap, need, *sectors, n_sectors);
+        *sectors = per ? per : n_sectors;
+        return per ? c->d_planes : nullptr;
+    };
+    // (memory that was short is not asked for again while some planes are there)
+    if (need <= c->planes_cap || c->capturing_tvs || (c->planes_cap >= one && need <= c->planes_short))
+        return as_they_are();
+    const tvs::AnyCapture any;
+    if (c->d_planes && (capture || c->planes_captured)) {  // these stay, for a graph or queued work
+        try {
+            c->old_planes.reserve(c->old_planes.size() + 1);
+        } catch (const std::bad_alloc &) {
+            return as_they_are();
         }
+        void *larger = nullptr;
+        size_t bytes = need;
+        if (tvs::plane_alloc(&larger, &bytes) != cudaSuccess) {
+            cudaGetLastError();
+            c->planes_short = need;
+            return as_they_are();
+        }
+        if (!capture) {
+            cudaStreamSynchronize(c->stream);
+            drop_tvs_graph(c);  // a captured sweep holds the old planes
+        }
+        c->old_planes.emplace_back(c->d_planes, c->planes_cap);
+        c->planes_captured = capture;
+        c->d_planes = larger;
+        c->planes_cap = bytes;
+        c->device_bytes += bytes;
+        return as_they_are();
+    }
+    if (c->d_planes) {
+        cudaStreamSynchronize(c->stream);
+        tvs::plane_free(c->d_planes, c->planes_cap);
+        c->device_bytes -= c->planes_cap;
         c->d_planes = nullptr;
         c->planes_cap = 0;
-        drop_tvs_graph(c);  // a captured sweep holds the old planes
-        size_t bytes = need;
-        if (tvs::plane_alloc(&c->d_planes, &bytes) == cudaSuccess) {
-            c->planes_cap = bytes;
-            c->device_bytes += bytes;
-            return c->d_planes;
-        }
+    }
+    if (!capture) drop_tvs_graph(c);  // a captured sweep holds the old planes, or none
+    size_t bytes = need;
+    if (tvs::plane_alloc(&c->d_planes, &bytes, one) == cudaSuccess) {
+        c->planes_cap = bytes;
+        c->device_bytes += bytes;
+    } else {
         cudaGetLastError();
         c->d_planes = nullptr;
     }
-    *sectors = n_sectors;
-    return nullptr;
+    c->planes_captured = capture;
+    c->planes_short = c->planes_cap < need ? need : 0;
+    return as_they_are();
 }
 
 // Sweep sectors [first, first+count) (slots == angles).  ring_slots != 0:

@@ -47,7 +47,7 @@ void give_back(FreedPlanes *f, std::unique_lock<std::mutex> lock, void *p = null
 
 }  // namespace
 
-cudaError_t plane_alloc(void **p, size_t *bytes) {
+cudaError_t plane_alloc(void **p, size_t *bytes, size_t one) {
     *p = nullptr;
     FreedPlanes *f = freed_of_current_device();
     if (f) {
@@ -65,7 +65,12 @@ cudaError_t plane_alloc(void **p, size_t *bytes) {
         }
     }
     const AnyCapture any;
-    const cudaError_t e = device_malloc(p, *bytes);
+    cudaError_t e = device_malloc(p, *bytes);
+    while (e == cudaErrorMemoryAllocation && one != 0 && *bytes >= 2 * one) {
+        cudaGetLastError();
+        *bytes = *bytes / one / 2 * one;
+        e = device_malloc(p, *bytes);
+    }
     if (e != cudaSuccess && f) {
         std::unique_lock<std::mutex> lock(mutex);
         if (--f->held == 0) give_back(f, std::move(lock));

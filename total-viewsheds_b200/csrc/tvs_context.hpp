@@ -46,6 +46,7 @@ struct tvs_context {
     uint32_t q_tiles_per_sector = 0, q_chunks = 0;
     void *d_planes = nullptr;                  // split_plane_bytes (grown on use)
     size_t planes_cap = 0;
+    size_t planes_short = 0;                   // what memory was short for (0: it was not)
     bool capturing_tvs = false;                // tvs_device_run_tvs captures its own graph
     bool planes_captured = false;              // a caller's graph may hold d_planes
     std::vector<std::pair<void *, size_t>> old_planes;  // ... or these
