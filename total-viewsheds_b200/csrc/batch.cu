@@ -275,6 +275,7 @@ int tvs_batch_set_sweep_config(tvs_batch *b, const tvs_sweep_config *cfg) {
         return bfail(b, TVS_ERR_INVALID_ARGUMENT, "sweep layouts 1-9 are not available for FP64");
     if (c.layout == 0 && b->precision == TVS_PRECISION_FP32)
         return bfail(b, TVS_ERR_INVALID_ARGUMENT, "the FP32 form runs on sweep layouts 1-9 only");
+    TVS_BCUDA(b, cudaSetDevice(b->device));  // (larger planes are allocated there)
     return set_config(b, tvs::run_config((int)b->precision, c));
 }
 
