@@ -2,6 +2,7 @@
 take the planes', and the sweeps that then find no room for planes give the same bits."""
 
 import contextlib
+import ctypes
 
 import numpy as np
 import pytest
@@ -22,18 +23,35 @@ def engine(tvs, z, precision="exact32"):
 
 @contextlib.contextmanager
 def leave(free):
-    """Holds the device's memory but for `free` bytes (to within an allocation's 2 MB)."""
+    """Holds the device's memory but for `free` bytes (in allocations of 2 MB).  What the
+    device reports as free cannot all be had, so `free` bytes are taken first, then all
+    that there is, and the first are given back."""
     import torch
 
     torch.empty(1, device="cuda")
-    torch.cuda.empty_cache()
     torch.cuda.synchronize()
-    held = torch.empty(torch.cuda.mem_get_info()[0] - free, dtype=torch.uint8, device="cuda")
+    torch.cuda.empty_cache()
+    cuda, held = ctypes.CDLL("libcuda.so.1"), []
+
+    def take(n):
+        p = ctypes.c_uint64()
+        rc = cuda.cuMemAlloc_v2(ctypes.byref(p), ctypes.c_size_t(n))
+        assert rc in (0, 2), rc  # (2: out of memory)
+        if rc == 0:
+            held.append(p)
+        return rc == 0
+
     try:
+        assert take(free)
+        n = torch.cuda.mem_get_info()[0] // (2 * MB) * 2 * MB
+        while n >= 2 * MB:
+            if not take(n):
+                n = n // (4 * MB) * 2 * MB
+        cuda.cuMemFree_v2(held.pop(0))
         yield
     finally:
-        held.untyped_storage().resize_(0)
-        torch.cuda.empty_cache()
+        for p in held:
+            cuda.cuMemFree_v2(p)
 
 
 @pytest.fixture(scope="module")
